@@ -72,14 +72,31 @@ HT_D Q4 q_addc(Q4 a, C2 b) { return q4(a.x + b.x, a.y + b.y, a.z + 0.0f, a.w + 0
 
 // ------------------------------------------------------------------- division
 // Correctly rounded quotients that share one reciprocal (Markstein's correction step):
-//   y = RN(1/b),  q0 = RN(a*y),  r = a - b*q0 (exact with an FMA),  q = RN(q0 + r*y) = RN(a/b)
+//   y = RN(1/b),  q0 = RN(a*y),  r = b*q0 - a (exact with an FMA),  q = RN(q0 - r*y) = RN(a/b)
 // (P. Markstein, "IA-64 and Elementary Functions", 2000; Muller et al., "Handbook of
-// Floating-Point Arithmetic", 2nd ed., section 4.7, Markstein's theorem). The identity
-// needs every intermediate to be a normal number, so each quotient checks that |q0| lies in
-// [2^-60, 2^60] (or a == 0, where q0 already carries the IEEE sign of zero) and each divisor
-// that |b| does; a group with any value outside redoes its divisions with IEEE division.
+// Floating-Point Arithmetic", 2nd ed., section 4.7, Markstein's theorem). Divisors here are
+// squared norms and lengths (b > 0); taking the residual as b*q0 - a keeps IEEE's sign of a
+// zero quotient without a select (a = -0: q0 = -0, r = +0, q = -0 + -0). The identity needs
+// every intermediate to be a normal number: each divisor lies in [2^-60, 2^60] and each
+// numerator is zero or at least 2^-60 (then |q0| >= 2^-120 and the residual's last place is at
+// least 2^-108). A numerator so large that q0 overflows makes q NaN, and NaN reaches the
+// length of the result, whose own range check fails. A group with any value outside redoes its
+// divisions with IEEE division. The numerators' check costs one add and half a 3-input minimum
+// per quotient (2 * bits - 1 drops the sign and maps zero to the largest word): about 4.5
+// instructions per quotient in place of 9 with a range test of every q0, 17 quotients per ray
+// map, three to nine maps per hop. Measured together with sincos_turn and the estimate's loop
+// per shape (ht_trace.cuh): 1080p / 200 objects, 8 passes 17.24 -> 16.09 ms; 800x600 / 18
+// objects, 64 passes 27.2 -> 24.4 ms; 24 mixed views batched 61.2 -> 57.2 ms.
 // tests/test_gpu_math.py compares qdiv with IEEE division on billions of inputs.
 struct Rcp { float b, y; };
+struct DivCheck {   // of one group of quotients
+    uint32_t least;   // over the numerators: 2 * bits - 1
+    bool bad;         // a divisor out of range
+};
+constexpr uint32_t DIV_LEAST = 2u * 0x21800000u - 1u;   // the word of 2^-60
+HT_D DivCheck div_check() { DivCheck c; c.least = 0xFFFFFFFFu; c.bad = false; return c; }
+HT_D bool div_failed(const DivCheck &c) { return c.bad | (c.least < DIV_LEAST); }
+HT_D uint32_t div_word(float a) { const uint32_t b = __float_as_uint(a); return b + b - 1u; }
 HT_D bool in_safe_range(float x) {
     const float ax = fabsf(x);
     return ax >= 0x1p-60f && ax <= 0x1p60f;
@@ -91,21 +108,42 @@ HT_D Rcp rcp_of(float b, bool &bad) {
     r.y = __frcp_rn(b);
     return r;
 }
-HT_D float qdiv(float a, const Rcp &r, bool &bad) {
+HT_D Rcp rcp_of(float b, DivCheck &c) { return rcp_of(b, c.bad); }
+HT_D float qdiv_unchecked(float a, const Rcp &r) {
     const float q0 = a * r.y;
-    const float e = fmaf(-r.b, q0, a);
-    const float q = fmaf(e, r.y, q0);
-    bad |= (a != 0.0f) & !in_safe_range(q0);
-    return q0 == 0.0f ? q0 : q;
+    const float e = fmaf(r.b, q0, -a);
+    return fmaf(-e, r.y, q0);
 }
-HT_D Q4 qdiv4(Q4 a, const Rcp &r, bool &bad) {
-    return q4(qdiv(a.x, r, bad), qdiv(a.y, r, bad), qdiv(a.z, r, bad), qdiv(a.w, r, bad));
+HT_D float qdiv(float a, const Rcp &r, DivCheck &c) {
+    c.least = min(c.least, div_word(a));
+    return qdiv_unchecked(a, r);
+}
+// One quotient with a check of its own, for a divisor of either sign.
+HT_D float qdiv(float a, const Rcp &r, bool &bad) {
+    bad |= (div_word(a) < DIV_LEAST) | (fabsf(a * r.y) > 0x1p60f) | (a == 0.0f & r.b < 0.0f);
+    return qdiv_unchecked(a, r);
+}
+HT_D Q4 qdiv4(Q4 a, const Rcp &r, DivCheck &c) {
+    c.least = min(min(c.least, div_word(a.x)), min(min(div_word(a.y), div_word(a.z)), div_word(a.w)));
+    return q4(qdiv_unchecked(a.x, r), qdiv_unchecked(a.y, r), qdiv_unchecked(a.z, r), qdiv_unchecked(a.w, r));
 }
 // normalize4 through one correctly rounded reciprocal of the length.
-HT_D Q4 normalize4_fast(Q4 a, bool &bad) {
+HT_D Q4 normalize4_fast(Q4 a, DivCheck &c) {
     float l = sqrtf(dot4(a, a));
-    Rcp r = rcp_of(l, bad);
-    return qdiv4(a, r, bad);
+    Rcp r = rcp_of(l, c);
+    return qdiv4(a, r, c);
+}
+
+// q_inverse(d) = conj(d) / |d|^2 through one reciprocal (the four divisions share it).
+static __device__ __noinline__ Q4 q_inverse_ieee(Q4 d) {
+    const float d2 = dot4(d, d);
+    return q4(d.x / d2, (-d.y) / d2, (-d.z) / d2, (-d.w) / d2);
+}
+HT_D Q4 q_inverse(Q4 d) {
+    DivCheck chk = div_check();
+    const Rcp r = rcp_of(dot4(d, d), chk);
+    const Q4 q = qdiv4(q4(d.x, -d.y, -d.z, -d.w), r, chk);
+    return div_failed(chk) ? q_inverse_ieee(d) : q;
 }
 
 // ------------------------------------------------------------------- Moebius
@@ -137,24 +175,24 @@ static __device__ __noinline__ HyRay ray_hy_map_ieee(const Mo m, const Q4 p, con
 // ray_<hy>_map (geometry/ray_map.inl:15-21): the nine divisions by |d|^2 share one
 // reciprocal, each normalize shares one; results are bit-identical to ray_hy_map_ieee.
 HT_D HyRay ray_hy_map(const Mo &m, Q4 p, Q4 v) {
-    bool bad = false;
+    DivCheck chk = div_check();
     Q4 u = q_addc(cq_mul(m.a, p), m.b);
     Q4 d = q_addc(cq_mul(m.c, p), m.d);
     float d2 = dot4(d, d);
-    Rcp rd = rcp_of(d2, bad);
-    Q4 di = qdiv4(q4(d.x, -d.y, -d.z, -d.w), rd, bad);
+    Rcp rd = rcp_of(d2, chk);
+    Q4 di = qdiv4(q4(d.x, -d.y, -d.z, -d.w), rd, chk);
     HyRay o;
     o.p = q_mul(u, di);
     Q4 g1 = q_mul(cq_mul(m.a, v), di);
     Q4 cv = cq_mul(m.c, v);
     Q4 g21 = q_conj(cv);
-    float k = qdiv(2.0f * dot4(d, cv), rd, bad);
+    float k = qdiv(2.0f * dot4(d, cv), rd, chk);
     Q4 dc = q_conj(d);
     Q4 g22 = q4(k * dc.x, k * dc.y, k * dc.z, k * dc.w);
-    Q4 g2 = q_mul(u, qdiv4(q_sub(g21, g22), rd, bad));
+    Q4 g2 = q_mul(u, qdiv4(q_sub(g21, g22), rd, chk));
     Q4 deriv = q_add(g1, g2);
-    o.v = normalize4_fast(normalize4_fast(deriv, bad), bad);
-    if (bad) return ray_hy_map_ieee(m, p, v);
+    o.v = normalize4_fast(normalize4_fast(deriv, chk), chk);
+    if (div_failed(chk)) return ray_hy_map_ieee(m, p, v);
     return o;
 }
 // The same map, out of line: the object scan and the hit path share this one copy of its
@@ -242,6 +280,37 @@ HT_D Q4 hy_dir_at(Q4 p, Q4 d, Q4 h) {
 }
 
 // ------------------------------------------------------------------- samplers / rotations
+// (float)sin(x) and (float)cos(x) of a float angle in [0, 2 pi], evaluated in FP64 and rounded
+// once: quarter turns taken off with pi/2 in two parts (Cody and Waite), then the Taylor series
+// on [-pi/4, pi/4] (the first term left out is below 2^-58 of the result). A sampler's angles
+// are 2 pi u of a 32-bit state, so every one of them was compared with CUDA's FP64 sincos
+// (tests/test_gpu_sincos.py): the same floats. That function also serves large angles, which
+// costs the hop kernels twice the instructions and a slow path in their instruction stream.
+HT_D void sincos_turn(float angle, float &sn, float &cs) {
+    const double x = (double)angle;
+    const double k = rint(x * 0.63661977236758134308);
+    const double r = fma(-k, 6.12323399573676603587e-17, fma(-k, 1.57079632679489655800, x));
+    const double z = r * r;
+    double s = fma(z, 1.0 / 355687428096000.0, -1.0 / 1307674368000.0);
+    double c = fma(z, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
+    s = fma(z, s, 1.0 / 6227020800.0);
+    c = fma(z, c, 1.0 / 479001600.0);
+    s = fma(z, s, -1.0 / 39916800.0);
+    c = fma(z, c, -1.0 / 3628800.0);
+    s = fma(z, s, 1.0 / 362880.0);
+    c = fma(z, c, 1.0 / 40320.0);
+    s = fma(z, s, -1.0 / 5040.0);
+    c = fma(z, c, -1.0 / 720.0);
+    s = fma(z, s, 1.0 / 120.0);
+    c = fma(z, c, 1.0 / 24.0);
+    s = fma(z, s, -1.0 / 6.0);
+    c = fma(z, c, -0.5);
+    const float fs = (float)fma(r * z, s, r), fc = (float)fma(z, c, 1.0);
+    const int q = (int)k;
+    const float a = q & 1 ? fc : fs, b = q & 1 ? fs : fc;
+    sn = q & 2 ? -a : a;
+    cs = (q + 1) & 2 ? -b : b;
+}
 // random_hemisphere_cosine (kernel/ocl/random.cc:37-39,53-59). cos/sin are evaluated in
 // FP64 and rounded once: this lands on the correctly rounded float, which the host libm
 // the reference is built against matches far more often than a float kernel does.
@@ -250,9 +319,9 @@ HT_D V3 hemisphere_cosine(uint32_t &s) {
     float sqr_cos_theta = rng_uniform(s);
     float cos_theta = sqrtf(sqr_cos_theta);
     float sin_theta = sqrtf(1.0f - sqr_cos_theta);
-    double sd, cd;
-    sincos((double)phi, &sd, &cd);
-    return v3((float)cd * sin_theta, (float)sd * sin_theta, cos_theta);
+    float sd, cd;
+    sincos_turn(phi, sd, cd);
+    return v3(cd * sin_theta, sd * sin_theta, cos_theta);
 }
 // rot3_look_at_cont / rot3_look_at / rot3_from_axis (kernel/ocl/transform/rotation.cc)
 HT_D Q4 rot3_look_at_cont(V3 d) {
@@ -266,11 +335,8 @@ HT_D Q4 rot3_look_at_cont(V3 d) {
 HT_D Q4 rot3_look_at(V3 d) {
     if (d.z < 0.0f) return rot3_look_at_cont(d);
     Q4 a = rot3_look_at_cont(v3(-d.x, -d.y, -d.z));
-    const float half = 3.14159265358979323846f / 2.0f;
-    double sh, ch;
-    sincos((double)half, &sh, &ch);
-    float s = (float)sh;
-    Q4 b = q4((float)ch, s * 1.0f, s * 0.0f, s * 0.0f);
+    // rot3_from_axis(x, pi): the FP64 sine and cosine of (float)pi / 2, each rounded to float
+    Q4 b = q4(-0x1.777a5cp-25f, 1.0f, 0.0f, 0.0f);
     return q_mul(a, b);
 }
 

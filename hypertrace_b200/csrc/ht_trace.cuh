@@ -252,15 +252,19 @@ HT_D bool culled_slot(const StagedScene &s, uint32_t q, const BoundRay &r, const
 // sure_crossing_e2) among the first HT_EST_OBJECTS / 2 planes and the first HT_EST_OBJECTS / 2
 // horospheres of the staged slots, +inf when none qualifies. A threshold derived from it
 // (cull_from_dist) then culls before the first exact test.
+// SHAPE: the slots' shape (planes come first, then horospheres), so each loop carries one
+// shape's test only.
+template <uint32_t SHAPE>
 HT_D float est_range(const StagedScene &s, uint32_t q0, uint32_t q1, const BoundRay &r, uint32_t prev_hash, float best) {
+#pragma unroll 1
     for (uint32_t q = q0; q < q1; ++q)   // warp-uniform: broadcast loads
-        best = fminf(best, sure_crossing_e2(bound_fw(s.bound[q], s.mag[q], r), s.shape[q], s.orig[q] == prev_hash, r.t));
+        best = fminf(best, sure_crossing_e2(bound_fw(s.bound[q], s.mag[q], r), SHAPE, SHAPE == 0 && s.orig[q] == prev_hash, r.t));
     return best;
 }
 HT_D float upper_estimate(const StagedScene &s, const BoundRay &r, uint32_t prev_hash) {
     const uint32_t half = HT_EST_OBJECTS / 2, h0 = (s.n_planes + 1) & ~1u;
-    float best = est_range(s, 0, min(half, s.n_planes), r, prev_hash, __int_as_float(0x7f800000));
-    best = est_range(s, h0, min(h0 + half, s.ns), r, prev_hash, best);
+    float best = est_range<0>(s, 0, min(half, s.n_planes), r, prev_hash, __int_as_float(0x7f800000));
+    best = est_range<1>(s, h0, min(h0 + half, s.ns), r, prev_hash, best);
     return best < __int_as_float(0x7f800000) ? dist_from_e2(best) : best;
 }
 

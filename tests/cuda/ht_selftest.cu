@@ -92,6 +92,31 @@ __global__ void k_monotone(unsigned long long *out) {
     atomicAdd(&out[1], viol);
 }
 
+// Exhaustive: sincos_turn at the sampler's angle of every 32-bit RNG state against CUDA's FP64
+// sincos rounded to float (random_hemisphere_cosine, kernel/ocl/random.cc:53-59).
+__global__ void k_sincos(unsigned long long *out) {
+    unsigned long long checked = 0, mism = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (1ull << 32); i += (uint64_t)gridDim.x * blockDim.x) {
+        const float phi = 2.0f * 3.14159265358979323846f * (__uint2float_rn((uint32_t)i) / 4294967296.0f);
+        float sn, cs;
+        sincos_turn(phi, sn, cs);
+        double sd, cd;
+        sincos((double)phi, &sd, &cd);
+        ++checked;
+        if (__float_as_uint(sn) != __float_as_uint((float)sd) || __float_as_uint(cs) != __float_as_uint((float)cd)) ++mism;
+    }
+    atomicAdd(&out[0], checked);
+    atomicAdd(&out[1], mism);
+}
+// rot3_look_at's half turn: the FP64 sine and cosine of (float)pi / 2, rounded to float.
+__global__ void k_half_turn(unsigned long long *out) {
+    volatile float half = 3.14159265358979323846f / 2.0f;
+    double sd, cd;
+    sincos((double)half, &sd, &cd);
+    out[0] = __float_as_uint((float)sd);
+    out[1] = __float_as_uint((float)cd);
+}
+
 static int run(void (*launch)(unsigned long long *), unsigned long long *host) {
     unsigned long long *d = nullptr;
     if (cudaMalloc(&d, 2 * sizeof(unsigned long long)) != cudaSuccess) return -2;
@@ -101,6 +126,13 @@ static int run(void (*launch)(unsigned long long *), unsigned long long *host) {
     if (e == cudaSuccess) e = cudaMemcpy(host, d, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
     cudaFree(d);
     return e == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int ht_selftest_sincos(unsigned long long *host_out) {
+    return run([](unsigned long long *d) { k_sincos<<<148 * 8, 256>>>(d); }, host_out);
+}
+extern "C" int ht_selftest_half_turn(unsigned long long *host_out) {
+    return run([](unsigned long long *d) { k_half_turn<<<1, 1>>>(d); }, host_out);
 }
 
 static uint64_t g_n, g_seed;
