@@ -147,6 +147,7 @@ struct Ctx {
     const float *bmag;
     const u32 *bkind;
     u32 culled;
+    float4 *win;    // shared, this thread's 2 float4: the local ray of a bounded scan's winner
 };
 HT_D bool is_repeat(const Ctx &c) { return c.hasher == c.prev; }
 HT_D void hash_usize(Ctx &c, u32 x) { const u32 h = c.hasher; c.hasher = x + (h << 6) + (h << 16) - h; }
@@ -186,9 +187,7 @@ HT_D V3 normalize_q(V3 a) { return normalize3(a); }
 HT_D Q4 mo_apply_pos(const Mo &m, Q4 p) {   // mo_apply_q (transform/moebius.cc:20-25)
     Q4 u = q_addc(cq_mul(m.a, p), m.b);
     Q4 d = q_addc(cq_mul(m.c, p), m.d);
-    float d2 = dot4(d, d);
-    Q4 di = q4(d.x / d2, (-d.y) / d2, (-d.z) / d2, (-d.w) / d2);
-    return q_mul(u, di);
+    return q_mul(u, q_inverse(d));
 }
 struct Moebius {
     typedef Mo V;
@@ -328,7 +327,7 @@ template <class M> struct EuMapOps {
 };
 template <class M> struct MapOps : EuMapOps<M> {};
 template <> struct MapOps<Moebius> {
-    HT_D static void ray(const Mo &m, Q4 &p, Q4 &v) { Moebius::ray(m, p, v); }
+    HT_D static void ray(const Mo &m, Q4 &p, Q4 &v) { ray_cold(m, p, v); }
     HT_D static void view(const Mo &m, Q4 &p, Q4 &v) { Moebius::view(m, p, v); }
     // The same map through one out-of-line copy, for the once-per-hop paths (the winner's
     // full detection, the interaction): only the distance scan keeps an inlined copy.
@@ -366,50 +365,65 @@ template <class G, class V, class M> struct MappedView {   // Mapped{phantom, ma
 // ============================================================================ shapes
 // detect(self, ctx, normal, light) -> distance (> -EPS on a hit); on a hit the light's ray
 // starts at the hit point.
-struct PlaneHy {   // shape/hy/plane.cc:4-37
+// The two hyperbolic shape tests (shape/hy/plane.cc:4-37, horosphere.cc:4-34) up to the hit
+// point: x of the hit distance (hy_x), or -1 on a miss.
+struct ShapeHit { float x; Q4 h; };   // x of the hit distance (-1: none), the hit point
+HT_D float plane_hy_x(Q4 p, Q4 d, Q4 &h) {
+    const float pd = dot4(p, d);
+    if (fabsf(pd) < EPSF) return -1.0f;
+    const float s = 1.0f - dot4(p, p);
+    const float t = s / (2.0f * pd);
+    if (t < -EPSF) return -1.0f;
+    const float hx = p.x + d.x * t, hy = p.y + d.y * t;
+    const float pxy2 = dot2(hx, hy, hx, hy);
+    if (pxy2 > 1.0f) return -1.0f;
+    h = q4(hx, hy, sqrtf(1.0f - pxy2), 0.0f);
+    return hy_x(p, h);
+}
+HT_D float horosphere_x(Q4 p, Q4 d, bool repeat, Q4 &h) {
+    const float dxy = sqrtf(dot2(d.x, d.y, d.x, d.y));
+    if (p.z < dxy) return -1.0f;
+    const float dt = sqrtf(p.z * p.z - dxy * dxy);
+    float t = p.z * d.z - dt;
+    const float w = repeat ? EPSF : -EPSF;
+    if (t < w) {
+        t += 2.0f * dt;
+        if (t < w) return -1.0f;
+    }
+    t /= dxy * dxy;
+    h = q4(p.x + d.x * t, p.y + d.y * t, 1.0f, 0.0f);
+    return hy_x(p, h);
+}
+// One test of either shape, out of line: every variant of a choice and both steps of a scan
+// (distances, then the winner) share one copy of its code.
+__device__ __noinline__ ShapeHit shape_hy_test(u32 kind, bool repeat, Q4 p, Q4 d) {
+    ShapeHit r;
+    r.h = p;
+    r.x = -1.0f;
+    if (kind != 0u) r.x = horosphere_x(p, d, repeat, r.h);
+    else if (!repeat) r.x = plane_hy_x(p, d, r.h);   // a geodesic plane is never hit twice in a row
+    return r;
+}
+template <int W, bool F> HT_D float shape_hy_detect(u32 kind, Ctx &c, Q4 &normal, Light<Hy> &l) {
+    const ShapeHit r = shape_hy_test(kind, is_repeat(c), l.p, l.v);
+    if (r.x == -1.0f) return -1.0f;
+    if (F) {
+        l.v = hy_dir_at(l.p, l.v, r.h);
+        l.p = r.h;
+        normal = kind == 0u ? q4(-r.h.x, -r.h.y, -r.h.z, -r.h.w) : q4(0.0f, 0.0f, -1.0f, 0.0f);
+    }
+    return hy_dist_from_x(r.x);
+}
+struct PlaneHy {
     template <int W> __host__ __device__ static constexpr Lay lay() { return Lay{0u, 1u}; }
     template <int W, bool F = true> HT_D static float detect(Ptr, Ctx &c, Q4 &normal, Light<Hy> &l) {
-        if (is_repeat(c)) return -1.0f;
-        const Q4 p = l.p, d = l.v;
-        const float pd = dot4(p, d);
-        if (fabsf(pd) < EPSF) return -1.0f;
-        const float s = 1.0f - dot4(p, p);
-        const float t = s / (2.0f * pd);
-        if (t < -EPSF) return -1.0f;
-        const float hx = p.x + d.x * t, hy = p.y + d.y * t;
-        const float pxy2 = dot2(hx, hy, hx, hy);
-        if (pxy2 > 1.0f) return -1.0f;
-        const Q4 h = q4(hx, hy, sqrtf(1.0f - pxy2), 0.0f);
-        if (F) {
-            l.p = h;
-            l.v = hy_dir_at(p, d, h);
-            normal = q4(-h.x, -h.y, -h.z, -h.w);
-        }
-        return hy_distance(p, h);
+        return shape_hy_detect<W, F>(0u, c, normal, l);
     }
 };
-struct Horosphere {   // shape/hy/horosphere.cc:4-34
+struct Horosphere {
     template <int W> __host__ __device__ static constexpr Lay lay() { return Lay{0u, 1u}; }
     template <int W, bool F = true> HT_D static float detect(Ptr, Ctx &c, Q4 &normal, Light<Hy> &l) {
-        const bool repeat = is_repeat(c);
-        const Q4 p = l.p, d = l.v;
-        const float dxy = sqrtf(dot2(d.x, d.y, d.x, d.y));
-        if (p.z < dxy) return -1.0f;
-        const float dt = sqrtf(p.z * p.z - dxy * dxy);
-        float t = p.z * d.z - dt;
-        const float w = repeat ? EPSF : -EPSF;
-        if (t < w) {
-            t += 2.0f * dt;
-            if (t < w) return -1.0f;
-        }
-        t /= dxy * dxy;
-        const Q4 h = q4(p.x + d.x * t, p.y + d.y * t, 1.0f, 0.0f);
-        if (F) {
-            l.p = h;
-            l.v = hy_dir_at(p, d, h);
-            normal = q4(0.0f, 0.0f, -1.0f, 0.0f);
-        }
-        return hy_distance(p, h);
+        return shape_hy_detect<W, F>(1u, c, normal, l);
     }
 };
 struct PlaneEu {   // shape/eu/plane.cc:3-21
@@ -501,6 +515,7 @@ template <class G, class S> struct ShapeVec {   // shape/vector.inl
         const u32 orig = c.hasher;
         float min_dist = -1.0f;
         u32 min_index = 0, min_hasher = orig;
+#pragma unroll 1
         for (u32 i = 0; i < n; ++i) {
             Light<G> cur = l;
             typename G::Dir cn;
@@ -669,15 +684,6 @@ struct GradBg {   // {direction, colors[2], power} (background/basic.rs:54-58), 
 // detect(self, ctx, cache, light) -> distance; interact(self, ctx, cache, light, emission).
 template <class G> struct NormalCache { typename G::Dir normal; };
 
-// A material's interaction out of line: one copy per material type however many variants of
-// an object choice share it (the tiled objects call it; each would otherwise inline it).
-// Measured on the hy.rs example type: +9 %; a plain covered object keeps it inline (one copy
-// anyway, and the call costs the eu.rs type 8 %).
-template <class M, int W>
-__device__ __noinline__ bool material_interact_shared(Ptr m, Ctx &c, V3 n, LightLocal &l, Col &e) {
-    return M::template interact<W>(m, c, n, l, e);
-}
-
 template <class G, class S, class M> struct Covered {   // {material, shape} (object/covered.rs:12-18)
     typedef NormalCache<G> Cache;
     template <int W> __host__ __device__ static constexpr Lay lay() { return Rec<W, Zst, M, S>::lay(); }
@@ -706,6 +712,11 @@ template <class G, class O, class M> struct MappedObject {   // object/mapped.in
         if (F) MapOps<M>::ray_cold(m, l.p, l.v);
         return dist;
     }
+    // detect<W, true> from the local ray on (the light already mapped in).
+    template <int W> HT_D static void detect_local(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
+        O::template detect<W, true>(self + Rec<W, Zst, M, O>::off(2), c, cache, l);
+        MapOps<M>::ray_cold(M::load(self + Rec<W, Zst, M, O>::off(1)), l.p, l.v);
+    }
     template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<G> &l, Col &e) {
         const typename M::V m = M::load(self + Rec<W, Zst, M, O>::off(1));
         MapOps<M>::ray_cold(M::inverse(m), l.p, l.v);
@@ -727,7 +738,7 @@ template <class G, class O> struct ObjectVec {   // object/vector.inl
         return n;
     }
     template <int W, bool F = true> HT_D static float detect(Ptr self, Ctx &c, Cache &cache, Light<G> &l);
-    template <int W, bool F> HT_D static float detect_culled(Ptr self, Ctx &c, Cache &cache, Light<G> &l);
+    template <int W, bool F> HT_D static float detect_bounded(Ptr self, Ctx &c, Cache &cache, Light<G> &l);
     template <int W, bool F = true> HT_D static float detect_all(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
         constexpr u32 stride = O::template lay<W>().size;
         constexpr u32 head = upm((u32)W, O::template lay<W>().align);
@@ -739,6 +750,7 @@ template <class G, class O> struct ObjectVec {   // object/vector.inl
         const u32 orig = c.hasher;
         float min_dist = -1.0f;
         u32 min_index = 0, min_hasher = orig;
+#pragma unroll 1
         for (u32 i = 0; i < n; ++i) {
             Light<G> cur = l;
             typename O::Cache cc;
@@ -767,47 +779,36 @@ template <class G, class O> struct ObjectVec {   // object/vector.inl
     }
 };
 
-// ObjectChoice: one cache per variant (objects/src/object/choice.rs: ChoiceCache).
+// ObjectChoice: one cache per variant (objects/src/object/choice.rs: ChoiceCache), or one for
+// all of them when every variant's is a NormalCache (ChoiceTraits).
 template <class... O> struct CacheTuple;
 template <> struct CacheTuple<> {};
 template <class O0, class... O> struct CacheTuple<O0, O...> { typename O0::Cache head; CacheTuple<O...> tail; };
+template <class O0, class... O> HT_D typename O0::Cache &cache_head(CacheTuple<O0, O...> &c) { return c.head; }
+template <class O0, class... O> HT_D CacheTuple<O...> &cache_tail(CacheTuple<O0, O...> &c) { return c.tail; }
+template <class G> HT_D NormalCache<G> &cache_head(NormalCache<G> &c) { return c; }
+template <class G> HT_D NormalCache<G> &cache_tail(NormalCache<G> &c) { return c; }
 template <class G, class... O> struct ObjectChoiceImpl;
 template <class G> struct ObjectChoiceImpl<G> {
-    template <int W, bool F = true> HT_D static float detect(u32, Ptr, Ctx &, CacheTuple<> &, Light<G> &) { return -1.0f; }
-    template <int W> HT_D static bool interact(u32, Ptr, Ctx &, CacheTuple<> &, Light<G> &, Col &) { return false; }
+    template <int W, bool F, class C> HT_D static float detect(u32, Ptr, Ctx &, C &, Light<G> &) { return -1.0f; }
+    template <int W, class C> HT_D static bool interact(u32, Ptr, Ctx &, C &, Light<G> &, Col &) { return false; }
 };
 template <class G, class O0, class... O> struct ObjectChoiceImpl<G, O0, O...> {
-    template <int W, bool F = true> HT_D static float detect(u32 i, Ptr pay, Ctx &c, CacheTuple<O0, O...> &cache, Light<G> &l) {
-        if (i == 0) return O0::template detect<W, F>(pay, c, cache.head, l);
-        return ObjectChoiceImpl<G, O...>::template detect<W, F>(i - 1, pay, c, cache.tail, l);
+    template <int W, bool F, class C> HT_D static float detect(u32 i, Ptr pay, Ctx &c, C &cache, Light<G> &l) {
+        if (i == 0) return O0::template detect<W, F>(pay, c, cache_head(cache), l);
+        return ObjectChoiceImpl<G, O...>::template detect<W, F>(i - 1, pay, c, cache_tail(cache), l);
     }
-    template <int W> HT_D static bool interact(u32 i, Ptr pay, Ctx &c, CacheTuple<O0, O...> &cache, Light<G> &l, Col &e) {
-        if (i == 0) return O0::template interact<W>(pay, c, cache.head, l, e);
-        return ObjectChoiceImpl<G, O...>::template interact<W>(i - 1, pay, c, cache.tail, l, e);
-    }
-};
-template <class G, class... O> struct ObjectChoice {   // object/choice/impl.inl
-    typedef CacheTuple<O...> Cache;
-    template <int W> __host__ __device__ static constexpr Lay lay() { return Enum<W, O...>::lay(); }
-    template <int W, bool F = true> HT_D static float detect(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
-        return ObjectChoiceImpl<G, O...>::template detect<W, F>(ldusize<W>(self), self + Enum<W, O...>::payload(), c, cache, l);
-    }
-    template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<G> &l, Col &e) {
-        return ObjectChoiceImpl<G, O...>::template interact<W>(ldusize<W>(self), self + Enum<W, O...>::payload(), c, cache, l, e);
+    template <int W, class C> HT_D static bool interact(u32 i, Ptr pay, Ctx &c, C &cache, Light<G> &l, Col &e) {
+        if (i == 0) return O0::template interact<W>(pay, c, cache_head(cache), l, e);
+        return ObjectChoiceImpl<G, O...>::template interact<W>(i - 1, pay, c, cache_tail(cache), l, e);
     }
 };
-
 // ---------------------------------------------------------------- tiled hyperbolic objects
 // Tilings (objects/src/object/tiling.rs) and their constants. The pentagonal tilings use
 // fixed Moebius maps and directions that the reference recomputes in float on every call
 // (object/hy/tiled_plane/impl.inl:50-110); here they are computed once per module by
 // tiling_init with the same float operations (transcendentals in FP64, rounded once) and
 // read from global memory.
-struct TilingUniform {};
-struct TilingSquare {};
-struct TilingHexagonal {};
-struct TilingPentagonal {};
-struct TilingPentastar {};
 
 struct PentaTables {
     float Q, S, L, K;
@@ -878,18 +879,6 @@ template <class M, class K, int N> struct TiledFields {   // {tiling, materials,
     struct Mats { template <int W> __host__ __device__ static constexpr Lay lay() { return Arr<N>::template lay<M, W>(); } };
     template <int W> using R = Rec<W, Zst, Mats, M, F32, F32>;
 };
-// Interaction of a tiled object: material chosen from the local hit point, then the
-// covered-object interaction (light to local, material, update).
-template <int W, class M>
-HT_D bool tiled_interact(Ptr material, Ctx &c, const Q4 &normal, Light<Hy> &l, Col &e) {
-    LightLocal ll;
-    ll.k = l.k;
-    ll.v = Hy::to_local(l.p, l.v);
-    const bool ret = material_interact_shared<M, W>(material, c, Hy::to_local(l.p, normal), ll, e);
-    l.v = Hy::from_local(l.p, ll.v);
-    l.k = ll.k;
-    return ret;
-}
 // The cell of a pentagonal / pentastar tiling (object/hy/tiled_plane/impl.inl:48-137): 0 / 1
 // the cell's material, 2 the border; `one` when the object has a single material. One
 // out-of-line copy for both tilings, its reflection loop kept rolled (instruction-cache
@@ -933,31 +922,6 @@ __device__ __noinline__ u32 penta_cell(float br, Q4 p, bool star, bool one) {
     return (w || one) ? 0u : 1u;
 }
 
-template <class M, class K, int N> struct TiledPlane {   // object/hy/tiled_plane/impl.inl
-    typedef NormalCache<Hy> Cache;
-    template <int W> using R = typename TiledFields<M, K, N>::template R<W>;
-    template <int W> __host__ __device__ static constexpr Lay lay() { return R<W>::lay(); }
-    template <int W, bool F = true> HT_D static float detect(Ptr, Ctx &c, Cache &cache, Light<Hy> &l) {
-        ++c.tests;
-        return PlaneHy::detect<W, F>(nullptr, c, cache.normal, l);
-    }
-    template <int W> HT_D static u32 cell(Ptr self, Q4 p) {   // 0 / 1: materials, 2: border
-        return penta_cell(ldf(self + R<W>::off(4)), p, K::star, N < 2);
-    }
-    template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<Hy> &l, Col &e) {
-        constexpr u32 msz = M::template lay<W>().size;
-        Ptr mat = self + R<W>::off(1);
-        if (K::penta) {
-            const u32 k = cell<W>(self, l.p);
-            mat = k == 2u ? self + R<W>::off(2) : self + R<W>::off(1) + k * msz;
-        }
-        return tiled_interact<W, M>(mat, c, cache.normal, l, e);
-    }
-};
-struct PlaneUniform { static constexpr bool penta = false, star = false; };
-struct PlanePentagonal { static constexpr bool penta = true, star = false; };
-struct PlanePentastar { static constexpr bool penta = true, star = true; };
-
 // (int)x of a float as the reference's host build converts it (x86 cvttss2si: out of range
 // and NaN give INT_MIN); in range it truncates like C.
 HT_D int f2i(float x) {
@@ -966,24 +930,29 @@ HT_D int f2i(float x) {
 }
 HT_D int remi(int a, int b) { return ((a % b) + b) % b; }   // math.hh rem
 
-struct HoroUniform { static constexpr int kind = 0; };
-struct HoroSquare { static constexpr int kind = 1; };
-struct HoroHexagonal { static constexpr int kind = 2; };
-template <class M, class K, int N> struct TiledHorosphere {   // object/hy/tiled_horosphere/impl.inl
-    typedef NormalCache<Hy> Cache;
-    template <int W> using R = typename TiledFields<M, K, N>::template R<W>;
-    template <int W> __host__ __device__ static constexpr Lay lay() { return R<W>::lay(); }
-    template <int W, bool F = true> HT_D static float detect(Ptr, Ctx &c, Cache &cache, Light<Hy> &l) {
-        ++c.tests;
-        return Horosphere::detect<W, F>(nullptr, c, cache.normal, l);
-    }
-    template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<Hy> &l, Col &e) {
-        int material_no = 0;
-        bool border = false;
-        const float cell_size = ldf(self + R<W>::off(3));
-        const float br = ldf(self + R<W>::off(4)) / cell_size;
-        const float gx = l.p.x, gy = l.p.y;
-        if (K::kind == 1) {
+// A tiled object's tiling as its variant describes it (materials at `mats`, n of them).
+enum TilingKind : u32 { TILING_UNIFORM, TILING_PENTA, TILING_SQUARE, TILING_HEXA };
+struct Tiling {
+    u32 kind;
+    int n;
+    bool star;
+    float cell_size, border_width;
+    Ptr mats, border;
+};
+// The material at the local hit point p (object/hy/tiled_plane/impl.inl:48-137,
+// object/hy/tiled_horosphere/impl.inl).
+template <int W, class M> HT_D Ptr tiling_material(const Tiling &q, Q4 p) {
+    int material_no = 0;
+    bool border = false;
+    if (q.kind == TILING_PENTA) {
+        const u32 k = penta_cell(q.border_width, p, q.star, q.n < 2);
+        border = k == 2u;
+        material_no = (int)k;
+    } else if (q.kind != TILING_UNIFORM) {
+        const float cell_size = q.cell_size;
+        const float br = q.border_width / cell_size;
+        const float gx = p.x, gy = p.y;
+        if (q.kind == TILING_SQUARE) {
             const float vx = gx / cell_size, vy = gy / cell_size;
             const float kx = floorf(vx), ky = floorf(vy);
             const float fx = vx - kx, fy = vy - ky;
@@ -993,7 +962,7 @@ template <class M, class K, int N> struct TiledHorosphere {   // object/hy/tiled
                 const int hx = remi(f2i(kx), 2), hy = remi(f2i(ky), 2);
                 material_no = 3 * hy - 2 * hx * hy + hx;
             }
-        } else if (K::kind == 2) {
+        } else {
             const float r3 = sqrtf(3.0f);
             const float bxx = 2.0f / r3, bxy = 0.0f;
             const float byx = -1.0f / r3, byy = 1.0f;
@@ -1012,9 +981,111 @@ template <class M, class K, int N> struct TiledHorosphere {   // object/hy/tiled
                 material_no = 2 * hx + hy;
             }
         }
-        constexpr u32 msz = M::template lay<W>().size;
-        const Ptr mat = border ? self + R<W>::off(2) : self + R<W>::off(1) + (u32)remi(material_no, N) * msz;
-        return tiled_interact<W, M>(mat, c, cache.normal, l, e);
+        material_no = remi(material_no, q.n);
+    }
+    return border ? q.border : q.mats + (u32)material_no * M::template lay<W>().size;
+}
+// Interaction of a tiled object: material chosen from the local hit point, then the
+// covered-object interaction (light to local, material, update).
+template <int W, class M>
+HT_D bool tiled_interact(Ptr material, Ctx &c, const Q4 &normal, Light<Hy> &l, Col &e) {
+    LightLocal ll;
+    ll.k = l.k;
+    ll.v = Hy::to_local(l.p, l.v);
+    const bool ret = M::template interact<W>(material, c, Hy::to_local(l.p, normal), ll, e);
+    l.v = Hy::from_local(l.p, ll.v);
+    l.k = ll.k;
+    return ret;
+}
+// K: PlaneUniform, PlanePentagonal, PlanePentastar
+template <class M, class K, int N> struct TiledPlane {   // object/hy/tiled_plane/impl.inl
+    typedef NormalCache<Hy> Cache;
+    template <int W> using R = typename TiledFields<M, K, N>::template R<W>;
+    template <int W> __host__ __device__ static constexpr Lay lay() { return R<W>::lay(); }
+    template <int W, bool F = true> HT_D static float detect(Ptr, Ctx &c, Cache &cache, Light<Hy> &l) {
+        ++c.tests;
+        return PlaneHy::detect<W, F>(nullptr, c, cache.normal, l);
+    }
+    template <int W> HT_D static void tiling(Ptr self, Tiling &q) {
+        q.kind = K::penta ? TILING_PENTA : TILING_UNIFORM;
+        q.n = N;
+        q.star = K::star;
+        q.border_width = ldf(self + R<W>::off(4));
+        q.mats = self + R<W>::off(1);
+        q.border = self + R<W>::off(2);
+    }
+    template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<Hy> &l, Col &e) {
+        Tiling q;
+        tiling<W>(self, q);
+        return tiled_interact<W, M>(tiling_material<W, M>(q, l.p), c, cache.normal, l, e);
+    }
+};
+struct PlaneUniform { static constexpr bool penta = false, star = false; };
+struct PlanePentagonal { static constexpr bool penta = true, star = false; };
+struct PlanePentastar { static constexpr bool penta = true, star = true; };
+
+struct HoroUniform { static constexpr TilingKind kind = TILING_UNIFORM; };
+struct HoroSquare { static constexpr TilingKind kind = TILING_SQUARE; };
+struct HoroHexagonal { static constexpr TilingKind kind = TILING_HEXA; };
+template <class M, class K, int N> struct TiledHorosphere {   // object/hy/tiled_horosphere/impl.inl
+    typedef NormalCache<Hy> Cache;
+    template <int W> using R = typename TiledFields<M, K, N>::template R<W>;
+    template <int W> __host__ __device__ static constexpr Lay lay() { return R<W>::lay(); }
+    template <int W, bool F = true> HT_D static float detect(Ptr, Ctx &c, Cache &cache, Light<Hy> &l) {
+        ++c.tests;
+        return Horosphere::detect<W, F>(nullptr, c, cache.normal, l);
+    }
+    template <int W> HT_D static void tiling(Ptr self, Tiling &q) {
+        q.kind = K::kind;
+        q.n = N;
+        q.star = false;
+        q.cell_size = ldf(self + R<W>::off(3));
+        q.border_width = ldf(self + R<W>::off(4));
+        q.mats = self + R<W>::off(1);
+        q.border = self + R<W>::off(2);
+    }
+    template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<Hy> &l, Col &e) {
+        Tiling q;
+        tiling<W>(self, q);
+        return tiled_interact<W, M>(tiling_material<W, M>(q, l.p), c, cache.normal, l, e);
+    }
+};
+
+// What an object choice can do once for all variants: `plain` when every variant is a geodesic
+// plane or a horosphere whose detection reads none of its bytes (BoundKind), `tiled` when every
+// variant is a tiled object of one material type. A warp's lanes hit objects of all variants, and
+// a dispatch that interacts inside each variant runs the tiling cell and the material once per
+// variant. With one scan for all variants that keeps the winner's local ray (detect_bounded) and
+// this: hy.rs example 5.24 -> 3.71 ms, 64 random tiled objects at 1080p 44.2 -> 30.7 ms.
+template <class... O> struct ChoiceTraits;
+template <class G, class... O> struct ObjectChoice {   // object/choice/impl.inl
+    typedef ChoiceTraits<O...> T;
+    typedef typename T::Cache Cache;
+    template <int W> __host__ __device__ static constexpr Lay lay() { return Enum<W, O...>::lay(); }
+    template <int W, bool F = true> HT_D static float detect(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
+        const u32 i = ldusize<W>(self);
+        if constexpr (T::plain) {
+            const u32 kind = T::kind(i);
+            if (kind > 1u) return -1.0f;
+            ++c.tests;
+            return shape_hy_detect<W, F>(kind, c, cache.normal, l);
+        } else {
+            return ObjectChoiceImpl<G, O...>::template detect<W, F>(i, self + Enum<W, O...>::payload(), c, cache, l);
+        }
+    }
+    template <int W> HT_D static bool interact(Ptr self, Ctx &c, Cache &cache, Light<G> &l, Col &e) {
+        const u32 i = ldusize<W>(self);
+        const Ptr payload = self + Enum<W, O...>::payload();
+        if constexpr (T::tiled) {
+            // each variant only says what its tiling is; the cell and the material run once for
+            // all of a warp's lanes (the example scene's shading: see render_generic)
+            Tiling q;
+            if (!T::template tiling<W>(i, payload, q)) return false;
+            return tiled_interact<W, typename T::Material>(tiling_material<W, typename T::Material>(q, l.p), c,
+                                                           cache.normal, l, e);
+        } else {
+            return ObjectChoiceImpl<G, O...>::template interact<W>(i, payload, c, cache, l, e);
+        }
     }
 };
 
@@ -1056,6 +1127,37 @@ template <class... S> struct BoundKind<ShapeChoice<Hy, S...>> {
 template <class... O> struct BoundKind<ObjectChoice<Hy, O...>> {
     static constexpr int kind = VariantKind<O...>::fixed ? 2 : -1;
     template <int W> HT_D static u32 of(Ptr self) { return kind == 2 ? VariantKind<O...>::of(ldusize<W>(self)) : 2u; }
+};
+
+template <bool B, class X, class Y> struct Select { typedef X T; };
+template <class X, class Y> struct Select<false, X, Y> { typedef Y T; };
+template <class O> struct TiledOf { static constexpr bool ok = false; typedef Zst Material; };
+template <class M, class K, int N> struct TiledOf<TiledPlane<M, K, N>> { static constexpr bool ok = true; typedef M Material; };
+template <class M, class K, int N> struct TiledOf<TiledHorosphere<M, K, N>> { static constexpr bool ok = true; typedef M Material; };
+template <class X, class Y> struct SameType { static constexpr bool ok = false; };
+template <class X> struct SameType<X, X> { static constexpr bool ok = true; };
+template <class M, class... O> struct AllTiled { static constexpr bool ok = true; };
+template <class M, class O0, class... O> struct AllTiled<M, O0, O...> {
+    static constexpr bool ok = TiledOf<O0>::ok && SameType<M, typename TiledOf<O0>::Material>::ok && AllTiled<M, O...>::ok;
+};
+template <int W, class... O> struct TilingOf { HT_D static bool get(u32, Ptr, Tiling &) { return false; } };
+template <int W, class O0, class... O> struct TilingOf<W, O0, O...> {
+    HT_D static bool get(u32 i, Ptr payload, Tiling &q) {
+        if (i != 0) return TilingOf<W, O...>::get(i - 1, payload, q);
+        O0::template tiling<W>(payload, q);
+        return true;
+    }
+};
+template <> struct ChoiceTraits<> {
+    static constexpr bool plain = false, tiled = false;
+    typedef CacheTuple<> Cache;
+};
+template <class O0, class... O> struct ChoiceTraits<O0, O...> {
+    typedef typename TiledOf<O0>::Material Material;
+    static constexpr bool plain = VariantKind<O0, O...>::fixed, tiled = plain && AllTiled<Material, O0, O...>::ok;
+    typedef typename Select<plain, NormalCache<Hy>, CacheTuple<O0, O...>>::T Cache;
+    HT_D static u32 kind(u32 i) { return VariantKind<O0, O...>::of(i); }
+    template <int W> HT_D static bool tiling(u32 i, Ptr payload, Tiling &q) { return TilingOf<W, O0, O...>::get(i, payload, q); }
 };
 
 // A vector of Moebius-mapped objects of a known shape gets distance bounds: one world-space
@@ -1103,41 +1205,44 @@ HT_D u32 stage_vec_bounds(Ptr self, Ptr end, float4 *rec, float *mag, u32 *kind)
 
 template <class G, class O> template <int W, bool F>
 HT_D float ObjectVec<G, O>::detect(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
-    if constexpr (VecBounds<G, O>::ok) {
-        if (c.bvec == self) return detect_culled<W, F>(self, c, cache, l);
-    }
-    return detect_all<W, F>(self, c, cache, l);
+    if constexpr (VecBounds<G, O>::ok) return detect_bounded<W, F>(self, c, cache, l);
+    else return detect_all<W, F>(self, c, cache, l);
 }
 
-// The scan of ObjectVec::detect_all with the distance bounds of the hand-written hyperbolic
-// kernel (ht_trace.cuh hop_hy): an upper estimate of the nearest sure crossing among the first
-// 32 elements sets a threshold before the first exact test, each chunk of 32 elements is
+// The scan of ObjectVec::detect_all for vectors of Moebius-mapped planes and horospheres. The
+// elements are visited in index order with the shape test of their kind directly (one copy of
+// the ray map and of the tests for all variants), the logarithm taken only where x = cosh of the
+// distance can win (hy_dist_from_x is non-decreasing), and the winner's local ray is kept for its
+// full detection: the same operations on the same values as detect_all, so the same bits.
+// When the kernel staged the vector's distance bounds, it culls as the hand-written hyperbolic
+// kernel does (ht_trace.cuh hop_hy): an upper estimate of the nearest sure crossing among the
+// first 32 elements sets a threshold before the first exact test, each chunk of 32 elements is
 // culled by the point bound (warp-uniform) and the ray-aware bound (per lane), and the
-// survivors are tested in index order with the threshold tightening on every nearer hit. The
-// elements are visited in index order, so the reference's comparison (object/vector.inl:37-50)
-// is unchanged; culling only skips elements that cannot be nearer than the threshold.
+// survivors are tested with the threshold tightening on every nearer hit. Culling only skips
+// elements that cannot be nearer than the threshold.
 template <class G, class O> template <int W, bool F>
-HT_D float ObjectVec<G, O>::detect_culled(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
+HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
+    typedef VecBounds<G, O> B;
     constexpr u32 stride = O::template lay<W>().size;
     constexpr u32 head = upm((u32)W, O::template lay<W>().align);
     const u32 n = count<W>(self, c);
-    const u32 orig = c.hasher;
+    const u32 orig = c.hasher, h0 = (orig << 6) + (orig << 16) - orig;   // hash_usize: element i's hash is i + h0
     const Q4 p = l.p, v = l.v;
-    const bool can = cull_point_ok(p);
+    const bool staged = c.bvec == self, can = staged && cull_point_ok(p);
     const BoundRay br = bound_ray(p, v);
     Cull cull = cull_none();
     if (can) {
         float best = __int_as_float(0x7f800000);
         const u32 ne = n < 32u ? n : 32u;
-        for (u32 i = 0; i < ne; ++i) {   // warp-uniform: broadcast loads
-            const u32 h = i + (orig << 6) + (orig << 16) - orig;   // the element's hash (hash_usize)
-            best = fminf(best, sure_crossing_e2(bound_fw(c.brec[i], c.bmag[i], br), c.bkind[i], h == c.prev, br.t));
-        }
+#pragma unroll 1
+        for (u32 i = 0; i < ne; ++i)   // warp-uniform: broadcast loads
+            best = fminf(best, sure_crossing_e2(bound_fw(c.brec[i], c.bmag[i], br), c.bkind[i], i + h0 == c.prev, br.t));
         if (best < __int_as_float(0x7f800000)) cull = cull_from_dist(dist_from_e2(best));
     }
     PointCut kp = point_cut(0, br.t, cull), kh = point_cut(1, br.t, cull);
-    float min_dist = -1.0f;
-    u32 min_index = 0, min_hasher = orig, tested = 0;
+    float min_dist = -1.0f, min_x = __int_as_float(0x7f800000);
+    u32 min_index = 0, tested = 0;
+#pragma unroll 1
     for (u32 c0 = 0; c0 < n; c0 += 32) {
         const u32 cn = n - c0 < 32u ? n - c0 : 32u;
         u32 mask = cn == 32u ? 0xFFFFFFFFu : (1u << cn) - 1u;
@@ -1161,29 +1266,39 @@ HT_D float ObjectVec<G, O>::detect_culled(Ptr self, Ctx &c, Cache &cache, Light<
             mask &= mask - 1;
             if (can && culled_point(c.brec[i], c.bmag[i], br, c.bkind[i] == 0u ? kp : kh)) continue;
             ++tested;
-            Light<G> cur = l;
-            typename O::Cache cc;
-            hash_usize(c, i);
-            const float dist = O::template detect<W, false>(self + head + i * stride, c, cc, cur);
-            if (dist > -EPSF && (min_dist <= -EPSF || dist < min_dist)) {
-                min_dist = dist; min_index = i; min_hasher = c.hasher;
-                cull = cull_from_dist(dist);
-                kp = point_cut(0, br.t, cull);
-                kh = point_cut(1, br.t, cull);
+            const Ptr elem = self + head + i * stride;
+            const u32 kind = staged ? c.bkind[i] : B::template kind_of<W>(elem);
+            if (kind > 1u) continue;   // a choice index out of range takes no variant
+            ++c.tests;
+            const HyRay r = ray_hy_map_call(mo_inverse(B::template map_of<W>(elem)), p, v);
+            const float x = shape_hy_test(kind, i + h0 == c.prev, r.p, r.v).x;
+            if (x >= 1.0f && x <= min_x) {
+                const float dist = hy_dist_from_x(x);
+                if (dist > -EPSF && (min_dist <= -EPSF || dist < min_dist)) {
+                    min_dist = dist; min_x = x; min_index = i;
+                    c.win[0] = make_float4(r.p.x, r.p.y, r.p.z, r.p.w);
+                    c.win[1] = make_float4(r.v.x, r.v.y, r.v.z, r.v.w);
+                    if (staged) {
+                        cull = cull_from_dist(dist);
+                        kp = point_cut(0, br.t, cull);
+                        kh = point_cut(1, br.t, cull);
+                    }
+                }
             }
-            c.hasher = orig;
         }
     }
     c.culled += n - tested;
     if (!(min_dist > -EPSF)) return -1.0f;
+    c.hasher = min_index + h0;
     if (F) {
         const u32 tests = c.tests;
-        hash_usize(c, min_index);
-        O::template detect<W, true>(self + head + min_index * stride, c, cache.inner, l);
+        const float4 a = c.win[0], b = c.win[1];
+        l.p = q4(a.x, a.y, a.z, a.w);
+        l.v = q4(b.x, b.y, b.z, b.w);
+        O::template detect_local<W>(self + head + min_index * stride, c, cache.inner, l);
         c.tests = tests;
         cache.index = min_index;
     }
-    c.hasher = min_hasher;
     return min_dist;
 }
 
@@ -1193,29 +1308,28 @@ template <class G, class V, class O, class B> struct SceneImpl {   // {phantom, 
     typedef O Object;
     typedef G Geometry;
     template <int W> __host__ __device__ static constexpr u32 static_size() { return R<W>::off(3) + O::template lay<W>().size; }
-    // render/scene.inl:16-44 with H = hops; returns the path's emission.
-    template <int W>
-    HT_D static Col sample(Ptr self, Ctx &c, float px, float py, float size, u32 hops, u32 &hops_done, u32 &hits) {
-        Light<G> l = V::template sample<W>(self + R<W>::off(1), c, px, py, size);
+    // render/scene.inl:16-44 in steps: the camera ray, one hop's detection, its interaction
+    // (false when the path ends).
+    template <int W> HT_D static void start(Ptr self, Ctx &c, float px, float py, float size, Light<G> &l, Col &e) {
+        l = V::template sample<W>(self + R<W>::off(1), c, px, py, size);
         l.k.x = 1.0f; l.k.y = 1.0f; l.k.z = 1.0f;
-        Col e; e.x = 0.0f; e.y = 0.0f; e.z = 0.0f;
+        e.x = 0.0f; e.y = 0.0f; e.z = 0.0f;
         c.prev = HASH_NEVER;
-        for (u32 i = 0; i < hops; ++i) {
-            c.hasher = 0u;
-            typename O::Cache cache;
-            ++hops_done;
-            const float dist = O::template detect<W, true>(self + R<W>::off(3), c, cache, l);
-            if (dist > -0.5f) {
-                ++hits;
-                const bool ret = O::template interact<W>(self + R<W>::off(3), c, cache, l, e);
-                if (!ret) break;
-                c.prev = c.hasher;
-            } else {
-                B::template interact<W>(self + R<W>::off(2), c, l, e);
-                break;
-            }
+    }
+    template <int W> HT_D static float detect(Ptr self, Ctx &c, typename O::Cache &cache, Light<G> &l) {
+        c.hasher = 0u;
+        return O::template detect<W, true>(self + R<W>::off(3), c, cache, l);
+    }
+    template <int W>
+    HT_D static bool shade(Ptr self, Ctx &c, typename O::Cache &cache, Light<G> &l, Col &e, float dist, u32 &hits) {
+        if (dist > -0.5f) {
+            ++hits;
+            if (!O::template interact<W>(self + R<W>::off(3), c, cache, l, e)) return false;
+            c.prev = c.hasher;
+            return true;
         }
-        return e;
+        B::template interact<W>(self + R<W>::off(2), c, l, e);
+        return false;
     }
 };
 
@@ -1225,25 +1339,42 @@ template <class G, class O> struct VecElem<ObjectVec<G, O>> { static constexpr b
 
 // ============================================================================ kernel
 // One thread per pixel (render/render.cl:6-27); `passes` samples of the pixel in order, the
-// same float additions as `passes` launches of one pass.
-// Resident 128-thread blocks per SM requested from ptxas (register cap 64): the scan is a
-// chain of dependent FP32 operations, so more resident warps beat the few spilled values
-// (8 blocks measured fastest against 1, 5, 6, 7 on the example scene types).
-#ifndef HTG_MIN_BLOCKS
-#define HTG_MIN_BLOCKS 8
-#endif
+// same float additions as `passes` launches of one pass. Blocks cover tiles of 32 pixels by
+// threads / 32, a warp 8 x 4 of them: the rays of a warp stay closer together than those of 32
+// pixels of a row (hy.rs example scene at 800x600, 16 passes: 6.03 -> 5.23 ms). `tiles` is their
+// number across the canvas, or 0 for blocks of consecutive pixels (canvases that tiles would
+// overhang by much).
+//
+// Launch: the hyperbolic types compile to 60-130 KB of code per kernel, and warps that
+// run through it at their own pace miss the instruction caches all the time (15 to 19 of 20
+// stalls, the schedulers issuing on 28-36 % of cycles). So their blocks are large and go
+// through each hop together: camera rays of the lanes whose path ended, then every lane's
+// detection, then every lane's interaction, with a barrier before each step -- an SM's warps
+// then share the few KB of the step they are in (hy.rs example: 10.3 -> 6.0 ms, 64 random
+// tiled objects at 1080p, 4 passes: 70.3 -> 44.3 ms; threads per block and blocks per SM measured
+// there: 512 x 2 3.71 and 30.7 ms, 256 x 4 4.19 and 30.0, 384 x 2 3.76 and 31.0, 1024 x 1 4.26 and
+// 34.9). A lane starts its next sample in the step after its path ended, so lanes wait for
+// a barrier, not for the block's longest path. The Euclidean types' code (40 KB) fits: there
+// each thread runs its own loops in blocks of 128 (the barriers cost the eu.rs example 13 %).
+template <class Geo> struct Launch { static constexpr u32 threads = 128u, blocks = 8u; };
+template <> struct Launch<Hy> { static constexpr u32 threads = 512u, blocks = 2u; };
+
 template <class Scene, int W>
-__global__ void __launch_bounds__(128, HTG_MIN_BLOCKS) render_generic(Ptr scene, uint64_t scene_size, u32 width, u32 height,
-                                                     u32 hops, u32 passes, u32 flags, float4 *canvas, u32 *seeds,
-                                                     unsigned long long *stats, u32 *err) {
-    const u32 idx = blockIdx.x * 128u + threadIdx.x;
-    u32 samples = 0, hops_done = 0, hits = 0, tests = 0, culled = 0;
+__global__ void __launch_bounds__(Launch<typename Scene::Geometry>::threads, Launch<typename Scene::Geometry>::blocks)
+render_generic(Ptr scene, uint64_t scene_size, u32 width, u32 height, u32 tiles, u32 hops, u32 passes, u32 flags,
+               float4 *canvas, u32 *seeds, unsigned long long *stats, u32 *err) {
     typedef typename Scene::Object Obj;
     typedef typename Scene::Geometry Geo;
-    Ptr bvec = nullptr;
-    const float4 *brec = nullptr;
-    const float *bmag = nullptr;
-    const u32 *bkind = nullptr;
+    Ctx c;
+    c.bvec = nullptr;
+    c.brec = nullptr;
+    c.bmag = nullptr;
+    c.bkind = nullptr;
+    c.win = nullptr;
+    if constexpr (SameType<Geo, Hy>::ok) {
+        __shared__ float4 s_win[2 * Launch<Geo>::threads];
+        c.win = s_win + 2 * threadIdx.x;
+    }
     if constexpr (VecBounds<Geo, typename VecElem<Obj>::T>::ok && VecElem<Obj>::is_vec) {
         // the top-level object vector's distance bounds, staged once per block
         __shared__ float4 s_rec[HTG_BOUND_CAP];
@@ -1253,43 +1384,83 @@ __global__ void __launch_bounds__(128, HTG_MIN_BLOCKS) render_generic(Ptr scene,
         const u32 nb = stage_vec_bounds<Geo, typename VecElem<Obj>::T, W>(vec, scene + scene_size, s_rec, s_mag, s_kind);
         __syncthreads();
         if (nb != 0xFFFFFFFFu) {
-            bvec = vec;
-            brec = s_rec;
-            bmag = s_mag;
-            bkind = s_kind;
+            c.bvec = vec;
+            c.brec = s_rec;
+            c.bmag = s_mag;
+            c.bkind = s_kind;
         }
     }
-    if (idx < width * height) {
-        const u32 x = idx % width, y = idx / width;
-        const float px = (__uint2float_rn(2u * x + 1u) - __uint2float_rn(width)) / __uint2float_rn(height);
-        const float py = (__uint2float_rn(height) - __uint2float_rn(2u * y + 1u)) / __uint2float_rn(height);
-        const float size = 2.0f / __uint2float_rn(height);
-        Ctx c;
-        c.rng = seeds[idx];
-        c.hasher = 0u;
-        c.prev = HASH_NEVER;
-        c.flags = flags;
-        c.tests = 0;
-        c.end = scene + scene_size;
-        c.err = err;
-        c.bvec = bvec;
-        c.brec = brec;
-        c.bmag = bmag;
-        c.bkind = bkind;
-        c.culled = 0;
-        float4 acc = canvas[idx];
-        for (u32 k = 0; k < passes; ++k) {
-            const Col col = Scene::template sample<W>(scene, c, px, py, size, hops, hops_done, hits);
-            acc.x += col.x; acc.y += col.y; acc.z += col.z; acc.w += 1.0f;
-            ++samples;
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    u32 x, y;
+    bool inside;
+    if (tiles) {
+        x = blockIdx.x % tiles * 32u + (warp & 3u) * 8u + (lane & 7u);
+        y = blockIdx.x / tiles * (blockDim.x >> 5) + (warp >> 2) * 4u + (lane >> 3);
+        inside = x < width && y < height;
+    } else {
+        const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+        x = i % width;
+        y = i / width;
+        inside = i < width * height;
+    }
+    const u32 idx = y * width + x;
+    const float px = (__uint2float_rn(2u * x + 1u) - __uint2float_rn(width)) / __uint2float_rn(height);
+    const float py = (__uint2float_rn(height) - __uint2float_rn(2u * y + 1u)) / __uint2float_rn(height);
+    const float size = 2.0f / __uint2float_rn(height);
+    c.rng = inside ? seeds[idx] : 0u;
+    c.hasher = 0u;
+    c.prev = HASH_NEVER;
+    c.flags = flags;
+    c.tests = 0;
+    c.end = scene + scene_size;
+    c.err = err;
+    c.culled = 0;
+    float4 acc = inside ? canvas[idx] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    u32 samples = 0, hops_done = 0, hits = 0;
+    Light<Geo> l;
+    Col e;
+    typename Obj::Cache cache;
+    if constexpr (SameType<Geo, Hy>::ok) {
+        u32 hop = hops;
+        bool active = inside && passes > 0;
+        while (__syncthreads_or(active)) {
+            if (active && hop >= hops) {
+                Scene::template start<W>(scene, c, px, py, size, l, e);
+                hop = 0;
+            }
+            __syncthreads();
+            float dist = -1.0f;
+            if (active) dist = Scene::template detect<W>(scene, c, cache, l);
+            __syncthreads();
+            if (active) {
+                ++hops_done;
+                ++hop;
+                if (!Scene::template shade<W>(scene, c, cache, l, e, dist, hits)) hop = hops;
+                if (hop >= hops) {
+                    acc.x += e.x; acc.y += e.y; acc.z += e.z; acc.w += 1.0f;
+                    ++samples;
+                    active = samples < passes;
+                }
+            }
         }
+    } else if (inside) {
+#pragma unroll 1
+        for (; samples < passes; ++samples) {
+            Scene::template start<W>(scene, c, px, py, size, l, e);
+            for (u32 hop = 0; hop < hops; ++hop) {
+                ++hops_done;
+                const float dist = Scene::template detect<W>(scene, c, cache, l);
+                if (!Scene::template shade<W>(scene, c, cache, l, e, dist, hits)) break;
+            }
+            acc.x += e.x; acc.y += e.y; acc.z += e.z; acc.w += 1.0f;
+        }
+    }
+    if (inside) {
         canvas[idx] = acc;
         seeds[idx] = c.rng;
-        tests = c.tests;
-        culled = c.culled;
     }
     if (stats) {   // samples, hops, object tests the reference makes, hits, tests evaluated
-        unsigned long long v[5] = {samples, hops_done, (unsigned long long)tests + culled, hits, tests};
+        unsigned long long v[5] = {samples, hops_done, (unsigned long long)c.tests + c.culled, hits, c.tests};
         for (int k = 0; k < 5; ++k) {
             for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xFFFFFFFFu, v[k], o);
         }

@@ -144,23 +144,36 @@ struct GenericProgram {
     const void *static_kernel = nullptr;   // built-in: render_generic<Scene, W>
     CUmodule module = nullptr;              // NVRTC: the loaded cubin
     CUfunction kernel = nullptr;
+    unsigned threads = 128;                 // largest block of the kernel (htg::Launch)
+    unsigned num_sms = 148;
     uint64_t min_size = 0;                  // serialized size of the scene without its dynamic part
     std::string type_expr;
 };
+
+static cudaError_t program_sms(unsigned *sms) {
+    int dev = 0, n = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) *sms = (unsigned)n;
+    return e;
+}
 
 int generic_program_create(int recipe, int address_width, GenericProgram **out) {
     GenericProgram *g = new GenericProgram();
     if (recipe == HTC_RECIPE_HY_TILED) {
         g->static_kernel = address_width == 64 ? (const void *)render_generic<SceneHyTiled, 8>
                                                : (const void *)render_generic<SceneHyTiled, 4>;
+        g->threads = Launch<Hy>::threads;
         g->min_size = address_width == 64 ? SceneHyTiled::static_size<8>() : SceneHyTiled::static_size<4>();
     } else {
         g->static_kernel = address_width == 64 ? (const void *)render_generic<SceneEuGradient, 8>
                                                : (const void *)render_generic<SceneEuGradient, 4>;
+        g->threads = Launch<Eu>::threads;
         g->min_size = address_width == 64 ? SceneEuGradient::static_size<8>() : SceneEuGradient::static_size<4>();
     }
     htg_tiling_init<<<1, 1>>>();
     cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = program_sms(&g->num_sms);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         delete g;
@@ -180,7 +193,7 @@ int generic_program_build(const char *type_expr, int address_width, char *log, s
     const int W = address_width == 64 ? 8 : 4;
     std::string src = "#include \"ht_generic.cuh\"\nnamespace htg {\ntypedef " + std::string(type_expr) +
                       " UserScene;\n}\nextern \"C\" __device__ unsigned long long htg_static_size = htg::UserScene::static_size<" +
-                      std::to_string(W) + ">();\n";
+                      std::to_string(W) + ">();\nextern \"C\" __device__ unsigned int htg_threads = htg::Launch<htg::UserScene::Geometry>::threads;\n";
     const std::string kname = "&htg::render_generic<htg::UserScene, " + std::to_string(W) + ">";
     void *prog = nullptr;
     const char *hdr_src[] = {k_header_ht_math, k_header_ht_bound, k_header_ht_generic};
@@ -226,15 +239,18 @@ int generic_program_build(const char *type_expr, int address_width, char *log, s
         delete g;
         return fail(HTC_ERR_CUDA, "loading the compiled scene program failed (CUresult " + std::to_string((int)r) + ")");
     }
-    // The static size of the scene type is a __device__ constant of the module.
-    CUdeviceptr gp = 0;
-    size_t gbytes = 0;
-    if (d.global(&gp, &gbytes, g->module, "htg_static_size") != CUDA_SUCCESS || gbytes != sizeof(uint64_t)) {
+    // The static size of the scene type and its block size are __device__ constants of the module.
+    CUdeviceptr gp = 0, tp = 0;
+    size_t gbytes = 0, tbytes = 0;
+    if (d.global(&gp, &gbytes, g->module, "htg_static_size") != CUDA_SUCCESS || gbytes != sizeof(uint64_t) ||
+        d.global(&tp, &tbytes, g->module, "htg_threads") != CUDA_SUCCESS || tbytes != sizeof(unsigned)) {
         d.unload(g->module);
         delete g;
-        return fail(HTC_ERR_CUDA, "compiled scene program lacks htg_static_size");
+        return fail(HTC_ERR_CUDA, "compiled scene program lacks htg_static_size or htg_threads");
     }
     cudaError_t e = cudaMemcpy(&g->min_size, reinterpret_cast<const void *>(gp), sizeof(uint64_t), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&g->threads, reinterpret_cast<const void *>(tp), sizeof(unsigned), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = program_sms(&g->num_sms);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         d.unload(g->module);
@@ -255,19 +271,30 @@ int generic_render(GenericProgram *g, uint32_t W, uint32_t H, uint32_t hops, uin
                    size_t scene_size, float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, uint32_t *d_err,
                    void *stream) {
     if (scene_size < g->min_size) return fail(HTC_ERR_SCENE, "scene buffer is smaller than the scene type's fixed part");
+    // Smaller blocks while the canvas would leave an SM without a block; a tile of 32 x
+    // (threads / 32) pixels per block where the tiles overhang the canvas by less than an eighth.
     const uint64_t pixels = (uint64_t)W * H;
-    const unsigned blocks = (unsigned)((pixels + 127) / 128);
+    unsigned threads = g->threads;
+    while (threads > 128 && pixels < (uint64_t)threads * g->num_sms) threads /= 2;
+    const unsigned rows = threads / 32;
+    unsigned tiles = (W - 1) / 32 + 1;
+    uint64_t blocks64 = (uint64_t)tiles * ((H - 1) / rows + 1);
+    if (blocks64 * threads > pixels + pixels / 8) {
+        tiles = 0;
+        blocks64 = (pixels + threads - 1) / threads;
+    }
+    const unsigned blocks = (unsigned)blocks64;
     const uint8_t *sc = reinterpret_cast<const uint8_t *>(scene);
     uint64_t ss = scene_size;
     float4 *cv = reinterpret_cast<float4 *>(canvas);
     unsigned long long *st = reinterpret_cast<unsigned long long *>(stats);
-    void *args[] = {(void *)&sc, (void *)&ss, (void *)&W, (void *)&H, (void *)&hops, (void *)&passes,
+    void *args[] = {(void *)&sc, (void *)&ss, (void *)&W, (void *)&H, (void *)&tiles, (void *)&hops, (void *)&passes,
                     (void *)&flags, (void *)&cv, (void *)&seeds, (void *)&st, (void *)&d_err};
     if (g->static_kernel) {
-        HTC_CUDA(cudaLaunchKernel(g->static_kernel, dim3(blocks), dim3(128), args, 0, reinterpret_cast<cudaStream_t>(stream)));
+        HTC_CUDA(cudaLaunchKernel(g->static_kernel, dim3(blocks), dim3(threads), args, 0, reinterpret_cast<cudaStream_t>(stream)));
         return HTC_OK;
     }
-    CUresult r = driver().launch(g->kernel, blocks, 1, 1, 128, 1, 1, 0, reinterpret_cast<CUstream>(stream), args, nullptr);
+    CUresult r = driver().launch(g->kernel, blocks, 1, 1, threads, 1, 1, 0, reinterpret_cast<CUstream>(stream), args, nullptr);
     if (r != CUDA_SUCCESS) return fail(HTC_ERR_CUDA, "cuLaunchKernel failed (CUresult " + std::to_string((int)r) + ")");
     return HTC_OK;
 }
