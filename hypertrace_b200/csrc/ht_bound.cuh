@@ -260,5 +260,78 @@ HT_D float sure_crossing_e2(const BoundFW &b, uint32_t shape, bool plane_repeat,
 // Distance of a crossing from its e^(2 s) bound (the threshold built from it adds 1e-2 margins).
 HT_D float dist_from_e2(float x) { return 0.5f * LN2F * lg2_approx(x); }
 
+// ---------------------------------------------------------------- Euclidean bounds
+// The same idea for unit spheres and planes under rigid maps: world-space tests with wide margins
+// that rule out objects the reference's test cannot report nearer than the best hit so far.
+// Per object one float4, staged once per launch (eu_stage_bound):
+//   sphere  its centre c. With m = c - p, b = m.v, the line passes the centre at a squared
+//           distance q2 = |m|^2 - b^2; the roots are b -+ sqrt(1 - q2). It is missed when q2 > 1,
+//           behind when b < 0 and |m| > 1, and no root is nearer than b - 1.
+//   plane   its normal n (local z) and w = -n.c: h = n.p + w and n.v are the local heights of the
+//           start and the direction; missed when they have one sign, else hit at -h / n.v.
+// Margins: the reference's local ray differs from the exact one by at most about 1e-6 of
+// (|p| + |c|) in position and, for a quaternion whose norm the staging lets pass, 1e-5 in scale;
+// the tests allow 1e-4 |m|^2 + 1.6e-5 |p|_1 + 1e-3 on q2 (|c|_1 <= |p|_1 + 2 |m|), 2e-3 + 8e-6 |p|_1
+// on h (planes with |c|_1 <= 250 only), 2e-5 on n.v, and 1e-4 relative + 1e-3 + 1.6e-5 |p|_1 on
+// distances. Other objects get NaN records, which no test culls; rays whose direction is not of
+// unit length to 2e-5, or that start beyond 10^4, are not culled at all.
+// tests/cull_check/eu_check.c runs them against the full scan on the CPU.
+HT_D float4 eu_stage_bound(const Hom &m, uint32_t shape) {
+    const double w = m.rot.x, x = m.rot.y, y = m.rot.z, z = m.rot.w;
+    const double cx = m.shift.x, cy = m.shift.y, cz = m.shift.z;
+    const double c1 = fabs(cx) + fabs(cy) + fabs(cz);
+    const float nan = __int_as_float(0x7fc00000);
+    if (!(fabs(w * w + x * x + y * y + z * z - 1.0) <= 1e-5 && c1 <= (shape == 0 ? 250.0 : 1e4)))
+        return make_float4(nan, nan, nan, nan);
+    if (shape != 0) return make_float4(m.shift.x, m.shift.y, m.shift.z, 0.0f);
+    const double nx = 2.0 * (x * z + w * y), ny = 2.0 * (y * z - w * x), nz = 1.0 - 2.0 * (x * x + y * y);
+    return make_float4((float)nx, (float)ny, (float)nz, (float)-(nx * cx + ny * cy + nz * cz));
+}
+struct EuBoundRay {
+    V3 p, v;
+    float base;   // 1 + the margin of q2 without its |m|^2 part
+    float dh;     // margin of a plane's h
+    float dd;     // absolute margin of a distance
+    bool can;     // the ray may be culled for
+};
+HT_D EuBoundRay eu_bound_ray(V3 p, V3 v) {
+    EuBoundRay r;
+    r.p = p;
+    r.v = v;
+    const float p1 = fabsf(p.x) + fabsf(p.y) + fabsf(p.z);
+    r.dd = fmaf(1.6e-5f, p1, 1e-3f);
+    r.base = 1.0f + r.dd;
+    r.dh = fmaf(8e-6f, p1, 2e-3f);
+    r.can = p1 <= 1e4f && fabsf(dot3(v, v) - 1.0f) <= 2e-5f;
+    return r;
+}
+// The limit that a hit at distance d sets: objects whose nearest possible hit lies beyond it
+// are culled.
+HT_D float eu_limit(float d, const EuBoundRay &r) { return fmaf(d, 1.0f + 1e-4f, r.dd); }
+// Whether one object is culled; `limit` is lowered when the object is surely hit.
+HT_D bool eu_culled_sphere(float4 rec, const EuBoundRay &r, float &limit) {
+    const float mx = rec.x - r.p.x, my = rec.y - r.p.y, mz = rec.z - r.p.z;
+    const float b = fmaf(mx, r.v.x, fmaf(my, r.v.y, mz * r.v.z));
+    const float mm = fmaf(mx, mx, fmaf(my, my, mz * mz));
+    const float q2 = fmaf(-b, b, mm), top = fmaf(1e-4f, mm, r.base);
+    const bool out = mm > top;
+    if (q2 > top || (b < 0.0f && out) || b - 1.0f > limit) return true;
+    const float s = (2.0f - top) - q2;   // lower bound of 1 - q2
+    if (s > 0.0f && b > 0.0f && out) limit = fminf(limit, eu_limit(fmaf(-(1.0f - 1e-6f), sqrt_approx(s), b), r));
+    return false;
+}
+HT_D bool eu_culled_plane(float4 rec, const EuBoundRay &r, bool repeat, float &limit) {
+    const float h = fmaf(rec.x, r.p.x, fmaf(rec.y, r.p.y, fmaf(rec.z, r.p.z, rec.w)));
+    const float n = fmaf(rec.x, r.v.x, fmaf(rec.y, r.v.y, rec.z * r.v.z));
+    const float hlo = fabsf(h) - r.dh, an = fabsf(n);
+    const bool ahead = (h > 0.0f) != (n > 0.0f);
+    if (repeat || (hlo > 0.0f && ((!ahead && an > 2e-5f) || hlo > limit * (an + 2e-5f)))) return true;
+    if (ahead && hlo > 0.0f && an > 0.01f) limit = fminf(limit, eu_limit((fabsf(h) + r.dh) * rcp_approx(an - 2e-5f) * (1.0f + 1e-6f), r));
+    return false;
+}
+// The far test alone, for a candidate whose turn has come.
+HT_D bool eu_far_sphere(float4 rec, const EuBoundRay &r, float limit) {
+    return fmaf(rec.x - r.p.x, r.v.x, fmaf(rec.y - r.p.y, r.v.y, (rec.z - r.p.z) * r.v.z)) - 1.0f > limit;
+}
 
 }  // namespace ht

@@ -48,7 +48,6 @@ HT_D float dot3(V3 a, V3 b) { float c = 0.0f; c += a.x * b.x; c += a.y * b.y; c 
 HT_D float dot4(Q4 a, Q4 b) {
     float c = 0.0f; c += a.x * b.x; c += a.y * b.y; c += a.z * b.z; c += a.w * b.w; return c;
 }
-HT_D V3 normalize3(V3 a) { float l = sqrtf(dot3(a, a)); return v3(a.x / l, a.y / l, a.z / l); }
 HT_D Q4 normalize4(Q4 a) { float l = sqrtf(dot4(a, a)); return q4(a.x / l, a.y / l, a.z / l, a.w / l); }
 HT_D V3 cross3(V3 a, V3 b) {
     return v3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
@@ -127,7 +126,15 @@ HT_D Q4 qdiv4(Q4 a, const Rcp &r, DivCheck &c) {
     c.least = min(min(c.least, div_word(a.x)), min(min(div_word(a.y), div_word(a.z)), div_word(a.w)));
     return q4(qdiv_unchecked(a.x, r), qdiv_unchecked(a.y, r), qdiv_unchecked(a.z, r), qdiv_unchecked(a.w, r));
 }
-// normalize4 through one correctly rounded reciprocal of the length.
+// normalize3 and normalize4 through one correctly rounded reciprocal of the length.
+static __device__ __noinline__ V3 normalize3_ieee(V3 a) { float l = sqrtf(dot3(a, a)); return v3(a.x / l, a.y / l, a.z / l); }
+HT_D V3 normalize3(V3 a) {
+    DivCheck c = div_check();
+    const Rcp r = rcp_of(sqrtf(dot3(a, a)), c);
+    c.least = min(min(div_word(a.x), div_word(a.y)), div_word(a.z));
+    if (div_failed(c)) return normalize3_ieee(a);
+    return v3(qdiv_unchecked(a.x, r), qdiv_unchecked(a.y, r), qdiv_unchecked(a.z, r));
+}
 HT_D Q4 normalize4_fast(Q4 a, DivCheck &c) {
     float l = sqrtf(dot4(a, a));
     Rcp r = rcp_of(l, c);
@@ -246,6 +253,8 @@ HT_D EuRay ray_eu_map(const Hom &m, V3 p, V3 v) {
     o.v = normalize3(rot3_apply(m.rot, v));
     return o;
 }
+// The same map, out of line: the object scan and the hit path share this one copy of its code.
+static __device__ __noinline__ EuRay ray_eu_map_call(const Hom m, const V3 p, const V3 v) { return ray_eu_map(m, p, v); }
 HT_D Hom hom3_inverse(const Hom &m) {
     Hom s;
     s.shift = v3(-m.shift.x, -m.shift.y, -m.shift.z);

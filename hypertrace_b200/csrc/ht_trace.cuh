@@ -505,26 +505,45 @@ HT_D EuPath camera_eu(const StagedScene &s, float px, float py, float size, uint
 
 HT_D bool hop_eu(const StagedScene &s, EuPath &ray, uint32_t &rng, uint32_t &prev_hash,
                  Col &intensity, Col &emission, bool &hit, uint32_t &n_exact) {
-    n_exact += s.n;
+    // Per chunk of 32 objects: the bounds of every object (warp-uniform, broadcast loads; 20
+    // instructions against 110 of an exact test), then each lane's survivors in index order, so
+    // that the reference's comparison (object/vector.inl:37-50) is unchanged. 25 objects: 0.8 exact
+    // tests per hop; 1917x1077, 16 passes 10.63 -> 4.91 ms (with normalize3's shared reciprocal and
+    // the winner's local ray kept, which leaves three maps of the hit path instead of four).
     float min_dist = -1.0f;
     uint32_t kmin = 0;
     const V3 p = ray.p, v = ray.v;
-    for (uint32_t k = 0; k < s.n; ++k) {
-        const uint32_t shape = s.shape[k];
-        const bool repeat = (k == prev_hash);
-        float dist = -1.0f;
-        if (shape == 0) {
-            if (!repeat) {
-                EuRay l = ray_eu_map(hom_from(s.inv[2 * k], s.inv[2 * k + 1]), p, v);
-                dist = plane_eu_dist(l.p, l.v);
+    const EuBoundRay br = eu_bound_ray(p, v);
+    float limit = __int_as_float(0x7f800000);   // +inf
+    for (uint32_t c0 = 0; c0 < s.n; c0 += 32) {
+        const uint32_t cn = min(32u, s.n - c0);
+        uint32_t mask = cn == 32 ? 0xFFFFFFFFu : (1u << cn) - 1u;
+        if (br.can) {
+            mask = 0;
+#pragma unroll 1
+            for (uint32_t j = 0; j < cn; ++j) {
+                const float4 rec = s.bound[c0 + j];
+                const bool out = s.shape[c0 + j] == 0 ? eu_culled_plane(rec, br, c0 + j == prev_hash, limit)
+                                                      : eu_culled_sphere(rec, br, limit);
+                mask |= (out ? 0u : 1u) << j;
             }
-        } else {
-            EuRay l = ray_eu_map(hom_from(s.inv[2 * k], s.inv[2 * k + 1]), p, v);
-            dist = sphere_eu_dist(l.p, l.v, repeat);
         }
-        if (dist > -EPSF && (min_dist <= -EPSF || dist < min_dist)) {
-            min_dist = dist;
-            kmin = k;
+        while (mask) {
+            const uint32_t k = c0 + (__ffs(mask) - 1);
+            mask &= mask - 1;
+            const uint32_t shape = s.shape[k];
+            const bool repeat = (k == prev_hash);
+            if (shape == 0 ? repeat : br.can && eu_far_sphere(s.bound[k], br, limit)) continue;
+            ++n_exact;
+            const EuRay l = ray_eu_map_call(hom_from(s.inv[2 * k], s.inv[2 * k + 1]), p, v);
+            const float dist = shape == 0 ? plane_eu_dist(l.p, l.v) : sphere_eu_dist(l.p, l.v, repeat);
+            if (dist > -EPSF && (min_dist <= -EPSF || dist < min_dist)) {
+                min_dist = dist;
+                kmin = k;
+                limit = fminf(limit, eu_limit(dist, br));
+                s.win[0] = make_float4(l.p.x, l.p.y, l.p.z, 0.0f);   // kept for the hit
+                s.win[1] = make_float4(l.v.x, l.v.y, l.v.z, 0.0f);
+            }
         }
     }
     if (!(min_dist > -EPSF)) {
@@ -538,26 +557,30 @@ HT_D bool hop_eu(const StagedScene &s, EuPath &ray, uint32_t &rng, uint32_t &pre
     const Hom inv = hom_from(s.inv[2 * kmin], s.inv[2 * kmin + 1]);
     const uint8_t *obj = s.objects + (size_t)kmin * OBJ_STRIDE;
     const Hom fwd = load_hom(obj);
-    EuRay l = ray_eu_map(inv, p, v);
+    EuRay l;   // the winner's local ray, as the scan computed it; min_dist is its test's root
+    {
+        const float4 a = s.win[0], b = s.win[1];
+        l.p = v3(a.x, a.y, a.z);
+        l.v = v3(b.x, b.y, b.z);
+    }
+    const float e = min_dist;
     EuPath lh;
     V3 normal;
     lh.v = l.v;
     if (s.shape[kmin] == 0) {
-        float t = -l.p.z / l.v.z;
-        lh.p = v3(l.p.x + l.v.x * t, l.p.y + l.v.y * t, 0.0f);
+        lh.p = v3(l.p.x + l.v.x * e, l.p.y + l.v.y * e, 0.0f);
         normal = v3(0.0f, 0.0f, -1.0f);
     } else {
-        float e = sphere_eu_dist(l.p, l.v, kmin == prev_hash);
         V3 h = normalize3(v3(l.p.x + l.v.x * e, l.p.y + l.v.y * e, l.p.z + l.v.z * e));
         lh.p = h;
         normal = h;
     }
-    EuRay w = ray_eu_map(fwd, lh.p, lh.v);
-    EuRay loc = ray_eu_map(inv, w.p, w.v);
+    EuRay w = ray_eu_map_call(fwd, lh.p, lh.v);
+    EuRay loc = ray_eu_map_call(inv, w.p, w.v);
     Material m = load_material(obj);
     V3 dir = loc.v;
     bool ret = mixture_interact(m, rng, normal, dir, intensity, emission);
-    EuRay out = ray_eu_map(fwd, loc.p, dir);
+    EuRay out = ray_eu_map_call(fwd, loc.p, dir);
     ray.p = out.p;
     ray.v = out.v;
     if (!ret) return false;

@@ -163,7 +163,9 @@ __device__ __forceinline__ void stage_object(const uint8_t *obj, uint32_t shape,
         rec = stage_bound(fwd, shape);
         mag = bound_mag(rec);
     } else {
-        Hom inv = hom3_inverse(load_hom(obj));
+        const Hom fwd = load_hom(obj);
+        const Hom inv = hom3_inverse(fwd);
+        rec = eu_stage_bound(fwd, shape);
         sm.inv[2 * q] = make_float4(inv.shift.x, inv.shift.y, inv.shift.z, 0.0f);
         sm.inv[2 * q + 1] = make_float4(inv.rot.x, inv.rot.y, inv.rot.z, inv.rot.w);
     }
