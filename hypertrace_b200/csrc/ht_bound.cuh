@@ -2,7 +2,7 @@
 // geodesic planes and horospheres and the culling tests on them. Shared by the hand-written
 // scene kernels (ht_trace.cuh) and the generic template kernels (ht_generic.cuh, also
 // compiled at run time by NVRTC). They decide only which objects are tested exactly, never a
-// result: tests/cull_check/cull_check.c restates them on the CPU and checks every hop's
+// result: tests/cull_check/scan_check.c restates them on the CPU and checks every hop's
 // winner against the full scan of the reference.
 #pragma once
 #include "ht_math.cuh"
@@ -29,9 +29,29 @@ namespace ht {
 // with p = (x, y, t) the ray start, v its unit direction (v.z along the height).
 // The threshold is thr = best (1 + CULL_REL) + CULL_ABS; objects with large map entries get
 // NaN records (never culled) and ray starts outside a well-conditioned box disable culling.
-constexpr float CULL_REL = 1e-2f, CULL_ABS = 1e-2f;
+//
+// Margins. The reference computes the local ray and the hit in f32, so what it reports differs
+// from the exact geometry; a test may cull only with more room than that. With eps = 2^-24,
+// N^2 the largest squared entry of the map (det 1) and G = 2 N^2 K0 / t >= 1 / t' (K0 = |p|^2 + |x| +
+// |y| + 1, t' the local height of the ray start):
+//   - the local start is off by about 10 eps N^2 K0 / t in the hyperbolic metric, a plane's
+//     |p'|^2 - 1 by 3 eps G in units of sinh(distance), and its hit point's height, sqrt(1 - |xy|^2),
+//     moves the hit by eps (3 G / |p'.d'| + G^2);
+//   - cosh(distance) is rounded to a multiple of 2 eps, which moves a distance d by 2 eps / d;
+//   - a root is reported from -EPS on: sinh(distance) up to 1e-6 G on the wrong side of a plane.
+// The additive allowance eF = mag K (K = K0^2 / t >= 2 K0) grows as these do: mag is
+// BOUND_EPS / 2 max(N^2, |rec|), plus PLANE_EPS N^4 for planes, which in sinh(distance) is at least
+// 2.5e-6 G + 2.4e-7 G^2, ten times the first item's linear and four times its quadratic part. On
+// top of it CULL_ABS = 2e-3 covers the rounding of distances (at most 4e-4 near d = 0) and
+// CULL_REL the hits far from the start, whose local height is e^-d of it; PLANE_M = 1e-3 t (5e-4
+// of sinh(distance)) keeps the signs of a plane's test apart. Fixed margins in place of the
+// allowance's quadratic part have to be sized for the worst map and let a hop test 20 % more
+// objects. tests/cull_check/scan_check.c runs all of this against the full scan on the CPU.
+constexpr float CULL_REL = 1e-2f, CULL_ABS = 2e-3f;
 
 constexpr float BOUND_EPS = 1e-5f;   // relative error allowance of F and W (>> f32 rounding)
+constexpr float PLANE_EPS = 2e-6f;   // allowance of a plane's hit point, per N^4
+constexpr float PLANE_M = 1e-3f;     // additive margin of the plane tests, in units of t
 constexpr float HORO_M = 1e-3f;      // relative margin of the horosphere root bounds
 
 // Hardware approximations (PTX rcp / sqrt / lg2 / ex2 .approx, relative error near 2^-22) for
@@ -44,17 +64,16 @@ HT_D float lg2_approx(float x) { float r; asm("lg2.approx.f32 %0, %1;" : "=f"(r)
 HT_D float ex2_approx(float x) { float r; asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 constexpr float LN2F = 0.693147180559945f, LOG2EF = 1.442695040888963f;
 
-// Error allowance of F for one object: BOUND_EPS * max |rec component|, so that
-// eF = mag * (|p|^2 + |x| + |y| + 1) >= BOUND_EPS * sum of |terms| of F (one multiply per object).
-HT_D float bound_mag(float4 rec) {
-    return BOUND_EPS * fmaxf(fmaxf(fabsf(rec.x), fabsf(rec.y)), fmaxf(fabsf(rec.z), fabsf(rec.w)));
-}
-
 struct Cull { float S, E, T; };   // sinh, exp, tanh of the threshold; S = E = inf, T = 1: none
 
-// World-space bound record of one object from its f32 map M, in FP64 (once per launch).
+// World-space bound record of one object from its f32 map M, in FP64 (once per launch), and the
+// magnitude `mag` of its error allowance.
 // N = adj(M) maps world to local (c22_inverse_n, matrix_complex.cc:60-65).
-HT_D float4 stage_bound(const Mo &m, uint32_t shape) {
+HT_D float bound_mag(float4 rec, double n2, uint32_t shape) {
+    const double m = fmax(n2, (double)fmaxf(fmaxf(fabsf(rec.x), fabsf(rec.y)), fmaxf(fabsf(rec.z), fabsf(rec.w))));
+    return (float)(0.5 * BOUND_EPS * m + (shape == 0 ? PLANE_EPS * m * m : 0.0));
+}
+HT_D float4 stage_bound(const Mo &m, uint32_t shape, float &mag) {
     const double ar = m.a.x, ai = m.a.y, br = m.b.x, bi = m.b.y;
     const double cr = m.c.x, ci = m.c.y, dr = m.d.x, di = m.d.y;
     const double det_r = (ar * dr - ai * di) - (br * cr - bi * ci);
@@ -62,7 +81,9 @@ HT_D float4 stage_bound(const Mo &m, uint32_t shape) {
     const double adet = sqrt(det_r * det_r + det_i * det_i);
     const double maxe = fmax(fmax(fabs(ar) + fabs(ai), fabs(br) + fabs(bi)), fmax(fabs(cr) + fabs(ci), fabs(dr) + fabs(di)));
     const float nan = __int_as_float(0x7fc00000);
+    mag = 0.0f;
     if (!(maxe <= 32.0 && adet >= 0.5 && adet <= 2.0)) return make_float4(nan, nan, nan, nan);
+    const double n2 = fmax(fmax(ar * ar + ai * ai, br * br + bi * bi), fmax(cr * cr + ci * ci, dr * dr + di * di)) / adet;
     // N = [[n11, n12], [n21, n22]] = [[d, -b], [-c, a]]
     const double n11r = dr, n11i = di, n12r = -br, n12i = -bi, n21r = -cr, n21i = -ci, n22r = ar, n22i = ai;
     if (shape == 0) {
@@ -71,7 +92,9 @@ HT_D float4 stage_bound(const Mo &m, uint32_t shape) {
         const double Br = (n11r * n12r + n11i * n12i) - (n21r * n22r + n21i * n22i);
         const double Bi = (n11r * n12i - n11i * n12r) - (n21r * n22i - n21i * n22r);
         const double C = (n12r * n12r + n12i * n12i) - (n22r * n22r + n22i * n22i);
-        return make_float4((float)(A / adet), (float)(2.0 * Br / adet), (float)(2.0 * Bi / adet), (float)(C / adet));
+        const float4 rec = make_float4((float)(A / adet), (float)(2.0 * Br / adet), (float)(2.0 * Bi / adet), (float)(C / adet));
+        mag = bound_mag(rec, n2, shape);
+        return rec;
     }
     // horosphere: scale N by 1 / sqrt|det| so the height formula holds
     const double k2 = 1.0 / adet;
@@ -79,14 +102,16 @@ HT_D float4 stage_bound(const Mo &m, uint32_t shape) {
     const double wr = (n22r * n21r + n22i * n21i) * k2;   // w = conj(n22) n21
     const double wi = (n22r * n21i - n22i * n21r) * k2;
     const double n22sq = (n22r * n22r + n22i * n22i) * k2;
-    return make_float4((float)c2, (float)(2.0 * wr), (float)(-2.0 * wi), (float)n22sq);
+    const float4 rec = make_float4((float)c2, (float)(2.0 * wr), (float)(-2.0 * wi), (float)n22sq);
+    mag = bound_mag(rec, n2, shape);
+    return rec;
 }
 
 // Per-hop constants of the bound evaluation.
 struct BoundRay {
-    float x, y, t, r2, pv, vx, vy, vz, ax, ay;
-    float K;    // |p|^2 + |x| + |y| + 1: eF = mag * K
-    float Kw;   // t (2 |p.v| + |vx| + |vy|): the part of eW that scales with mag
+    float x, y, t, r2, pv, vx, vy, vz;
+    float K;    // (|p|^2 + |x| + |y| + 1)^2 / t: eF = mag * K
+    float Kw;   // t (2 |p.v| + |vx| + |vy|) (|p|^2 + |x| + |y| + 1) / t: the part of eW that scales with mag
 };
 HT_D bool cull_point_ok(Q4 p) {
     return p.z >= 0x1p-20f && p.z <= 0x1p20f && fabsf(p.x) + fabsf(p.y) <= 0x1p10f * p.z &&
@@ -98,9 +123,9 @@ HT_D BoundRay bound_ray(Q4 p, Q4 v) {
     b.r2 = fmaf(p.x, p.x, fmaf(p.y, p.y, p.z * p.z));
     b.pv = fmaf(p.x, v.x, fmaf(p.y, v.y, p.z * v.z));
     b.vx = v.x; b.vy = v.y; b.vz = v.z;
-    b.ax = fabsf(p.x); b.ay = fabsf(p.y);
-    b.K = b.r2 + b.ax + b.ay + 1.0f;
-    b.Kw = b.t * (2.0f * fabsf(b.pv) + fabsf(b.vx) + fabsf(b.vy));
+    const float K0 = b.r2 + fabsf(p.x) + fabsf(p.y) + 1.0f;
+    b.K = K0 * K0 * rcp_approx(b.t);
+    b.Kw = K0 * (2.0f * fabsf(b.pv) + fabsf(b.vx) + fabsf(b.vy));
     return b;
 }
 // eF and eW of one object (the bounds of the float error of F and W)
@@ -170,18 +195,17 @@ HT_D BoundFW bound_fw(float4 rec, float mag, const BoundRay &r) {
     b.eW = bound_eW(mag, b.eF, b.W, r);
     return b;
 }
-HT_D bool culled_fw(const BoundFW &b, uint32_t shape, float t, const Cull &c) {
+// The ray-aware test of one object that the point bound kept.
+HT_D bool culled_ray(const BoundFW &b, uint32_t shape, float t, const Cull &c) {
     const float F = b.F, eF = b.eF, W = b.W, eW = b.eW;
     if (shape == 0) {
         const float Fa = fabsf(F) - eF;       // lower bound of |2 t a|
         const float Wlo = fabsf(W) - eW, Whi = fabsf(W) + eW;
-        // starts off the plane and moves away from it: |a| > 0.01, |b| > 0.001, same signs
-        const bool away = (F > 0.0f) == (W > 0.0f) && Fa > 0.02f * t && Wlo > 0.002f * t;
-        // |a| > 1.01 T |b| + 0.01: no root (T = 1) or the root lies beyond the threshold
-        const bool far = Fa > fmaf(1.01f * c.T, Whi, 0.02f * t);
-        // the start point itself is farther than the threshold
-        const bool point = Fa > 2.0f * t * c.S;
-        return away || far || point;
+        // starts off the plane and moves away from it: |a| > 5e-4 and more, |b| > 0.001, same signs
+        const bool away = (F > 0.0f) == (W > 0.0f) && Fa > fmaf(PLANE_M, t, eF) && Wlo > 0.002f * t;
+        // |a| > 1.01 T |b| + 5e-4: no root (T = 1) or the root lies beyond the threshold
+        const bool far = Fa > fmaf(1.01f * c.T, Whi, PLANE_M * t);
+        return away || far;
     } else {
         // In the object's frame the reference's horosphere test (shape/hy/horosphere.cc:4-34)
         // looks at two roots; with P = F/t (1 / local height), V = W/t (its derivative along
@@ -192,7 +216,6 @@ HT_D bool culled_fw(const BoundFW &b, uint32_t shape, float t, const Cull &c) {
         // culled when every root that can be reported lies farther than the threshold.
         const float Flo = F - eF, Fhi = F + eF, Wlo = W - eW, Whi = W + eW;
         const float aWlo = fmaxf(fabsf(W) - eW, 0.0f), aWhi = fabsf(W) + eW;
-        if (t > c.E * Fhi || t * c.E < Flo) return true;   // every point farther than the threshold
         if (!(Flo > 0.0f)) return false;
         const float R2lo = t * t - Fhi * Fhi + aWlo * aWlo, R2hi = t * t - Flo * Flo + aWhi * aWhi;
         if (R2hi < -HORO_M * t * t) return true;        // no crossing
@@ -208,18 +231,6 @@ HT_D bool culled_fw(const BoundFW &b, uint32_t shape, float t, const Cull &c) {
         return (!r1 || r1_far) && (!r2 || r2_far);
     }
 }
-static __device__ __noinline__ bool culled_fw_call(const BoundFW b, uint32_t shape, float t, const Cull c) {
-    return culled_fw(b, shape, t, c);
-}
-// OOL: the root tests out of line (one copy of their code, called per survivor). Measured at
-// 1920x1080 / 200 objects: the single-view wavefront kernel 5.95 -> 5.55 ms per pass out of
-// line, the batched kernels (both recipes per module) 954 -> 938 Msamples/s: each kernel takes
-// the faster form.
-template <bool OOL>
-HT_D bool culled(float4 rec, float mag, uint32_t shape, const BoundRay &r, const Cull &c) {
-    const BoundFW b = bound_fw(rec, mag, r);
-    return OOL ? culled_fw_call(b, shape, r.t, c) : culled_fw(b, shape, r.t, c);
-}
 
 // Upper bound of e^(2 s) at the nearest crossing of one object that the reference surely
 // reports (s = distance along the ray): geodesic planes crossed ahead (tanh s = |F| / |W|,
@@ -232,7 +243,7 @@ HT_D float sure_crossing_e2(const BoundFW &b, uint32_t shape, bool plane_repeat,
     if (shape == 0) {
         if (plane_repeat) return inf;   // a plane is never hit twice in a row
         const float Fa = fabsf(F) - eF, Wlo = fabsf(W) - eW;
-        if (!((F > 0.0f) != (W > 0.0f) && Fa > 0.02f * t && Wlo > 0.0f)) return inf;
+        if (!((F > 0.0f) != (W > 0.0f) && Fa > fmaf(PLANE_M, t, eF) && Wlo > 0.02f * t)) return inf;
         const float rr = (fabsf(F) + eF) * rcp_approx(Wlo);   // >= tanh s
         if (!(rr < 0.99f)) return inf;
         return (1.0f + rr) * rcp_approx(1.0f - rr);
@@ -256,6 +267,33 @@ HT_D float sure_crossing_e2(const BoundFW &b, uint32_t shape, bool plane_repeat,
         if (D > 0.02f) e = (Fhi - Wlo) * it * rcp_approx(1.0f + sqrt_approx(D));
     }
     return e * e;
+}
+// Whether the scan has to test one object exactly, from the point bound `k` of its shape and the
+// ray-aware test.
+HT_D bool keep_object(float4 rec, float mag, uint32_t shape, const BoundRay &r, const PointCut &k, const Cull &c) {
+    const BoundFW b = bound_fw(rec, mag, r);
+    return !(b.F + b.eF < k.lo.x || b.F - b.eF > k.hi.x || culled_ray(b, shape, r.t, c));
+}
+// The threshold of a scan: the nearest hit found, or surely to be found, so far.
+struct Limit {
+    float d;        // that distance (+inf: none)
+    Cull cull;
+    PointCut kp, kh;
+};
+HT_D Limit limit_none(float t) {
+    Limit l;
+    l.d = __int_as_float(0x7f800000);
+    l.cull = cull_none();
+    l.kp = point_cut(0, t, l.cull);
+    l.kh = point_cut(1, t, l.cull);
+    return l;
+}
+HT_D void limit_lower(Limit &l, float d, float t) {
+    if (!(d < l.d)) return;
+    l.d = d;
+    l.cull = cull_from_dist(d);
+    l.kp = point_cut(0, t, l.cull);
+    l.kh = point_cut(1, t, l.cull);
 }
 // Distance of a crossing from its e^(2 s) bound (the threshold built from it adds 1e-2 margins).
 HT_D float dist_from_e2(float x) { return 0.5f * LN2F * lg2_approx(x); }

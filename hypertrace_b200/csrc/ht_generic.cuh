@@ -184,11 +184,6 @@ HT_D V3 normalize_q(V3 a) { return normalize3(a); }
 // Each map: V (the value), lay, load, inverse, pos, dir (apply_dir), normal (apply_normal),
 // ray (ray_<geo>_map: start = pos, direction = normalize(dir), geometry/ray_map.inl:15-21)
 // and view (view/mapped.inl:20-26: direction = dir, then start = pos).
-HT_D Q4 mo_apply_pos(const Mo &m, Q4 p) {   // mo_apply_q (transform/moebius.cc:20-25)
-    Q4 u = q_addc(cq_mul(m.a, p), m.b);
-    Q4 d = q_addc(cq_mul(m.c, p), m.d);
-    return q_mul(u, q_inverse(d));
-}
 struct Moebius {
     typedef Mo V;
     template <int W> __host__ __device__ static constexpr Lay lay() { return Lay{32u, 32u}; }   // comp2x2 (matrix.rs:174-209)
@@ -1195,9 +1190,9 @@ HT_D u32 stage_vec_bounds(Ptr self, Ptr end, float4 *rec, float *mag, u32 *kind)
     for (u32 i = threadIdx.x; i < n; i += blockDim.x) {
         const Ptr elem = self + head + i * stride;
         const u32 k = B::template kind_of<W>(elem);
-        const float4 r = k <= 1u ? stage_bound(B::template map_of<W>(elem), k) : make_float4(nan, nan, nan, nan);
-        rec[i] = r;
-        mag[i] = bound_mag(r);
+        float m = 0.0f;
+        rec[i] = k <= 1u ? stage_bound(B::template map_of<W>(elem), k, m) : make_float4(nan, nan, nan, nan);
+        mag[i] = m;
         kind[i] = k;
     }
     return n;
@@ -1230,41 +1225,38 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
     const Q4 p = l.p, v = l.v;
     const bool staged = c.bvec == self, can = staged && cull_point_ok(p);
     const BoundRay br = bound_ray(p, v);
-    Cull cull = cull_none();
+    Limit lim = limit_none(br.t);
     if (can) {
         float best = __int_as_float(0x7f800000);
         const u32 ne = n < 32u ? n : 32u;
 #pragma unroll 1
         for (u32 i = 0; i < ne; ++i)   // warp-uniform: broadcast loads
             best = fminf(best, sure_crossing_e2(bound_fw(c.brec[i], c.bmag[i], br), c.bkind[i], i + h0 == c.prev, br.t));
-        if (best < __int_as_float(0x7f800000)) cull = cull_from_dist(dist_from_e2(best));
+        if (best < __int_as_float(0x7f800000)) limit_lower(lim, dist_from_e2(best), br.t);
     }
-    PointCut kp = point_cut(0, br.t, cull), kh = point_cut(1, br.t, cull);
     float min_dist = -1.0f, min_x = __int_as_float(0x7f800000);
     u32 min_index = 0, tested = 0;
 #pragma unroll 1
-    for (u32 c0 = 0; c0 < n; c0 += 32) {
+    for (u32 c0 = 0; c0 < n; c0 += 32u) {
         const u32 cn = n - c0 < 32u ? n - c0 : 32u;
         u32 mask = cn == 32u ? 0xFFFFFFFFu : (1u << cn) - 1u;
         if (can) {
             u32 m = 0;
 #pragma unroll 1
             for (u32 j = 0; j < cn; ++j) {   // warp-uniform: broadcast loads
-                const u32 k = c0 + j;
-                if (!culled_point(c.brec[k], c.bmag[k], br, c.bkind[k] == 0u ? kp : kh)) m |= 1u << j;
+                if (!culled_point(c.brec[c0 + j], c.bmag[c0 + j], br, c.bkind[c0 + j] == 0u ? lim.kp : lim.kh)) m |= 1u << j;
             }
-            mask = m;
+            mask = 0;
             while (m) {   // per lane: the ray-aware bound on the survivors
-                const u32 j = __ffs(m) - 1;
+                const u32 j = __ffs(m) - 1, i = c0 + j;
                 m &= m - 1;
-                const u32 k = c0 + j;
-                if (culled<true>(c.brec[k], c.bmag[k], c.bkind[k], br, cull)) mask &= ~(1u << j);
+                if (keep_object(c.brec[i], c.bmag[i], c.bkind[i], br, c.bkind[i] == 0u ? lim.kp : lim.kh, lim.cull)) mask |= 1u << j;
             }
         }
         while (mask) {   // this lane's candidates, in index order
             const u32 i = c0 + (__ffs(mask) - 1);
             mask &= mask - 1;
-            if (can && culled_point(c.brec[i], c.bmag[i], br, c.bkind[i] == 0u ? kp : kh)) continue;
+            if (can && culled_point(c.brec[i], c.bmag[i], br, c.bkind[i] == 0u ? lim.kp : lim.kh)) continue;
             ++tested;
             const Ptr elem = self + head + i * stride;
             const u32 kind = staged ? c.bkind[i] : B::template kind_of<W>(elem);
@@ -1278,11 +1270,7 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
                     min_dist = dist; min_x = x; min_index = i;
                     c.win[0] = make_float4(r.p.x, r.p.y, r.p.z, r.p.w);
                     c.win[1] = make_float4(r.v.x, r.v.y, r.v.z, r.v.w);
-                    if (staged) {
-                        cull = cull_from_dist(dist);
-                        kp = point_cut(0, br.t, cull);
-                        kh = point_cut(1, br.t, cull);
-                    }
+                    if (staged) limit_lower(lim, dist, br.t);
                 }
             }
         }

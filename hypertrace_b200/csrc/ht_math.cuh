@@ -206,6 +206,10 @@ HT_D HyRay ray_hy_map(const Mo &m, Q4 p, Q4 v) {
 // code (instruction-cache footprint; an inlined copy in the scan measured slower).
 static __device__ __noinline__ HyRay ray_hy_map_call(const Mo m, const Q4 p, const Q4 v) { return ray_hy_map(m, p, v); }
 
+HT_D Q4 mo_apply_pos(const Mo &m, Q4 p) {   // mo_apply_q (transform/moebius.cc:20-25)
+    return q_mul(q_addc(cq_mul(m.a, p), m.b), q_inverse(q_addc(cq_mul(m.c, p), m.d)));
+}
+
 // Camera map (view/mapped.inl:20-26): direction = mo_apply_dir (one normalize), then start.
 // Once per sample, so plain IEEE division.
 HT_D HyRay view_hy_map(const Mo &m, Q4 p, Q4 v) {

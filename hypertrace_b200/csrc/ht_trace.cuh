@@ -219,9 +219,14 @@ static __device__ __noinline__ HyPath camera_hy(const StagedScene &s, float px, 
 // One hop (one iteration of render/scene.inl:25-41). Returns true while the path goes on.
 // `hit` reports whether the scan found an object (for the hop statistics).
 // ---------------------------------------------------------------- the scan's packed point bound
-// Objects the upper estimate looks at (the first ones in index order).
+// Objects the upper estimate looks at: the first half of them planes, the others horospheres, the
+// nearest to the camera of each (stage_scene's slot order). 1080p / 200 objects, 8 passes: 8 objects
+// 11.84 ms, 12 11.29, 16 11.56, 24 12.10; 24 mixed views batched 41.1, 41.0, 41.9, 44.0 ms. In scene
+// order 24 to 40 objects were best, and the scan tested 3.2-4.9 objects per hop where it now
+// tests 1.4-2.2 (16.3 and 55.3 ms before the slot order, the allowances of ht_bound.cuh and the
+// warp-uniform ray-aware tests).
 #ifndef HT_EST_OBJECTS
-#define HT_EST_OBJECTS 24u   // 12 planes + 12 horospheres: 492.6 Msamples/s at 1080p, 16: 480.4, 32: 485.8, 40: 470.3
+#define HT_EST_OBJECTS 12u
 #endif
 struct PairRay { float2 r2, x, y, K; };   // the bound ray's constants, each in both halves
 HT_D PairRay pair_ray(const BoundRay &r) {
@@ -244,10 +249,6 @@ HT_D uint32_t survivors2(float4 a, float4 b, float2 mag, const PairRay &r, const
     const bool c1 = up.y < k.lo.y || dn.y > k.hi.y;
     return (c0 ? 0u : 1u) | (c1 ? 0u : 2u);
 }
-HT_D bool culled_slot(const StagedScene &s, uint32_t q, const BoundRay &r, const PointCut &kp, const PointCut &kh) {
-    return culled_point(s.bound[q], s.mag[q], r, s.shape[q] == 0 ? kp : kh);
-}
-
 // Upper estimate of the nearest hit that the reference surely reports (the least
 // sure_crossing_e2) among the first HT_EST_OBJECTS / 2 planes and the first HT_EST_OBJECTS / 2
 // horospheres of the staged slots, +inf when none qualifies. A threshold derived from it
@@ -328,7 +329,7 @@ HT_D uint32_t warp_survivors(const StagedScene &s, uint32_t c0, uint32_t valid, 
 
 // WARP: the warp pre-cull is compiled in; `full_warp` (all 32 lanes of the warp are in this
 // call together, uniform across the warp) turns it on.
-template <bool OOL, bool WARP = false>
+template <bool WARP = false>
 HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &prev_hash,
                  Col &intensity, Col &emission, bool &hit, uint32_t &n_exact, bool full_warp = false) {
     // Nearest hit with ties to the lowest scene index (object/vector.inl:37-50): candidates
@@ -341,13 +342,9 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
     const Q4 p = ray.p, v = ray.v;
     const bool can_cull = cull_point_ok(p);
     const BoundRay br = bound_ray(p, v);
-    const PairRay pr = pair_ray(br);
-    Cull cull = cull_none();
-    if (can_cull) {   // a threshold before the first exact test, from the first slots' crossings
-        const float u = upper_estimate(s, br, prev_hash);
-        if (u < __int_as_float(0x7f800000)) cull = cull_from_dist(u);
-    }
-    PointCut kp = point_cut(0, br.t, cull), kh = point_cut(1, br.t, cull);
+    Limit lim = limit_none(br.t);
+    if (can_cull) limit_lower(lim, upper_estimate(s, br, prev_hash), br.t);   // before the first exact test
+    const uint32_t h0 = (s.n_planes + 1) & ~1u;   // the first horosphere's slot
     bool warp_pre = false;
     WarpBox wb;
     if constexpr (WARP) {
@@ -357,54 +354,46 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
             if (warp_pre) wb = warp_box(br);
         }
     }
+#pragma unroll 1
     for (uint32_t c0 = 0; c0 < s.ns; c0 += 32) {
         const uint32_t cn = min(32u, s.ns - c0);
         uint32_t valid = cn == 32 ? 0xFFFFFFFFu : (1u << cn) - 1u;
         if (s.dummy - c0 < 32u) valid &= ~(1u << (s.dummy - c0));
         uint32_t mask = valid;
         if (can_cull) {
-            mask = 0;
+            uint32_t m = valid;   // objects to look at one by one
             if constexpr (WARP) {
-                // one copy of the pair loop for both cases (instruction fetch): over the pairs
-                // with a slot the warp keeps, or over every valid pair without the warp test
-                uint32_t keep = valid;
+                // those that the warp keeps: one object at a time for all lanes, so loads are
+                // broadcasts and a shape's test runs without divergence (each lane taking its own
+                // survivors of the point bound: 1080p / 200 objects, 8 passes 15.0 against 14.1 ms)
                 if (warp_pre) {   // uniform: every lane can cull
                     __syncwarp();
-                    keep = warp_survivors(s, c0, valid, wb, kp, kh);
+                    m = warp_survivors(s, c0, valid, wb, lim.kp, lim.kh);
                 }
-                uint32_t pm = (keep | (keep >> 1)) & 0x55555555u;
-                while (pm) {   // this lane's point test
-                    const uint32_t j = __ffs(pm) - 1;
-                    pm &= pm - 1;
-                    const uint32_t pq = (c0 + j) >> 1;
-                    const PointCut &k = c0 + j >= s.n_planes ? kh : kp;
-                    mask |= survivors2(s.pa[pq], s.pb[pq], s.pmag[pq], pr, k) << j;
-                }
-                mask &= keep;
             } else {
+                // this lane's survivors of the point bound, two slots at once
+                m = 0;
                 // kept rolled: the kernel is bound by instruction fetch as much as by issue
 #pragma unroll 1
-                for (uint32_t j = 0; j < cn; j += 2) {   // warp-uniform: broadcast loads, two slots at once
+                for (uint32_t j = 0; j < cn; j += 2) {   // warp-uniform: broadcast loads
                     const uint32_t pq = (c0 + j) >> 1;
-                    const PointCut &k = c0 + j >= s.n_planes ? kh : kp;
-                    mask |= survivors2(s.pa[pq], s.pb[pq], s.pmag[pq], pr, k) << j;
+                    m |= survivors2(s.pa[pq], s.pb[pq], s.pmag[pq], pair_ray(br), c0 + j >= s.n_planes ? lim.kh : lim.kp) << j;
                 }
+                m &= valid;
             }
-            mask &= valid;
-            // per lane: the ray-aware bound on the survivors only
-            uint32_t m = mask;
+            mask = 0;
             while (m) {
-                const uint32_t j = __ffs(m) - 1;
+                const uint32_t j = __ffs(m) - 1, q = c0 + j;
                 m &= m - 1;
-                const uint32_t q = c0 + j;
-                if (culled<OOL>(s.bound[q], s.mag[q], s.shape[q], br, cull)) mask &= ~(1u << j);
+                const uint32_t shape = q >= h0 ? 1u : 0u;
+                if (keep_object(s.bound[q], s.mag[q], shape, br, shape == 0 ? lim.kp : lim.kh, lim.cull)) mask |= 1u << j;
             }
         }
         while (mask) {   // this lane's candidates, in slot order
             const uint32_t q = c0 + (__ffs(mask) - 1);
             mask &= mask - 1;
-            const uint32_t shape = s.shape[q];
-            if (can_cull && culled_slot(s, q, br, kp, kh)) continue;
+            const uint32_t shape = q >= h0 ? 1u : 0u;
+            if (can_cull && culled_point(s.bound[q], s.mag[q], br, shape == 0 ? lim.kp : lim.kh)) continue;
             const uint32_t k = s.orig[q];
             const bool repeat = (k == prev_hash);
             if (shape == 0 && repeat) continue;   // a geodesic plane is never hit twice in a row
@@ -422,9 +411,7 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
                     min_x = x;
                     kmin = q;
                     kmin_orig = k;
-                    cull = cull_from_dist(dist);
-                    kp = point_cut(0, br.t, cull);
-                    kh = point_cut(1, br.t, cull);
+                    limit_lower(lim, dist, br.t);
                     s.win[0] = make_float4(l.p.x, l.p.y, l.p.z, l.p.w);   // kept for the hit
                     s.win[1] = make_float4(l.v.x, l.v.y, l.v.z, l.v.w);
                 }

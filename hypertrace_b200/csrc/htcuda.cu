@@ -105,8 +105,11 @@ struct htc_program {
 // Loads the scene header and the per-object data the scan reads into shared memory. Returns
 // false (uniformly across the block) when the scene bytes fail validation.
 //
-// Hyperbolic scenes are staged in scan order, geodesic planes first (in index order), then
-// horospheres (in index order); when the plane count is odd a dummy slot follows the planes,
+// Hyperbolic scenes are staged in scan order, geodesic planes first, then horospheres, each by
+// their distance from the camera (scenes of up to STAGE_SORT_MAX objects; index order beyond):
+// the paths of a view stay near it, so the first few slots of a shape nearly always hold a sure
+// crossing close to the winner's (upper_estimate), and the later chunks fall to the warp
+// pre-cull. When the plane count is odd a dummy slot follows the planes,
 // so that every pair of slots (2p, 2p + 1) holds one shape and the point-bound loop can test
 // two objects per packed FP32 instruction. `orig[slot]` is the object's index in the scene:
 // the scan compares hits on (distance, index), the reference's nearest-hit rule
@@ -119,6 +122,7 @@ struct htc_program {
 // bound magnitude and scene index per slot (u32 / f32 / u32), then 2 float4 per thread of a
 // 128-thread block (the scan's winner, local frame).
 constexpr uint32_t BLOCK_THREADS = 128;
+constexpr uint32_t STAGE_SORT_MAX = 2 * BLOCK_THREADS * 4;   // words of the winners' slots, the sort's scratch
 struct SceneSmem {
     float4 *inv, *bound, *pa, *pb;
     float2 *pmag;
@@ -160,8 +164,7 @@ __device__ __forceinline__ void stage_object(const uint8_t *obj, uint32_t shape,
         Mo inv = mo_inverse(fwd);
         sm.inv[2 * q] = make_float4(inv.a.x, inv.a.y, inv.b.x, inv.b.y);
         sm.inv[2 * q + 1] = make_float4(inv.c.x, inv.c.y, inv.d.x, inv.d.y);
-        rec = stage_bound(fwd, shape);
-        mag = bound_mag(rec);
+        rec = stage_bound(fwd, shape, mag);
     } else {
         const Hom fwd = load_hom(obj);
         const Hom inv = hom3_inverse(fwd);
@@ -209,15 +212,28 @@ __device__ bool stage_scene(const uint8_t *scene, size_t scene_size, uint32_t ma
     bool bad = false;
     uint32_t n_planes = 0, dummy = 0xFFFFFFFFu;
     if (R == RECIPE_HY) {
-        // pass 1: the number of planes
+        // pass 1: the number of planes, and every object's sort key (shape, distance from the
+        // camera; both shapes' distances grow with |F| or max(F, 1 / F) of the bound record)
+        uint32_t *keys = reinterpret_cast<uint32_t *>(sm.win);
+        const bool by_distance = n <= STAGE_SORT_MAX;
+        const Q4 cam = mo_apply_pos(load_mo(scene), q4(0.0f, 0.0f, 1.0f, 0.0f));
+        const BoundRay at = bound_ray(cam, q4(1.0f, 0.0f, 0.0f, 0.0f));
         for (uint32_t r0 = 0; r0 < n; r0 += nthreads) {
             const uint32_t k = r0 + tid;
-            const bool plane = k < n && ldu(objects + (size_t)k * OBJ_STRIDE, O_SHAPE) == 0;
-            n_planes += (uint32_t)__syncthreads_count(plane ? 1 : 0);
+            const uint8_t *obj = objects + (size_t)k * OBJ_STRIDE;
+            const uint32_t shape = k < n ? ldu(obj, O_SHAPE) : 1u;
+            if (by_distance && k < n) {
+                float mag;
+                const float F = bound_fw(stage_bound(load_mo(obj), min(shape, 1u), mag), 0.0f, at).F / at.t;
+                const float d = shape == 0 ? fabsf(F) : fmaxf(F, 1.0f / F);
+                keys[k] = (shape == 0 ? 0u : 0x80000000u) | (d >= 0.0f ? __float_as_uint(d) : 0u);   // NaN records first
+            }
+            n_planes += (uint32_t)__syncthreads_count(shape == 0 ? 1 : 0);
         }
-        // pass 2: slot = rank among the planes, or n_planes (rounded up to even) + rank among
-        // the horospheres; ranks from a ballot per warp and the warps' counts in s_hdr[2..]
-        const uint32_t h0 = (n_planes + 1) & ~1u;
+        // pass 2: slot = rank among the keys (ties by index); horospheres start at an even slot.
+        // Beyond the sort: rank among the planes, from a ballot per warp and the warps' counts in
+        // s_hdr[2..], or among the horospheres
+        const uint32_t gap = n_planes & 1u, h0 = n_planes + gap;
         const uint32_t lane = tid & 31u, warp = tid >> 5, nwarps = (nthreads + 31) >> 5;
         uint32_t before = 0;   // planes among the objects before this block-wide step
         for (uint32_t r0 = 0; r0 < n; r0 += nthreads) {
@@ -225,21 +241,32 @@ __device__ bool stage_scene(const uint8_t *scene, size_t scene_size, uint32_t ma
             const bool in = k < n;
             const uint8_t *obj = objects + (size_t)k * OBJ_STRIDE;
             const uint32_t shape = in ? ldu(obj, O_SHAPE) : 1u;
-            const uint32_t ballot = __ballot_sync(0xffffffffu, in && shape == 0);
-            if (lane == 0) s_hdr[2 + warp] = (uint32_t)__popc(ballot);
-            __syncthreads();
-            uint32_t rank = before + (uint32_t)__popc(ballot & ((1u << lane) - 1u)), total = 0;
-            for (uint32_t w = 0; w < nwarps; ++w) {
-                const uint32_t c = s_hdr[2 + w];
-                if (w < warp) rank += c;
-                total += c;
+            uint32_t slot = 0;
+            if (by_distance) {
+                const uint32_t mine = in ? keys[k] : 0u;
+                for (uint32_t j = 0; j < n; ++j) {   // broadcast loads
+                    const uint32_t other = keys[j];
+                    slot += other < mine || (other == mine && j < k) ? 1u : 0u;
+                }
+                slot += shape == 0 ? 0u : gap;
+            } else {
+                const uint32_t ballot = __ballot_sync(0xffffffffu, in && shape == 0);
+                if (lane == 0) s_hdr[2 + warp] = (uint32_t)__popc(ballot);
+                __syncthreads();
+                uint32_t rank = before + (uint32_t)__popc(ballot & ((1u << lane) - 1u)), total = 0;
+                for (uint32_t w = 0; w < nwarps; ++w) {
+                    const uint32_t c = s_hdr[2 + w];
+                    if (w < warp) rank += c;
+                    total += c;
+                }
+                __syncthreads();
+                before += total;
+                slot = shape == 0 ? rank : h0 + (k - rank);
             }
-            __syncthreads();
-            before += total;
             if (in) {
                 if (address_width == 64 && ldu(obj, O_SHAPE + 4) != 0) bad = true;
                 if (shape > 1) bad = true;
-                stage_object<R>(obj, shape > 1 ? 1u : shape, k, shape == 0 ? rank : h0 + (k - rank), sm);
+                stage_object<R>(obj, shape > 1 ? 1u : shape, k, slot, sm);
             }
         }
         if (n_planes & 1u) {   // the dummy slot: never a candidate (masked), NaN bound record
@@ -303,12 +330,12 @@ __device__ __forceinline__ typename PathOf<R>::T camera(const StagedScene &s, fl
 }
 // WARP / full_warp: the hyperbolic scan's warp pre-cull (hop_hy), for callers whose warps
 // enter together.
-template <int R, bool OOL = true, bool WARP = false>
+template <int R, bool WARP = false>
 __device__ __forceinline__ bool hop(const StagedScene &s, typename PathOf<R>::T &ray, uint32_t &rng,
                                     uint32_t &prev_hash, Col &intensity, Col &emission, bool &hit,
                                     uint32_t &n_exact, bool full_warp = false) {
     if constexpr (R == RECIPE_HY)
-        return hop_hy<OOL, WARP>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact, full_warp);
+        return hop_hy<WARP>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact, full_warp);
     else return hop_eu(s, ray, rng, prev_hash, intensity, emission, hit, n_exact);
 }
 
@@ -368,9 +395,7 @@ __global__ void __launch_bounds__(128, HT_PLAIN_MINB) render_plain(
         for (uint32_t i = 0; i < hops; ++i) {
             bool hit;
             n_hops += 1;
-            // root tests inline: faster for this kernel (per view on the mixed workload's
-            // views, 2138 vs 2177 ms), unlike the wavefront kernel
-            bool go = hop<R, false>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact);
+            bool go = hop<R>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact);
             n_hits += hit ? 1 : 0;
             if (!go) break;
         }
@@ -575,7 +600,7 @@ __host__ __device__ inline WaveQueue wave_at(const WaveQueue &q, uint64_t off) {
 // FH: 1 = hop 0 (pixels), 2 = a later hop (queue), known at compile time so that each
 // kernel carries only its own half (the kernel is bound by instruction fetch as much as by
 // issue); 0 = decided by `first_hop` at run time.
-template <int R, int FH, bool OOL = true>
+template <int R, int FH>
 __device__ __forceinline__ void wave_chunk(const StagedScene &s, uint32_t base, uint32_t n, bool first_hop,
                                            bool last_hop, uint32_t W, uint32_t H, uint32_t flags,
                                            float4 *__restrict__ canvas, uint32_t *__restrict__ seeds,
@@ -610,7 +635,7 @@ __device__ __forceinline__ void wave_chunk(const StagedScene &s, uint32_t base, 
         bool hit;
         st.hops += 1;
         st.tests += s.n;
-        const bool go = hop<R, OOL, true>(s, ray, rng, prev_hash, intensity, emission, hit, st.exact, full_warp);
+        const bool go = hop<R, true>(s, ray, rng, prev_hash, intensity, emission, hit, st.exact, full_warp);
         st.hits += hit ? 1 : 0;
         cont = go && !last_hop;
         if (!cont) {
@@ -1017,10 +1042,10 @@ __global__ void __launch_bounds__(128, RF ? HT_BATCH_MINB : HT_PERSIST_MINB) ren
             // slots are pixel numbers on hop 0, tile-relative queue slots later
             const uint32_t b0 = first_hop ? first + base : base, n0 = first_hop ? first + count : count;
             if (recipe == RECIPE_HY)
-                wave_chunk<RECIPE_HY, FH, false>(s, b0, n0, first_hop, last_hop, v.width, v.height, v.flags, canvas, seeds, vin,
+                wave_chunk<RECIPE_HY, FH>(s, b0, n0, first_hop, last_hop, v.width, v.height, v.flags, canvas, seeds, vin,
                                       vout, out_count, st);
             else
-                wave_chunk<RECIPE_EU, FH, false>(s, b0, n0, first_hop, last_hop, v.width, v.height, v.flags, canvas, seeds, vin,
+                wave_chunk<RECIPE_EU, FH>(s, b0, n0, first_hop, last_hop, v.width, v.height, v.flags, canvas, seeds, vin,
                                       vout, out_count, st);
         }
     }
