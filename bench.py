@@ -361,10 +361,11 @@ def main():
 
     # roofline of render_wave (one launch per hop depth, `passes * hops` launches per step):
     # measured operations per path-hop x this run's path-hops, over the device time of the
-    # step, which also holds the coherence sort between hop depths (4 launches per depth of a
+    # step, which also holds the coherence sort between hop depths (2 launches per depth of a
     # hyperbolic pass after the first)
     launches = args.steps * args.passes * sc.hops
-    sort_launches = args.steps * args.passes * (sc.hops - 1) * 4 if sc.recipe == _lib.HTC_RECIPE_HY else 0
+    sort_launches = args.steps * args.passes * (sc.hops - 1) * 2 if sc.recipe == _lib.HTC_RECIPE_HY else 0
+    sort_launches += args.steps   # the scene's image, once per call
     per_launch_s = dev_s / launches
     achieved = FP32_OPS_PER_HOP * hops / dev_s / 1e12 if FP32_OPS_PER_HOP else None
     ref_tflops = tests * REF_OPS_PER_OBJECT_TEST / dev_s / 1e12
