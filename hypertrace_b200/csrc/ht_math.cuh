@@ -158,8 +158,9 @@ HT_D Q4 q_inverse(Q4 d) {
 // the denominator d, |d|^2 and q_inverse(d) = conj(d) / |d|^2.
 struct HyRay { Q4 p, v; };
 
-// Reference evaluation with IEEE division everywhere (the fallback of ray_hy_map).
-static __device__ __noinline__ HyRay ray_hy_map_ieee(const Mo m, const Q4 p, const Q4 v) {
+// Reference evaluation with IEEE division everywhere (the fallback of the maps below). `twice`:
+// mo_apply_dir normalizes, ray_map.inl:19 again.
+static __device__ __noinline__ HyRay hy_map_ieee(const Mo m, const Q4 p, const Q4 v, bool twice) {
     Q4 u = q_addc(cq_mul(m.a, p), m.b);
     Q4 d = q_addc(cq_mul(m.c, p), m.d);
     float d2 = dot4(d, d);
@@ -174,14 +175,16 @@ static __device__ __noinline__ HyRay ray_hy_map_ieee(const Mo m, const Q4 p, con
     Q4 g22 = q4(k * dc.x, k * dc.y, k * dc.z, k * dc.w);
     Q4 t = q_sub(g21, g22);
     Q4 g2 = q_mul(u, q4(t.x / d2, t.y / d2, t.z / d2, t.w / d2));
-    Q4 deriv = q_add(g1, g2);
-    o.v = normalize4(normalize4(deriv));   // mo_apply_dir normalizes, ray_map.inl:19 again
+    o.v = normalize4(q_add(g1, g2));
+    if (twice) o.v = normalize4(o.v);
     return o;
 }
+static __device__ __forceinline__ HyRay ray_hy_map_ieee(const Mo m, const Q4 p, const Q4 v) { return hy_map_ieee(m, p, v, true); }
 
-// ray_<hy>_map (geometry/ray_map.inl:15-21): the nine divisions by |d|^2 share one
-// reciprocal, each normalize shares one; results are bit-identical to ray_hy_map_ieee.
-HT_D HyRay ray_hy_map(const Mo &m, Q4 p, Q4 v) {
+// ray_<hy>_map (geometry/ray_map.inl:15-21; TWICE) and the camera map (view/mapped.inl:20-26:
+// direction = mo_apply_dir, one normalize, then start): the nine divisions by |d|^2 share one
+// reciprocal, each normalize shares one; results are bit-identical to hy_map_ieee.
+template <bool TWICE> HT_D HyRay hy_map(const Mo &m, Q4 p, Q4 v) {
     DivCheck chk = div_check();
     Q4 u = q_addc(cq_mul(m.a, p), m.b);
     Q4 d = q_addc(cq_mul(m.c, p), m.d);
@@ -197,11 +200,13 @@ HT_D HyRay ray_hy_map(const Mo &m, Q4 p, Q4 v) {
     Q4 dc = q_conj(d);
     Q4 g22 = q4(k * dc.x, k * dc.y, k * dc.z, k * dc.w);
     Q4 g2 = q_mul(u, qdiv4(q_sub(g21, g22), rd, chk));
-    Q4 deriv = q_add(g1, g2);
-    o.v = normalize4_fast(normalize4_fast(deriv, chk), chk);
-    if (div_failed(chk)) return ray_hy_map_ieee(m, p, v);
+    o.v = normalize4_fast(q_add(g1, g2), chk);
+    if (TWICE) o.v = normalize4_fast(o.v, chk);
+    if (div_failed(chk)) return hy_map_ieee(m, p, v, TWICE);
     return o;
 }
+HT_D HyRay ray_hy_map(const Mo &m, Q4 p, Q4 v) { return hy_map<true>(m, p, v); }
+HT_D HyRay view_hy_map(const Mo &m, Q4 p, Q4 v) { return hy_map<false>(m, p, v); }
 // The same map, out of line: the object scan and the hit path share this one copy of its
 // code (instruction-cache footprint; an inlined copy in the scan measured slower).
 static __device__ __noinline__ HyRay ray_hy_map_call(const Mo m, const Q4 p, const Q4 v) { return ray_hy_map(m, p, v); }
@@ -210,26 +215,6 @@ HT_D Q4 mo_apply_pos(const Mo &m, Q4 p) {   // mo_apply_q (transform/moebius.cc:
     return q_mul(q_addc(cq_mul(m.a, p), m.b), q_inverse(q_addc(cq_mul(m.c, p), m.d)));
 }
 
-// Camera map (view/mapped.inl:20-26): direction = mo_apply_dir (one normalize), then start.
-// Once per sample, so plain IEEE division.
-HT_D HyRay view_hy_map(const Mo &m, Q4 p, Q4 v) {
-    Q4 u = q_addc(cq_mul(m.a, p), m.b);
-    Q4 d = q_addc(cq_mul(m.c, p), m.d);
-    float d2 = dot4(d, d);
-    Q4 di = q4(d.x / d2, (-d.y) / d2, (-d.z) / d2, (-d.w) / d2);
-    HyRay o;
-    o.p = q_mul(u, di);
-    Q4 g1 = q_mul(cq_mul(m.a, v), di);
-    Q4 cv = cq_mul(m.c, v);
-    Q4 g21 = q_conj(cv);
-    float k = (2.0f * dot4(d, cv)) / d2;
-    Q4 dc = q_conj(d);
-    Q4 g22 = q4(k * dc.x, k * dc.y, k * dc.z, k * dc.w);
-    Q4 t = q_sub(g21, g22);
-    Q4 g2 = q_mul(u, q4(t.x / d2, t.y / d2, t.z / d2, t.w / d2));
-    o.v = normalize4(q_add(g1, g2));
-    return o;
-}
 // c22_inverse_n (kernel/ocl/algebra/matrix_complex.cc:60-65): adjugate, det = 1 assumed.
 HT_D Mo mo_inverse(const Mo &m) {
     Mo r;

@@ -120,6 +120,27 @@ HT_D bool mixture_interact(const Material &m, uint32_t &rng, V3 normal, V3 &dir,
     return false;
 }
 
+// The interaction on a path's last hop: the same draws (the pixel's RNG goes on from them) and the
+// emission, without the direction that nothing will follow -- and so without the hit point and
+// the ray maps that only it needs.
+HT_D void mixture_last(const Material &m, uint32_t &rng, const Col &intensity, Col &emission) {
+    float alpha = rng_uniform(rng);
+    alpha -= m.diffuse;
+    if (alpha < 0.0f) {
+        rng_next(rng);
+        rng_next(rng);
+        return;
+    }
+    alpha -= m.specular;
+    if (alpha < 0.0f) return;
+    alpha -= m.luminous;
+    if (alpha < 0.0f) {
+        emission.x += intensity.x * m.emission.x;
+        emission.y += intensity.y * m.emission.y;
+        emission.z += intensity.z * m.emission.z;
+    }
+}
+
 // Staged scene, per slot in shared memory (hyperbolic scenes: planes first, then
 // horospheres, each in scene order; Euclidean scenes: slot = scene index).
 struct StagedScene {
@@ -216,7 +237,8 @@ static __device__ __noinline__ HyPath camera_hy(const StagedScene &s, float px, 
     return o;
 }
 
-// One hop (one iteration of render/scene.inl:25-41). Returns true while the path goes on.
+// One hop (one iteration of render/scene.inl:25-41). Returns true while the path goes on; `last`:
+// it ends here whatever is hit.
 // `hit` reports whether the scan found an object (for the hop statistics).
 // ---------------------------------------------------------------- the scan's packed point bound
 // Objects the upper estimate looks at: the first half of them planes, the others horospheres, the
@@ -331,7 +353,7 @@ HT_D uint32_t warp_survivors(const StagedScene &s, uint32_t c0, uint32_t valid, 
 // call together, uniform across the warp) turns it on.
 template <bool WARP = false>
 HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &prev_hash,
-                 Col &intensity, Col &emission, bool &hit, uint32_t &n_exact, bool full_warp = false) {
+                 Col &intensity, Col &emission, bool &hit, uint32_t &n_exact, bool last, bool full_warp = false) {
     // Nearest hit with ties to the lowest scene index (object/vector.inl:37-50): candidates
     // are compared on (distance, index), so the order of the slots does not matter; x =
     // cosh(distance) is compared first and the logarithm taken only when x can win; objects
@@ -426,8 +448,12 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
         return false;
     }
     hit = true;
-    const Mo inv = mo_from(s.inv[2 * kmin], s.inv[2 * kmin + 1]);
     const uint8_t *obj = s.objects + (size_t)kmin_orig * OBJ_STRIDE;
+    if (last) {
+        mixture_last(load_material(obj), rng, intensity, emission);
+        return false;
+    }
+    const Mo inv = mo_from(s.inv[2 * kmin], s.inv[2 * kmin + 1]);
     const Mo fwd = load_mo(obj);
     const bool repeat = (kmin_orig == prev_hash);
     HyRay l;   // the winner's local ray, as the scan computed it (the same map, the same bits)
@@ -491,7 +517,7 @@ HT_D EuPath camera_eu(const StagedScene &s, float px, float py, float size, uint
 }
 
 HT_D bool hop_eu(const StagedScene &s, EuPath &ray, uint32_t &rng, uint32_t &prev_hash,
-                 Col &intensity, Col &emission, bool &hit, uint32_t &n_exact) {
+                 Col &intensity, Col &emission, bool &hit, uint32_t &n_exact, bool last) {
     // Per chunk of 32 objects: the bounds of every object (warp-uniform, broadcast loads; 20
     // instructions against 110 of an exact test), then each lane's survivors in index order, so
     // that the reference's comparison (object/vector.inl:37-50) is unchanged. 25 objects: 0.8 exact
@@ -541,8 +567,12 @@ HT_D bool hop_eu(const StagedScene &s, EuPath &ray, uint32_t &rng, uint32_t &pre
         return false;
     }
     hit = true;
-    const Hom inv = hom_from(s.inv[2 * kmin], s.inv[2 * kmin + 1]);
     const uint8_t *obj = s.objects + (size_t)kmin * OBJ_STRIDE;
+    if (last) {
+        mixture_last(load_material(obj), rng, intensity, emission);
+        return false;
+    }
+    const Hom inv = hom_from(s.inv[2 * kmin], s.inv[2 * kmin + 1]);
     const Hom fwd = load_hom(obj);
     EuRay l;   // the winner's local ray, as the scan computed it; min_dist is its test's root
     {

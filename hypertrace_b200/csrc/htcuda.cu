@@ -40,34 +40,24 @@ thread_local std::string g_last_error;
 // Minimum resident blocks per SM requested from ptxas for the render kernels (register cap).
 // The scan is latency-bound on dependent FP32 chains, so resident warps matter, but the
 // packed point-bound loop and the slot bookkeeping hold more values than the earlier scan.
-// Measured on the current code at 1080p / 200 objects (Msamples/s): 7 -> 6 -> 5 blocks (72 ->
-// 80 -> 96 registers) took the wavefront kernel 368.6 -> 373.2 -> 377.4 and the batched mix
-// (spp / 16) 994 -> 1012 -> 1019; the one-pass kernel 288.6 -> 296.5 -> 295.6. The earlier
-// scan had measured 7 best (239.5 against 232 for 6). With the coherence sort and the warp
-// pre-cull, 6 -> 5 -> 4 blocks gave the single-view wavefront kernel 489.5 -> 493.0 -> 508.1
-// and the batched kernels (mix at spp / 16) 1170.8 -> 1210.2 -> 1172.2, so the two now have
-// caps of their own; 3 blocks for the later hops measured 462.2, 6 for hop 0 508.6 (510.3).
+// Measured at 4 / 5 / 6 blocks: later hops of the wavefronts 9.30 / 9.32 / - ms (1080p, 200 objects, 8
+// passes), hop 0 9.35 / 9.30 / 9.24 ms (and 4.87 / 4.92 / 4.74 ms, Euclidean 1917x1077, 16 passes), the
+// batched kernels 37.3 / 36.2 / 37.7 ms (24 mixed views), the one-pass kernel - / 3.32 / 3.43 ms, 8 blocks
+// 3.48 (one pass of the 1080p frame).
 #ifndef HT_PERSIST_MINB
 #define HT_PERSIST_MINB 6
 #endif
 #ifndef HT_PLAIN_MINB
-#define HT_PLAIN_MINB 6
+#define HT_PLAIN_MINB 5
 #endif
 #ifndef HT_WAVE_MINB    // render_wave, hop depths after the first
 #define HT_WAVE_MINB 4
 #endif
-#ifndef HT_WAVE0_MINB   // render_wave, hop depth 0 (camera rays: 0.764 ms per launch at 5, 0.792 at 4)
-#define HT_WAVE0_MINB 5
+#ifndef HT_WAVE0_MINB   // render_wave, hop depth 0
+#define HT_WAVE0_MINB 6
 #endif
 #ifndef HT_BATCH_MINB   // render_batch_wave (one recipe per kernel)
 #define HT_BATCH_MINB 5
-#endif
-// htc_render_passes: 2 = wavefronts (one launch per hop depth), 1 = the persistent kernel,
-// 0 = one launch of the one-pass kernel per pass. All three give the same bits. Measured at
-// 1920x1080 / 200 objects / H = 8 (Msamples/s): wavefronts 286.9, one-pass kernel 239.3,
-// persistent kernel 208.6.
-#ifndef HT_PASSES_MODE
-#define HT_PASSES_MODE 2
 #endif
 #ifndef HT_BATCH_SORT   // coherence sort of the batch's hyperbolic views
 #define HT_BATCH_SORT 1
@@ -109,7 +99,6 @@ struct htc_program {
     int address_width;
     uint32_t flags;
     uint32_t *d_err;     // device error word
-    uint32_t *d_queue;   // [0] next pixel, [1] finished blocks (persistent kernel)
     int num_sms;
     int max_smem;
     GenericProgram *generic;   // scene types served by render_generic (htgeneric.cu), else NULL
@@ -120,6 +109,9 @@ struct htc_program {
     size_t sort_slots;
     float4 *image;             // the scene's image (stage_image), grown on demand
     size_t image_cap;          // its size in float4
+    cudaMemPool_t pool;        // workspaces of wavefronts that a call takes and gives back (render_wave_pooled)
+    std::mutex pool_mutex;
+    size_t pool_keep;          // the largest workspace so far: what the pool keeps between calls
     int double_support;        // scene bytes in the double_support layout, narrowed before rendering
     uint8_t *narrow_buf;       // the narrowed (f32 layout) scene, grown on demand
     size_t narrow_bytes;
@@ -403,10 +395,10 @@ __device__ __forceinline__ typename PathOf<R>::T camera(const StagedScene &s, fl
 template <int R, bool WARP = false>
 __device__ __forceinline__ bool hop(const StagedScene &s, typename PathOf<R>::T &ray, uint32_t &rng,
                                     uint32_t &prev_hash, Col &intensity, Col &emission, bool &hit,
-                                    uint32_t &n_exact, bool full_warp = false) {
+                                    uint32_t &n_exact, bool last, bool full_warp = false) {
     if constexpr (R == RECIPE_HY)
-        return hop_hy<WARP>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact, full_warp);
-    else return hop_eu(s, ray, rng, prev_hash, intensity, emission, hit, n_exact);
+        return hop_hy<WARP>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact, last, full_warp);
+    else return hop_eu(s, ray, rng, prev_hash, intensity, emission, hit, n_exact, last);
 }
 
 // Pixel centre and size (render.cl:12-18).
@@ -465,7 +457,7 @@ __global__ void __launch_bounds__(128, HT_PLAIN_MINB) render_plain(
         for (uint32_t i = 0; i < hops; ++i) {
             bool hit;
             n_hops += 1;
-            bool go = hop<R>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact);
+            bool go = hop<R>(s, ray, rng, prev_hash, intensity, emission, hit, n_exact, i + 1 == hops);
             n_hits += hit ? 1 : 0;
             if (!go) break;
         }
@@ -562,7 +554,7 @@ __device__ __forceinline__ void trace_pixels(const StagedScene &s, uint32_t *cou
         if (in_path) {
             bool hit;
             st.hops += 1;
-            bool go = hop<R>(s, ray, rng, prev_hash, intensity, emission, hit, st.exact);
+            bool go = hop<R>(s, ray, rng, prev_hash, intensity, emission, hit, st.exact, hop_i + 1 >= hops);
             st.hits += hit ? 1 : 0;
             hop_i += 1;
             if (!go || hop_i >= hops) {
@@ -705,9 +697,9 @@ __device__ __forceinline__ void wave_chunk(const StagedScene &s, uint32_t base, 
         bool hit;
         st.hops += 1;
         st.tests += s.n;
-        const bool go = hop<R, true>(s, ray, rng, prev_hash, intensity, emission, hit, st.exact, full_warp);
+        const bool go = hop<R, true>(s, ray, rng, prev_hash, intensity, emission, hit, st.exact, last_hop, full_warp);
         st.hits += hit ? 1 : 0;
-        cont = go && !last_hop;
+        cont = go;
         if (!cont) {
             st.samples += 1;
             float4 c = canvas[pixel];
@@ -1491,20 +1483,25 @@ int htc_program_create(int recipe, uint32_t light_hops, int address_width, int d
     cudaError_t e = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e == cudaSuccess) e = cudaMalloc(&p->d_err, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_queue, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(p->d_err, 0, sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(p->d_queue, 0, 2 * sizeof(uint32_t));
     if (e != cudaSuccess) {
         if (p->d_err) cudaFree(p->d_err);
-        if (p->d_queue) cudaFree(p->d_queue);
         delete p;
         return cuda_fail(e, "htc_program_create");
+    }
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    if (cudaMemPoolCreate(&p->pool, &props) != cudaSuccess) {   // without one, the calls that would use it run the one-pass kernel
+        cudaGetLastError();
+        p->pool = nullptr;
     }
     p->max_smem -= 1024;   // static shared memory of the kernels
     int rc = recipe == HTC_RECIPE_HY ? set_smem_attr<RECIPE_HY>(p->max_smem) : set_smem_attr<RECIPE_EU>(p->max_smem);
     if (rc) {
         cudaFree(p->d_err);
-        cudaFree(p->d_queue);
+        if (p->pool) cudaMemPoolDestroy(p->pool);
         delete p;
         return rc;
     }
@@ -1515,11 +1512,11 @@ int htc_program_create(int recipe, uint32_t light_hops, int address_width, int d
 void htc_program_destroy(htc_program *p) {
     if (!p) return;
     cudaFree(p->d_err);
-    if (p->d_queue) cudaFree(p->d_queue);
     if (p->wave_buf) cudaFree(p->wave_buf);
     if (p->d_wave_ctr) cudaFree(p->d_wave_ctr);
     if (p->sort_buf) cudaFree(p->sort_buf);
     if (p->image) cudaFree(p->image);
+    if (p->pool) cudaMemPoolDestroy(p->pool);
     if (p->narrow_buf) cudaFree(p->narrow_buf);
     if (p->generic) generic_program_destroy(p->generic);
     delete p;
@@ -1638,13 +1635,9 @@ static int narrow_scene(htc_program *p, const void **scene, size_t *scene_size, 
     return HTC_OK;
 }
 
-static int render_ex_impl(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
-                          float *canvas, uint32_t *seeds, uint64_t *stats, void *stream) {
-    if (p && p->generic) return render_generic_program(p, W, H, scene, scene_size, canvas, seeds, 1, stats, stream);
-    uint32_t max_objects = 0;
-    size_t smem = 0;
-    int rc = validate_render_args(p, W, H, scene, scene_size, canvas, seeds, &max_objects, &smem);
-    if (rc) return rc;
+// One pass with the one-pass kernel (checked arguments).
+static int render_plain_pass(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, uint32_t max_objects,
+                             size_t smem, float *canvas, uint32_t *seeds, uint64_t *stats, void *stream) {
     dim3 grid((W + 31) / 32, (H + 3) / 4);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const uint8_t *sc = reinterpret_cast<const uint8_t *>(scene);
@@ -1659,23 +1652,6 @@ static int render_ex_impl(htc_program *p, uint32_t W, uint32_t H, const void *sc
     return HTC_OK;
 }
 
-extern "C" {
-
-int htc_render_ex(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
-                  float *canvas, uint32_t *seeds, uint64_t *stats, void *stream) {
-    if (p && canvas && seeds && W && H) {   // argument errors are reported by the render checks
-        int rc = narrow_scene(p, &scene, &scene_size, stream);
-        if (rc) return rc;
-    }
-    return render_ex_impl(p, W, H, scene, scene_size, canvas, seeds, stats, stream);
-}
-
-int htc_render(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, float *canvas,
-               uint32_t *seeds, void *stream) {
-    return htc_render_ex(p, W, H, scene, scene_size, canvas, seeds, nullptr, stream);
-}
-
-}  // extern "C"
 
 // Whether a call's hyperbolic wavefronts are sorted between hop depths. The two sort launches
 // cost 15 us per depth on small queues and 50 us on 2 M paths; below 2^19 pixels or 100 objects
@@ -1719,9 +1695,38 @@ static int wave_reserve(htc_program *p, size_t slots, uint32_t max_objects) {
     p->wave_slots = slots;
     return HTC_OK;
 }
-static WaveQueue wave_queue(htc_program *p, int which) {
-    const size_t n = p->wave_slots;
-    uint8_t *b = reinterpret_cast<uint8_t *>(p->wave_buf) + (size_t)which * WAVE_SLOT_BYTES * n;
+// What one call's launches work in: the program's own buffers, or a block of its pool.
+struct WaveWork {
+    float4 *image;
+    uint32_t *ctr;      // 4 words per hop depth
+    void *sort;
+    size_t sort_slots;
+    void *queues;
+    size_t slots;       // per queue
+};
+static WaveWork wave_work_owned(const htc_program *p) {
+    return WaveWork{p->image, p->d_wave_ctr, p->sort_buf, p->sort_slots, p->wave_buf, p->wave_slots};
+}
+// The same laid out in one block at `base`; returns its size.
+static size_t wave_work_block(const htc_program *p, uint64_t pixels, uint32_t max_objects, uint8_t *base, WaveWork *w) {
+    const size_t slots = (size_t)((pixels + 63) & ~(uint64_t)63);
+    size_t at = 0;
+    const auto take = [&](size_t bytes) {
+        uint8_t *r = base + at;
+        at += (bytes + 255) & ~(size_t)255;
+        return r;
+    };
+    w->image = reinterpret_cast<float4 *>(take(sizeof(float4) * image_words(max_objects)));
+    w->ctr = reinterpret_cast<uint32_t *>(take(4 * sizeof(uint32_t) * (size_t)p->hops));
+    w->sort_slots = p->recipe == HTC_RECIPE_HY && wave_sorted(p, pixels, max_objects) ? slots : 0;
+    w->sort = take(w->sort_slots ? sort_bytes(slots, (uint32_t)p->num_sms) : 0);
+    w->queues = take(2 * WAVE_SLOT_BYTES * slots);
+    w->slots = slots;
+    return at;
+}
+static WaveQueue wave_queue(const WaveWork &w, int which) {
+    const size_t n = w.slots;
+    uint8_t *b = reinterpret_cast<uint8_t *>(w.queues) + (size_t)which * WAVE_SLOT_BYTES * n;
     WaveQueue q;
     q.p = reinterpret_cast<float4 *>(b);
     q.v = q.p + n;
@@ -1732,7 +1737,7 @@ static WaveQueue wave_queue(htc_program *p, int which) {
     return q;
 }
 template <int R>
-static int launch_wave(htc_program *p, uint32_t W, uint32_t H, const uint8_t *sc, size_t scene_size,
+static int launch_wave(const htc_program *p, const WaveWork &w, uint32_t W, uint32_t H, const uint8_t *sc, size_t scene_size,
                        uint32_t max_objects, size_t smem, float4 *cv, uint32_t *seeds, uint32_t passes,
                        uint64_t *stats, cudaStream_t st) {
     int per_sm = 0;
@@ -1745,21 +1750,21 @@ static int launch_wave(htc_program *p, uint32_t W, uint32_t H, const uint8_t *sc
     const uint64_t needed = ((uint64_t)W * H + 127) / 128;
     const uint64_t blocks = std::min<uint64_t>((uint64_t)per_sm * (uint64_t)p->num_sms, needed);
     const uint64_t blocks0 = std::min<uint64_t>((uint64_t)per_sm0 * (uint64_t)p->num_sms, needed);
-    const WaveQueue q[2] = {wave_queue(p, 0), wave_queue(p, 1)};
+    const WaveQueue q[2] = {wave_queue(w, 0), wave_queue(w, 1)};
     const WaveQueue none = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     const bool sorted = R == RECIPE_HY && wave_sorted(p, (uint64_t)W * H, max_objects);
     const unsigned sort_blocks = (unsigned)p->num_sms;
-    const SortBuf sb = sorted ? sort_buf_at(p->sort_buf, p->sort_slots, sort_blocks) : SortBuf{};
+    const SortBuf sb = sorted ? sort_buf_at(w.sort, w.sort_slots, sort_blocks) : SortBuf{};
     const size_t sort_smem = sizeof(uint32_t) * SORT_BINS;
     uint32_t sorts = 0;   // both histograms start cleared; k_sort_scatter clears the one its depth did not use
     if (sorted) HTC_CUDA(cudaMemsetAsync(sb.hist, 0, 2 * sizeof(uint32_t) * SORT_BINS, st));
     // two sets of counters in turn: a pass's hop 0 clears the next one's
     const uint32_t n_ctr = 2 * p->hops;
-    HTC_CUDA(cudaMemsetAsync(p->d_wave_ctr, 0, 2 * sizeof(uint32_t) * (size_t)n_ctr, st));
-    k_stage<R><<<1, STAGE_THREADS, 0, st>>>(sc, scene_size, max_objects, p->address_width, p->d_err, p->image);
+    HTC_CUDA(cudaMemsetAsync(w.ctr, 0, 2 * sizeof(uint32_t) * (size_t)n_ctr, st));
+    k_stage<R><<<1, STAGE_THREADS, 0, st>>>(sc, scene_size, max_objects, p->address_width, p->d_err, w.image);
     HTC_CUDA(cudaGetLastError());
     for (uint32_t pass = 0; pass < passes; ++pass) {
-        uint32_t *ctr = p->d_wave_ctr + (size_t)(pass & 1u) * n_ctr, *next = p->d_wave_ctr + (size_t)(~pass & 1u) * n_ctr;
+        uint32_t *ctr = w.ctr + (size_t)(pass & 1u) * n_ctr, *next = w.ctr + (size_t)(~pass & 1u) * n_ctr;
         for (uint32_t h = 0; h < p->hops; ++h) {
             WaveQueue in = h == 0 ? none : q[(h - 1) & 1];
             const uint32_t *in_count = h == 0 ? nullptr : ctr + 2 * (h - 1) + 1;
@@ -1771,16 +1776,70 @@ static int launch_wave(htc_program *p, uint32_t W, uint32_t H, const uint8_t *sc
                 in.o = sb.perm;
             }
             HTC_CUDA(launch(true, h == 0 ? render_wave<R, 1> : render_wave<R, 2>, (unsigned)(h == 0 ? blocks0 : blocks),
-                            BLOCK_THREADS, smem, st, p->image, sc, max_objects, pass + h > 0, W, H, p->hops, h, p->flags, cv, seeds,
+                            BLOCK_THREADS, smem, st, w.image, sc, max_objects, pass + h > 0, W, H, p->hops, h, p->flags, cv, seeds,
                             stats, in, in_count, q[h & 1], ctr + 2 * h, next, n_ctr));
         }
     }
     return HTC_OK;
 }
 
-extern "C" {
+static int launch_wave_any(const htc_program *p, const WaveWork &w, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
+                           uint32_t max_objects, size_t smem, float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats,
+                           cudaStream_t st) {
+    const uint8_t *sc = reinterpret_cast<const uint8_t *>(scene);
+    float4 *cv = reinterpret_cast<float4 *>(canvas);
+    return p->recipe == HTC_RECIPE_HY
+        ? launch_wave<RECIPE_HY>(p, w, W, H, sc, scene_size, max_objects, smem, cv, seeds, passes, stats, st)
+        : launch_wave<RECIPE_EU>(p, w, W, H, sc, scene_size, max_objects, smem, cv, seeds, passes, stats, st);
+}
 
-}  // extern "C"
+// Whether one pass is faster as wavefronts than with the one-pass kernel. Small canvases leave the
+// deeper hop launches most of the GPU idle; a hop count beyond the workloads' would add launches
+// for queues that are empty. Measured, one call of one pass, one-pass kernel / wavefronts in us:
+// hyperbolic scenes of 18, 77, 200 objects at 400x300 132/145, 234/257, 298/306, at 512x384 184/171,
+// 333/300, 402/342, at 800x600 358/309, 646/479, 821/471; Euclidean scenes of 9, 25, 33 objects at
+// 1024x768 88/107, 176/179, 279/269, at 1600x900 139/151, 282/250, 425/359.
+constexpr uint32_t WAVE_MAX_HOPS = 16;
+static bool wave_pays(const htc_program *p, uint64_t pixels, uint32_t max_objects) {
+    if (p->hops > WAVE_MAX_HOPS) return false;
+    return p->recipe == HTC_RECIPE_HY ? pixels >= 9u << 14 : pixels >= (1u << 20) && max_objects >= 16;
+}
+
+// Wavefronts in a workspace taken from the program's pool and given back in stream order, so that
+// calls of one program on several streams or threads do not meet. *done = false: none was to be
+// had (no pool, no memory, a capturing stream); nothing was launched.
+static int render_wave_pooled(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, uint32_t max_objects,
+                              size_t smem, float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, cudaStream_t st,
+                              bool *done) {
+    *done = false;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!p->pool || cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return HTC_OK;
+    }
+    WaveWork w;
+    const size_t bytes = wave_work_block(p, (uint64_t)W * H, max_objects, nullptr, &w);
+    {   // the pool keeps two workspaces of the largest size between calls; its reservations are larger
+        // than what is taken from them, and one over the limit would go back to the system at
+        // every synchronisation (200 us a call)
+        std::lock_guard<std::mutex> lock(p->pool_mutex);
+        if (bytes > p->pool_keep) {
+            uint64_t keep = 2 * (uint64_t)bytes + (64u << 20);
+            HTC_CUDA(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+            p->pool_keep = bytes;
+        }
+    }
+    void *block = nullptr;
+    if (cudaMallocFromPoolAsync(&block, bytes, p->pool, st) != cudaSuccess) {
+        cudaGetLastError();
+        return HTC_OK;
+    }
+    *done = true;
+    wave_work_block(p, (uint64_t)W * H, max_objects, reinterpret_cast<uint8_t *>(block), &w);
+    const int rc = launch_wave_any(p, w, W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats, st);
+    const cudaError_t e = cudaFreeAsync(block, st);
+    return rc ? rc : e != cudaSuccess ? cuda_fail(e, "cudaFreeAsync") : HTC_OK;
+}
 
 static int render_wavefront_impl(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
                                  float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, void *stream) {
@@ -1792,15 +1851,36 @@ static int render_wavefront_impl(htc_program *p, uint32_t W, uint32_t H, const v
     if (passes == 0) return HTC_OK;
     rc = wave_reserve(p, (size_t)W * H, max_objects);
     if (rc) return rc;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const uint8_t *sc = reinterpret_cast<const uint8_t *>(scene);
-    float4 *cv = reinterpret_cast<float4 *>(canvas);
-    if (p->recipe == HTC_RECIPE_HY)
-        return launch_wave<RECIPE_HY>(p, W, H, sc, scene_size, max_objects, smem, cv, seeds, passes, stats, st);
-    return launch_wave<RECIPE_EU>(p, W, H, sc, scene_size, max_objects, smem, cv, seeds, passes, stats, st);
+    return launch_wave_any(p, wave_work_owned(p), W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats,
+                           reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" {
+
+int htc_render_ex(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
+                  float *canvas, uint32_t *seeds, uint64_t *stats, void *stream) {
+    if (p && p->generic) return render_generic_program(p, W, H, scene, scene_size, canvas, seeds, 1, stats, stream);
+    if (p && canvas && seeds && W && H) {   // argument errors are reported by the render checks
+        int rc = narrow_scene(p, &scene, &scene_size, stream);
+        if (rc) return rc;
+    }
+    uint32_t max_objects = 0;
+    size_t smem = 0;
+    int rc = validate_render_args(p, W, H, scene, scene_size, canvas, seeds, &max_objects, &smem);
+    if (rc) return rc;
+    if (wave_pays(p, (uint64_t)W * H, max_objects)) {
+        bool done = false;
+        rc = render_wave_pooled(p, W, H, scene, scene_size, max_objects, smem, canvas, seeds, 1, stats,
+                                reinterpret_cast<cudaStream_t>(stream), &done);
+        if (rc || done) return rc;
+    }
+    return render_plain_pass(p, W, H, scene, scene_size, max_objects, smem, canvas, seeds, stats, stream);
+}
+
+int htc_render(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, float *canvas,
+               uint32_t *seeds, void *stream) {
+    return htc_render_ex(p, W, H, scene, scene_size, canvas, seeds, nullptr, stream);
+}
 
 int htc_render_wavefront(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
                          float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, void *stream) {
@@ -1823,43 +1903,21 @@ int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene,
     int rc = validate_render_args(p, W, H, scene, scene_size, canvas, seeds, &max_objects, &smem);
     if (rc) return rc;
     if (passes == 0) return HTC_OK;
-    // Small canvases of cheap scenes run the one-pass kernel: their deeper hop launches would
-    // leave most of the GPU idle (measured per view, 256x256 and 640x480: Euclidean 26.9 vs
-    // 34.6 ms, hyperbolic with fewer than 100 objects 122.7 vs 131.5 ms, one-pass vs
-    // wavefronts). Either way the result is the same bits.
-    const bool cheap = (uint64_t)W * H < (1u << 19) && (p->recipe == HTC_RECIPE_EU || max_objects < 100);
-    if (HT_PASSES_MODE == 2 && !cheap)
+    // The program keeps queues of its own for large canvases and for hyperbolic scenes of 100 objects
+    // on; the other calls may run on several streams at once and work in the pool.
+    const uint64_t pixels = (uint64_t)W * H;
+    if (pixels >= (1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100))
         return render_wavefront_impl(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);
-    if (HT_PASSES_MODE == 0 || HT_PASSES_MODE == 2) {
-        for (uint32_t k = 0; k < passes; ++k) {
-            int rc2 = render_ex_impl(p, W, H, scene, scene_size, canvas, seeds, stats, stream);
-            if (rc2) return rc2;
-        }
-        return HTC_OK;
+    if (wave_pays(p, pixels, max_objects)) {
+        bool done = false;
+        rc = render_wave_pooled(p, W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats,
+                                reinterpret_cast<cudaStream_t>(stream), &done);
+        if (rc || done) return rc;
     }
-    int per_sm = 0;
-    cudaError_t e;
-    if (p->recipe == HTC_RECIPE_HY)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_persistent<RECIPE_HY>, 128, smem);
-    else
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, render_persistent<RECIPE_EU>, 128, smem);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (per_sm < 1) per_sm = 1;
-    uint64_t blocks = (uint64_t)per_sm * (uint64_t)p->num_sms;
-    const uint64_t needed = ((uint64_t)W * H + 127) / 128;
-    if (blocks > needed) blocks = needed;
-    cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const uint8_t *sc = reinterpret_cast<const uint8_t *>(scene);
-    float4 *cv = reinterpret_cast<float4 *>(canvas);
-    if (p->recipe == HTC_RECIPE_HY)
-        render_persistent<RECIPE_HY><<<(unsigned)blocks, 128, smem, st>>>(sc, scene_size, max_objects, p->address_width, W, H,
-                                                                          p->hops, passes, p->flags, cv, seeds, stats,
-                                                                          p->d_err, p->d_queue);
-    else
-        render_persistent<RECIPE_EU><<<(unsigned)blocks, 128, smem, st>>>(sc, scene_size, max_objects, p->address_width, W, H,
-                                                                          p->hops, passes, p->flags, cv, seeds, stats,
-                                                                          p->d_err, p->d_queue);
-    HTC_CUDA(cudaGetLastError());
+    for (uint32_t k = 0; k < passes; ++k) {
+        rc = render_plain_pass(p, W, H, scene, scene_size, max_objects, smem, canvas, seeds, stats, stream);
+        if (rc) return rc;
+    }
     return HTC_OK;
 }
 

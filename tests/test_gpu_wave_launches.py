@@ -28,11 +28,24 @@ def _bits(canvas):
     return canvas.image.cpu().numpy().view(np.uint32), canvas.seeds.cpu().numpy()
 
 
+def _capture(render, buffer, canvas, passes, stats=None):
+    """`passes` one-pass calls, captured and replayed: on a capturing stream a call has no workspace
+    and runs the one-pass kernel, whatever the canvas."""
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            render.render(buffer, canvas, stats=stats, sync=False)
+        for _ in range(passes):
+            graph.replay()
+        stream.synchronize()
+
+
 def _plain(ctx, sc, W, H, passes):
     render, buffer, canvas = P.Render(ctx, sc.recipe, sc.hops), P.EntityBuffer(ctx, sc), P.Canvas(ctx, (W, H), 5)
     stats = torch.zeros(8, dtype=torch.int64, device=ctx.device)
-    for _ in range(passes):
-        render.render(buffer, canvas, stats=stats)
+    _capture(render, buffer, canvas, passes, stats)
     return _bits(canvas), stats.cpu().tolist()
 
 
@@ -74,3 +87,47 @@ def test_captured_wavefronts_replay(built, hops, passes):
         stream.synchronize()
     got = _bits(canvas)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("geometry,n,W,H,hops", [("hy", 40, 512, 288, 4), ("hy", 40, 511, 289, 4), ("hy", 130, 1031, 521, 4),
+                                                ("hy", 40, 512, 288, 17), ("eu", 16, 1024, 1024, 3), ("eu", 15, 1024, 1024, 3)])
+def test_one_pass_calls_on_two_streams(built, geometry, n, W, H, hops):
+    """One program, one-pass and small multi-pass calls on two streams at once: each call works in
+    memory of its own, and both canvases come out as on one stream (sizes around the least that
+    render as wavefronts)."""
+    ctx = P.Context(0)
+    sc = _scene(geometry, n, hops)
+    render, buffer = P.Render(ctx, sc.recipe, sc.hops), P.EntityBuffer(ctx, sc)
+    canvases = [P.Canvas(ctx, (W, H), s) for s in (5, 6, 5, 6)]
+    for c in canvases[2:]:
+        for _ in range(4):
+            render.render(buffer, c)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    small = W * H < 1 << 19 and n < 100
+    for k in range(2):
+        for c, stream in zip(canvases[:2], streams):
+            with torch.cuda.stream(stream):
+                render.render(buffer, c, sync=False)
+                if small:
+                    render.render_passes(buffer, c, 1, sync=False)
+                else:
+                    render.render(buffer, c, sync=False)
+    torch.cuda.synchronize()
+    for a, b in zip(canvases[:2], canvases[2:]):
+        assert np.array_equal(_bits(a)[0], _bits(b)[0]) and np.array_equal(_bits(a)[1], _bits(b)[1])
+
+
+@pytest.mark.parametrize("geometry,n,W,H,hops", [("hy", 130, 1031, 521, 4), ("hy", 20, 400, 300, 3), ("hy", 20, 512, 289, 3),
+                                                ("eu", 20, 1200, 900, 5)])
+def test_one_pass_calls_equal_one_pass_kernel(built, geometry, n, W, H, hops):
+    ctx = P.Context(0)
+    sc = _scene(geometry, n, hops)
+    want, want_stats = _plain(ctx, sc, W, H, 3)
+    render, buffer, canvas = P.Render(ctx, sc.recipe, sc.hops), P.EntityBuffer(ctx, sc), P.Canvas(ctx, (W, H), 5)
+    stats = torch.zeros(8, dtype=torch.int64, device=ctx.device)
+    render.render(buffer, canvas, stats=stats)
+    render.render_passes(buffer, canvas, 2, stats=stats)
+    got = _bits(canvas)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert stats.cpu().tolist() == want_stats
