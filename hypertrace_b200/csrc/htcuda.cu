@@ -109,9 +109,7 @@ struct htc_program {
     size_t sort_slots;
     float4 *image;             // the scene's image (stage_image), grown on demand
     size_t image_cap;          // its size in float4
-    cudaMemPool_t pool;        // workspaces of wavefronts that a call takes and gives back (render_wave_pooled)
-    std::mutex pool_mutex;
-    size_t pool_keep;          // the largest workspace so far: what the pool keeps between calls
+    int device;                // whose pool it uses (render_wave_pooled); -1: none
     int double_support;        // scene bytes in the double_support layout, narrowed before rendering
     uint8_t *narrow_buf;       // the narrowed (f32 layout) scene, grown on demand
     size_t narrow_bytes;
@@ -1376,6 +1374,67 @@ __global__ void __launch_bounds__(256) k_fma_probe(float *out, int iters) {
     out[blockIdx.x * blockDim.x + threadIdx.x] = a0 + a1 + a2 + a3 + a4 + a5 + a6 + a7;
 }
 
+// ============================================================================ workspace pools
+// One memory pool per device for the workspaces that calls take and give back in stream order
+// (render_wave_pooled), shared by the device's programs so that a new program finds memory that
+// an earlier one's calls have mapped (a pool per program made its first call 2 to 15 ms long). Made
+// by the first call that needs it, destroyed with the last program; between calls it keeps two
+// workspaces of the largest size taken so far and 64 MB (its reservations are larger than what
+// is taken from them, and what is over the limit goes back to the system at every
+// synchronisation: 200 us a call).
+namespace {
+constexpr int MAX_DEVICES = 64;
+struct DevicePool {
+    std::mutex mutex;
+    cudaMemPool_t pool = nullptr;
+    uint32_t programs = 0;
+    size_t largest = 0;
+} g_pools[MAX_DEVICES];
+int pool_enter(int dev) {
+    if (dev < 0 || dev >= MAX_DEVICES) return -1;
+    std::lock_guard<std::mutex> lock(g_pools[dev].mutex);
+    ++g_pools[dev].programs;
+    return dev;
+}
+void pool_leave(int dev) {
+    if (dev < 0) return;
+    DevicePool &d = g_pools[dev];
+    std::lock_guard<std::mutex> lock(d.mutex);
+    if (--d.programs == 0 && d.pool) {
+        cudaMemPoolDestroy(d.pool);   // blocks still in use are freed with their last use
+        d.pool = nullptr;
+        d.largest = 0;
+    }
+}
+// A block of `bytes` for work on `st`, or NULL.
+void *pool_take(int dev, size_t bytes, cudaStream_t st) {
+    if (dev < 0) return nullptr;
+    DevicePool &d = g_pools[dev];
+    std::lock_guard<std::mutex> lock(d.mutex);
+    cudaError_t e = cudaSuccess;
+    if (!d.pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        e = cudaMemPoolCreate(&d.pool, &props);
+        if (e != cudaSuccess) d.pool = nullptr;
+    }
+    if (e == cudaSuccess && bytes > d.largest) {
+        uint64_t keep = 2 * (uint64_t)bytes + (64u << 20);
+        e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e == cudaSuccess) d.largest = bytes;
+    }
+    void *block = nullptr;
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&block, bytes, d.pool, st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();   // the caller renders without
+        return nullptr;
+    }
+    return block;
+}
+}  // namespace
+
 // ============================================================================ C ABI
 static int check_program(const htc_program *p) {
     if (!p) return fail(HTC_ERR_INVALID, "program is NULL");
@@ -1427,6 +1486,7 @@ static int wrap_generic(GenericProgram *g, int recipe, uint32_t light_hops, int 
     p->address_width = address_width;
     p->flags = flags;
     p->generic = g;
+    p->device = -1;
     cudaError_t e = cudaMalloc(&p->d_err, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(p->d_err, 0, sizeof(uint32_t));
     if (e != cudaSuccess) {
@@ -1489,22 +1549,14 @@ int htc_program_create(int recipe, uint32_t light_hops, int address_width, int d
         delete p;
         return cuda_fail(e, "htc_program_create");
     }
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    if (cudaMemPoolCreate(&p->pool, &props) != cudaSuccess) {   // without one, the calls that would use it run the one-pass kernel
-        cudaGetLastError();
-        p->pool = nullptr;
-    }
     p->max_smem -= 1024;   // static shared memory of the kernels
     int rc = recipe == HTC_RECIPE_HY ? set_smem_attr<RECIPE_HY>(p->max_smem) : set_smem_attr<RECIPE_EU>(p->max_smem);
     if (rc) {
         cudaFree(p->d_err);
-        if (p->pool) cudaMemPoolDestroy(p->pool);
         delete p;
         return rc;
     }
+    p->device = pool_enter(dev);
     *out = p;
     return HTC_OK;
 }
@@ -1516,7 +1568,7 @@ void htc_program_destroy(htc_program *p) {
     if (p->d_wave_ctr) cudaFree(p->d_wave_ctr);
     if (p->sort_buf) cudaFree(p->sort_buf);
     if (p->image) cudaFree(p->image);
-    if (p->pool) cudaMemPoolDestroy(p->pool);
+    pool_leave(p->device);
     if (p->narrow_buf) cudaFree(p->narrow_buf);
     if (p->generic) generic_program_destroy(p->generic);
     delete p;
@@ -1695,7 +1747,7 @@ static int wave_reserve(htc_program *p, size_t slots, uint32_t max_objects) {
     p->wave_slots = slots;
     return HTC_OK;
 }
-// What one call's launches work in: the program's own buffers, or a block of its pool.
+// What one call's launches work in: the program's own buffers, or a block of the device's pool.
 struct WaveWork {
     float4 *image;
     uint32_t *ctr;      // 4 words per hop depth
@@ -1805,35 +1857,23 @@ static bool wave_pays(const htc_program *p, uint64_t pixels, uint32_t max_object
     return p->recipe == HTC_RECIPE_HY ? pixels >= 9u << 14 : pixels >= (1u << 20) && max_objects >= 16;
 }
 
-// Wavefronts in a workspace taken from the program's pool and given back in stream order, so that
+// Wavefronts in a workspace taken from the device's pool and given back in stream order, so that
 // calls of one program on several streams or threads do not meet. *done = false: none was to be
-// had (no pool, no memory, a capturing stream); nothing was launched.
+// had (no memory, a capturing stream); nothing was launched.
 static int render_wave_pooled(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, uint32_t max_objects,
                               size_t smem, float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, cudaStream_t st,
                               bool *done) {
     *done = false;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (!p->pool || cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
         cudaGetLastError();
         return HTC_OK;
     }
+    if (capture != cudaStreamCaptureStatusNone) return HTC_OK;
     WaveWork w;
     const size_t bytes = wave_work_block(p, (uint64_t)W * H, max_objects, nullptr, &w);
-    {   // the pool keeps two workspaces of the largest size between calls; its reservations are larger
-        // than what is taken from them, and one over the limit would go back to the system at
-        // every synchronisation (200 us a call)
-        std::lock_guard<std::mutex> lock(p->pool_mutex);
-        if (bytes > p->pool_keep) {
-            uint64_t keep = 2 * (uint64_t)bytes + (64u << 20);
-            HTC_CUDA(cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &keep));
-            p->pool_keep = bytes;
-        }
-    }
-    void *block = nullptr;
-    if (cudaMallocFromPoolAsync(&block, bytes, p->pool, st) != cudaSuccess) {
-        cudaGetLastError();
-        return HTC_OK;
-    }
+    void *block = pool_take(p->device, bytes, st);
+    if (!block) return HTC_OK;
     *done = true;
     wave_work_block(p, (uint64_t)W * H, max_objects, reinterpret_cast<uint8_t *>(block), &w);
     const int rc = launch_wave_any(p, w, W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats, st);
