@@ -145,7 +145,7 @@ struct Ctx {
     Ptr bvec;
     const float4 *brec;
     const float *bmag;
-    const u32 *bkind;
+    const u32 *bkind;     // bits 0-1: kind, the rest: the element's index
     u32 culled;
     float4 *win;    // shared, this thread's 2 float4: the local ray of a bounded scan's winner
 };
@@ -1157,14 +1157,15 @@ template <class O0, class... O> struct ChoiceTraits<O0, O...> {
 
 // A vector of Moebius-mapped objects of a known shape gets distance bounds: one world-space
 // record per element (stage_bound of the element's map) in shared memory, staged once per
-// block by render_generic when the vector is the scene's top-level object and holds between
-// HTG_BOUND_MIN and HTG_BOUND_CAP elements (below 32 the bound arithmetic costs more than the
-// exact tests it saves: the hy.rs example's 4 objects ran 625 Msamples/s with it, 644 without).
+// block by render_generic when the vector is the scene's top-level object and holds up to
+// HTG_BOUND_CAP elements. With the elements ordered by distance even a few are worth it (hy_tiled
+// type at 800x600, 6 hops, 4 passes, with / without the bounds: 4 elements 1645 / 1738 us, 12 3008 /
+// 3616, 31 3414 / 7683; 64 in index order with an estimate over 32 6049, by distance over 16 3874).
+#ifndef HTG_EST   // elements the upper estimate looks at (64 at 1080p, 4 passes: 8 26.6 ms, 12 22.2, 16 22.1, 24 22.6)
+#define HTG_EST 16u
+#endif
 #ifndef HTG_BOUND_CAP
 #define HTG_BOUND_CAP 256u
-#endif
-#ifndef HTG_BOUND_MIN
-#define HTG_BOUND_MIN 32u
 #endif
 template <class G, class O> struct VecBounds { static constexpr bool ok = false; };
 template <class X> struct VecBounds<Hy, MappedObject<Hy, X, Moebius>> {
@@ -1174,26 +1175,48 @@ template <class X> struct VecBounds<Hy, MappedObject<Hy, X, Moebius>> {
     }
     template <int W> HT_D static Mo map_of(Ptr elem) { return Moebius::load(elem + Rec<W, Zst, Moebius, X>::off(1)); }
 };
-// Stages the records of the vector at `self` (all threads of the block; returns the element
-// count staged, or 0xFFFFFFFF when the vector is too small or too large for the bounds or its
-// count does not fit the bytes).
+// Where the view's rays start, for the order of the records (any point serves: it orders, no more).
+template <class V> struct ViewStart {
+    template <int W> HT_D static Q4 at(Ptr) { return Hy::origin(); }
+};
+template <class V> struct ViewStart<MappedView<Hy, V, Moebius>> {
+    template <int W> HT_D static Q4 at(Ptr self) { return mo_apply_pos(Moebius::load(self + Rec<W, Zst, Moebius, V>::off(1)), Hy::origin()); }
+};
+// Stages the records of the vector at `self` by their distance from `start` (ties by index), so
+// that the scan's estimate looks at the elements next to the paths (ht_trace.cuh does the same):
+// all threads of the block; returns the element count staged, or 0xFFFFFFFF when the vector is too
+// large for the bounds or its count does not fit the bytes.
 template <class G, class O, int W>
-HT_D u32 stage_vec_bounds(Ptr self, Ptr end, float4 *rec, float *mag, u32 *kind) {
+HT_D u32 stage_vec_bounds(Ptr self, Ptr end, Q4 start, float4 *rec, float *mag, u32 *kind, float *key) {
     typedef VecBounds<G, O> B;
     constexpr u32 stride = O::template lay<W>().size;
     constexpr u32 head = upm((u32)W, O::template lay<W>().align);
     const u32 n = ldusize<W>(self);
-    if (stride == 0 || end < self + head || n > (u32)((end - self - head) / stride) || n > HTG_BOUND_CAP ||
-        n < HTG_BOUND_MIN)
+    if (stride == 0 || end < self + head || n > (u32)((end - self - head) / stride) || n > HTG_BOUND_CAP)
         return 0xFFFFFFFFu;
     const float nan = __int_as_float(0x7fc00000);
+    const BoundRay at = bound_ray(start, q4(1.0f, 0.0f, 0.0f, 0.0f));
+    for (u32 i = threadIdx.x; i < n; i += blockDim.x) {   // the keys
+        const Ptr elem = self + head + i * stride;
+        const u32 k = B::template kind_of<W>(elem);
+        float m, d = 0.0f;   // elements without a record first
+        if (k <= 1u) {
+            const float F = bound_fw(stage_bound(B::template map_of<W>(elem), k, m), 0.0f, at).F / at.t;
+            d = logf(k == 0u ? 0.5f * fabsf(F) + sqrtf(fmaf(0.25f * F, F, 1.0f)) : fmaxf(F, 1.0f / F));   // asinh(F / 2), |ln F|
+        }
+        key[i] = d >= 0.0f ? d : 0.0f;
+    }
+    __syncthreads();
     for (u32 i = threadIdx.x; i < n; i += blockDim.x) {
+        const float mine = key[i];
+        u32 slot = 0;
+        for (u32 j = 0; j < n; ++j) slot += key[j] < mine || (key[j] == mine && j < i) ? 1u : 0u;
         const Ptr elem = self + head + i * stride;
         const u32 k = B::template kind_of<W>(elem);
         float m = 0.0f;
-        rec[i] = k <= 1u ? stage_bound(B::template map_of<W>(elem), k, m) : make_float4(nan, nan, nan, nan);
-        mag[i] = m;
-        kind[i] = k;
+        rec[slot] = k <= 1u ? stage_bound(B::template map_of<W>(elem), k, m) : make_float4(nan, nan, nan, nan);
+        mag[slot] = m;
+        kind[slot] = k | (i << 2);
     }
     return n;
 }
@@ -1204,15 +1227,16 @@ HT_D float ObjectVec<G, O>::detect(Ptr self, Ctx &c, Cache &cache, Light<G> &l) 
     else return detect_all<W, F>(self, c, cache, l);
 }
 
-// The scan of ObjectVec::detect_all for vectors of Moebius-mapped planes and horospheres. The
-// elements are visited in index order with the shape test of their kind directly (one copy of
-// the ray map and of the tests for all variants), the logarithm taken only where x = cosh of the
-// distance can win (hy_dist_from_x is non-decreasing), and the winner's local ray is kept for its
-// full detection: the same operations on the same values as detect_all, so the same bits.
+// The scan of ObjectVec::detect_all for vectors of Moebius-mapped planes and horospheres: the shape
+// test of an element's kind directly (one copy of the ray map and of the tests for all
+// variants), the logarithm taken only where x = cosh of the distance can win (hy_dist_from_x is
+// non-decreasing), and the winner's local ray kept for its full detection: the same operations on
+// the same values as detect_all, so the same bits; hits are compared on (distance, index), the
+// reference's nearest-hit rule, whatever the order.
 // When the kernel staged the vector's distance bounds, it culls as the hand-written hyperbolic
 // kernel does (ht_trace.cuh hop_hy): an upper estimate of the nearest sure crossing among the
-// first 32 elements sets a threshold before the first exact test, each chunk of 32 elements is
-// culled by the point bound (warp-uniform) and the ray-aware bound (per lane), and the
+// elements nearest the camera sets a threshold before the first exact test, each chunk of 32 elements
+// is culled by the point bound (warp-uniform) and the ray-aware bound (per lane), and the
 // survivors are tested with the threshold tightening on every nearer hit. Culling only skips
 // elements that cannot be nearer than the threshold.
 template <class G, class O> template <int W, bool F>
@@ -1228,14 +1252,16 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
     Limit lim = limit_none(br.t);
     if (can) {
         float best = __int_as_float(0x7f800000);
-        const u32 ne = n < 32u ? n : 32u;
+        const u32 ne = n < HTG_EST ? n : HTG_EST;
 #pragma unroll 1
-        for (u32 i = 0; i < ne; ++i)   // warp-uniform: broadcast loads
-            best = fminf(best, sure_crossing_e2(bound_fw(c.brec[i], c.bmag[i], br), c.bkind[i], i + h0 == c.prev, br.t));
+        for (u32 q = 0; q < ne; ++q) {   // warp-uniform: broadcast loads
+            const u32 k = c.bkind[q];
+            best = fminf(best, sure_crossing_e2(bound_fw(c.brec[q], c.bmag[q], br), k & 3u, (k >> 2) + h0 == c.prev, br.t));
+        }
         if (best < __int_as_float(0x7f800000)) limit_lower(lim, dist_from_e2(best), br.t);
     }
     float min_dist = -1.0f, min_x = __int_as_float(0x7f800000);
-    u32 min_index = 0, tested = 0;
+    u32 min_index = 0xFFFFFFFFu, tested = 0;
 #pragma unroll 1
     for (u32 c0 = 0; c0 < n; c0 += 32u) {
         const u32 cn = n - c0 < 32u ? n - c0 : 32u;
@@ -1244,29 +1270,35 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
             u32 m = 0;
 #pragma unroll 1
             for (u32 j = 0; j < cn; ++j) {   // warp-uniform: broadcast loads
-                if (!culled_point(c.brec[c0 + j], c.bmag[c0 + j], br, c.bkind[c0 + j] == 0u ? lim.kp : lim.kh)) m |= 1u << j;
+                if (!culled_point(c.brec[c0 + j], c.bmag[c0 + j], br, (c.bkind[c0 + j] & 3u) == 0u ? lim.kp : lim.kh)) m |= 1u << j;
             }
             mask = 0;
             while (m) {   // per lane: the ray-aware bound on the survivors
-                const u32 j = __ffs(m) - 1, i = c0 + j;
+                const u32 j = __ffs(m) - 1, q = c0 + j, k = c.bkind[q] & 3u;
                 m &= m - 1;
-                if (keep_object(c.brec[i], c.bmag[i], c.bkind[i], br, c.bkind[i] == 0u ? lim.kp : lim.kh, lim.cull)) mask |= 1u << j;
+                if (keep_object(c.brec[q], c.bmag[q], k, br, k == 0u ? lim.kp : lim.kh, lim.cull)) mask |= 1u << j;
             }
         }
-        while (mask) {   // this lane's candidates, in index order
-            const u32 i = c0 + (__ffs(mask) - 1);
+        while (mask) {   // this lane's candidates
+            const u32 q = c0 + (__ffs(mask) - 1);
             mask &= mask - 1;
-            if (can && culled_point(c.brec[i], c.bmag[i], br, c.bkind[i] == 0u ? lim.kp : lim.kh)) continue;
+            u32 i = q, kind;
+            if (staged) {
+                kind = c.bkind[q];
+                i = kind >> 2;
+                kind &= 3u;
+            }
+            if (can && culled_point(c.brec[q], c.bmag[q], br, kind == 0u ? lim.kp : lim.kh)) continue;
             ++tested;
             const Ptr elem = self + head + i * stride;
-            const u32 kind = staged ? c.bkind[i] : B::template kind_of<W>(elem);
+            if (!staged) kind = B::template kind_of<W>(elem);
             if (kind > 1u) continue;   // a choice index out of range takes no variant
             ++c.tests;
             const HyRay r = ray_hy_map_call(mo_inverse(B::template map_of<W>(elem)), p, v);
             const float x = shape_hy_test(kind, i + h0 == c.prev, r.p, r.v).x;
-            if (x >= 1.0f && x <= min_x) {
+            if (x >= 1.0f && (x <= min_x || i < min_index)) {
                 const float dist = hy_dist_from_x(x);
-                if (dist > -EPSF && (min_dist <= -EPSF || dist < min_dist)) {
+                if (dist > -EPSF && (min_dist <= -EPSF || dist < min_dist || (dist == min_dist && i < min_index))) {
                     min_dist = dist; min_x = x; min_index = i;
                     c.win[0] = make_float4(r.p.x, r.p.y, r.p.z, r.p.w);
                     c.win[1] = make_float4(r.v.x, r.v.y, r.v.z, r.v.w);
@@ -1293,6 +1325,7 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
 // ============================================================================ scene
 template <class G, class V, class O, class B> struct SceneImpl {   // {phantom, view, background, object}
     template <int W> using R = Rec<W, Zst, V, B, O>;
+    typedef V View;
     typedef O Object;
     typedef G Geometry;
     template <int W> __host__ __device__ static constexpr u32 static_size() { return R<W>::off(3) + O::template lay<W>().size; }
@@ -1369,7 +1402,10 @@ render_generic(Ptr scene, uint64_t scene_size, u32 width, u32 height, u32 tiles,
         __shared__ float s_mag[HTG_BOUND_CAP];
         __shared__ u32 s_kind[HTG_BOUND_CAP];
         const Ptr vec = scene + Scene::template R<W>::off(3);
-        const u32 nb = stage_vec_bounds<Geo, typename VecElem<Obj>::T, W>(vec, scene + scene_size, s_rec, s_mag, s_kind);
+        const Q4 from = ViewStart<typename Scene::View>::template at<W>(scene + Scene::template R<W>::off(1));
+        // (the winners' slots hold the sort's keys: 128 threads and more have 1024 floats)
+        const u32 nb = stage_vec_bounds<Geo, typename VecElem<Obj>::T, W>(vec, scene + scene_size, from, s_rec, s_mag, s_kind,
+                                                                         reinterpret_cast<float *>(c.win - 2 * threadIdx.x));
         __syncthreads();
         if (nb != 0xFFFFFFFFu) {
             c.bvec = vec;
