@@ -1348,12 +1348,28 @@ __global__ void k_fill_seeds(uint32_t n, uint32_t global_seed, uint32_t offset, 
         seeds[i] = fmix32(global_seed ^ fmix32(i + offset));
 }
 
+// pack1(gamma1(x, g)) for g > 0 without the FP64 power where an FP32 one decides the byte: y =
+// exp2(g log2 x) is within 2.3e-6 relative of x^g while 255 y >= 1 (|g log2 x| <= 8; log2f is good to
+// 1 ulp, exp2f to 2), so the byte is that of y unless 255 y lies within 3e-6 (255 y) + 1e-6 of a
+// whole number (about one value in 1000). The power of x >= 1 clamps to 1. The fused kernel was
+// bound by the four FP64 powers a pixel: 1920x1080 71 us, now 27 (its instructions; the 41 MB that
+// it reads and writes take 6.4).
+static __device__ __noinline__ uint8_t gamma_pack_exact(float x, float g) { return pack1(gamma1(x, g)); }
+__device__ __forceinline__ uint8_t gamma_pack(float x, float g) {
+    if (x >= 1.0f) return 255;
+    if (!(x > 0.0f)) return 0;   // max(x, 0) = 0, NaN too
+    const float v = 255.0f * exp2f(g * log2f(x));
+    if (!(fabsf(v - rintf(v)) > fmaf(v, 3e-6f, 1e-6f))) return gamma_pack_exact(x, g);
+    return (uint8_t)__float2uint_rz(v);
+}
 __global__ void k_extract_gamma_pack(uint32_t n, float passes, float g, const float4 *__restrict__ canvas,
                                      uchar4 *__restrict__ out) {
+    const bool usual = g > 0.0f && g < 16.0f;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 c = canvas[i];
-        out[i] = make_uchar4(pack1(gamma1(c.x / passes, g)), pack1(gamma1(c.y / passes, g)),
-                             pack1(gamma1(c.z / passes, g)), pack1(gamma1(c.w / passes, g)));
+        const float4 c = canvas[i];
+        const float x = c.x / passes, y = c.y / passes, z = c.z / passes, w = c.w / passes;
+        out[i] = usual ? make_uchar4(gamma_pack(x, g), gamma_pack(y, g), gamma_pack(z, g), gamma_pack(w, g))
+                       : make_uchar4(gamma_pack_exact(x, g), gamma_pack_exact(y, g), gamma_pack_exact(z, g), gamma_pack_exact(w, g));
     }
 }
 
