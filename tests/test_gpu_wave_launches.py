@@ -24,6 +24,27 @@ def _scene(geometry, n, hops):
     return S.hyperbolic_scene(n - horo, horo, 6.0, hops, 500 + n, camera=S.random_moebius(rng, 0.5))
 
 
+@pytest.mark.parametrize("tile", [1, 33, 100, 512])
+def test_batch_tiles_cover_hop_0_tiles(built, tile):
+    """Views whose hop 0 takes 8 x 4 pixel tiles (ragged edges) and views too small for them, batch
+    tiles of any size."""
+    ctx = P.Context(0)
+    views = []
+    for i, (geometry, n, W, H) in enumerate([("hy", 20, 131, 67), ("eu", 9, 64, 32), ("hy", 110, 63, 200), ("eu", 5, 257, 33),
+                                             ("hy", 40, 72, 31)]):
+        views.append(B.View(_scene(geometry, n, 4), W, H, 16, 40 + i))
+        views[-1].allocate(ctx)
+    renderer = B.BatchRenderer(ctx)
+    renderer.set_views(views, [2] * len(views), tile_pixels=tile)
+    renderer.render()
+    renderer.check()
+    for v in views:
+        canvas = P.Canvas(ctx, (v.width, v.height), v.global_seed)
+        P.Render(ctx, v.scene.recipe, v.scene.hops).render_wavefront(v.buffer, canvas, 1)
+        P.Render(ctx, v.scene.recipe, v.scene.hops).render(v.buffer, canvas)
+        assert np.array_equal(_bits(canvas)[0], _bits(v.canvas)[0]) and np.array_equal(_bits(canvas)[1], _bits(v.canvas)[1])
+
+
 def _bits(canvas):
     return canvas.image.cpu().numpy().view(np.uint32), canvas.seeds.cpu().numpy()
 
