@@ -232,7 +232,7 @@ static __device__ __noinline__ HyPath camera_hy(const StagedScene &s, float px, 
     float sx = px + size * (jx - 0.5f);
     float sy = py + size * (jy - 0.5f);
     V3 ld = normalize3(v3(sx, sy, -1.0f / s.fov));
-    HyRay r = view_hy_map(mo_from(s.cam0, s.cam1), q4(0.0f, 0.0f, 1.0f, 0.0f), q4(ld.x, ld.y, ld.z, 0.0f));
+    HyRay r = view_hy_map_packed(mo_from(s.cam0, s.cam1), q4(0.0f, 0.0f, 1.0f, 0.0f), q4(ld.x, ld.y, ld.z, 0.0f));
     HyPath o; o.p = r.p; o.v = r.v;
     return o;
 }
@@ -422,7 +422,7 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
             ++n_exact;
             // the out-of-line copy of the map, shared with the hit path: one copy of its code
             // (the kernel is bound by instruction fetch as much as by issue)
-            HyRay l = ray_hy_map_call(mo_from(s.inv[2 * q], s.inv[2 * q + 1]), p, v);
+            HyRay l = ray_hy_map_packed(mo_from(s.inv[2 * q], s.inv[2 * q + 1]), qq(p, v));
             const float x = shape == 0 ? plane_hy_x(l.p, l.v) : horosphere_x(l.p, l.v, repeat);
             // x above the best's gives a distance no smaller (hy_dist_from_x is non-decreasing),
             // which can only win a tie, and only from a lower scene index
@@ -466,12 +466,12 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
     Q4 normal;
     if (s.shape[kmin] == 0) plane_hy_hit(l.p, l.v, lh, normal);
     else horosphere_hit(l.p, l.v, repeat, lh, normal);
-    HyRay w = ray_hy_map_call(fwd, lh.p, lh.v);          // detect: map back (mapped.inl:34)
-    HyRay loc = ray_hy_map_call(inv, w.p, w.v);          // interact: to local (mapped.inl:46-47)
+    HyRay w = ray_hy_map_packed(fwd, qq(lh.p, lh.v));          // detect: map back (mapped.inl:34)
+    HyRay loc = ray_hy_map_packed(inv, qq(w.p, w.v));          // interact: to local (mapped.inl:46-47)
     Material m = load_material(obj);
     V3 dir = v3(loc.v.x, loc.v.y, loc.v.z);          // light_hy_to_local (light/hy.cc:3-8)
     bool ret = mixture_interact(m, rng, v3(normal.x, normal.y, normal.z), dir, intensity, emission);
-    HyRay out = ray_hy_map_call(fwd, loc.p, q4(dir.x, dir.y, dir.z, 0.0f));  // mapped.inl:49
+    HyRay out = ray_hy_map_packed(fwd, qq(loc.p, q4(dir.x, dir.y, dir.z, 0.0f)));  // mapped.inl:49
     ray.p = out.p;
     ray.v = out.v;
     if (!ret) return false;

@@ -77,6 +77,37 @@ __global__ void k_raymap(uint64_t n, uint64_t seed, unsigned long long *out) {
     atomicAdd(&out[1], mism);
 }
 
+// The packed ray map and camera map against the IEEE form, all 8 outputs; with `zeros`, half of
+// the inputs are zeros of either sign.
+__global__ void k_raymap_packed(uint64_t n, uint64_t seed, int zeros, unsigned long long *out) {
+    unsigned long long cnt = 0, mism = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        float f[16];
+        for (int k = 0; k < 16; ++k) {
+            const uint64_t h = splitmix(seed ^ (i * 16 + k));
+            f[k] = ((float)(h >> 40) / 16777216.0f) * 4.0f - 2.0f;
+            if (zeros && (h & 1)) f[k] = (h & 2) ? -0.0f : 0.0f;
+        }
+        Mo m;
+        m.a.x = f[0]; m.a.y = f[1]; m.b.x = f[2]; m.b.y = f[3];
+        m.c.x = f[4]; m.c.y = f[5]; m.d.x = f[6]; m.d.y = f[7];
+        const Q4 p = q4(f[8], f[9], fabsf(f[10]) + 0.01f, zeros ? f[14] : 0.0f);
+        const Q4 v = normalize4(q4(f[11], f[12], f[13] + 0.01f, zeros ? f[15] : 0.0f));
+        for (int twice = 0; twice < 2; ++twice) {
+            const HyRay a = twice ? ray_hy_map_packed(m, qq(p, v)) : view_hy_map_packed(m, p, v);
+            const HyRay b = hy_map_ieee(m, p, v, twice != 0);
+            const float x[8] = {a.p.x, a.p.y, a.p.z, a.p.w, a.v.x, a.v.y, a.v.z, a.v.w};
+            const float y[8] = {b.p.x, b.p.y, b.p.z, b.p.w, b.v.x, b.v.y, b.v.z, b.v.w};
+            bool same = true;
+            for (int k = 0; k < 8; ++k) same &= __float_as_uint(x[k]) == __float_as_uint(y[k]);
+            ++cnt;
+            if (!same) ++mism;
+        }
+    }
+    atomicAdd(&out[0], cnt);
+    atomicAdd(&out[1], mism);
+}
+
 // Exhaustive: hy_dist_from_x(x) <= hy_dist_from_x(next float after x) for every float x in
 // [1, +inf). Counts violations (a NaN result counts as one).
 __global__ void k_monotone(unsigned long long *out) {
@@ -145,6 +176,10 @@ extern "C" int ht_selftest_div(uint64_t n, uint64_t seed, int mode, unsigned lon
 extern "C" int ht_selftest_raymap(uint64_t n, uint64_t seed, unsigned long long *host_out) {
     g_n = n; g_seed = seed;
     return run([](unsigned long long *d) { k_raymap<<<148 * 8, 256>>>(g_n, g_seed, d); }, host_out);
+}
+extern "C" int ht_selftest_raymap_packed(uint64_t n, uint64_t seed, int zeros, unsigned long long *host_out) {
+    g_n = n; g_seed = seed; g_mode = zeros;
+    return run([](unsigned long long *d) { k_raymap_packed<<<148 * 8, 256>>>(g_n, g_seed, g_mode, d); }, host_out);
 }
 extern "C" int ht_selftest_monotone(unsigned long long *host_out) {
     return run([](unsigned long long *d) { k_monotone<<<148 * 16, 256>>>(d); }, host_out);
