@@ -97,13 +97,12 @@ HT_D QQ cqq_mul(C2 a, const QQ &b) {   // cq_mul of both
     r.w = add2(mul2(x, b.w), mul2(y, b.z));
     return r;
 }
-HT_D QQ qq_mul(const QQ &a, Q4 b) {   // q_mul of both by b
-    const float2 x = both(b.x), y = both(b.y), z = both(b.z), w = both(b.w);
+HT_D QQ qq_mul(const QQ &a, const QQ &b) {   // q_mul of both
     QQ r;
-    r.x = sub2(sub2(sub2(mul2(a.x, x), mul2(a.y, y)), mul2(a.z, z)), mul2(a.w, w));
-    r.y = sub2(add2(add2(mul2(a.x, y), mul2(a.y, x)), mul2(a.z, w)), mul2(a.w, z));
-    r.z = add2(sub2(add2(mul2(a.x, z), mul2(a.z, x)), mul2(a.y, w)), mul2(a.w, y));
-    r.w = sub2(add2(add2(mul2(a.x, w), mul2(a.w, x)), mul2(a.y, z)), mul2(a.z, y));
+    r.x = sub2(sub2(sub2(mul2(a.x, b.x), mul2(a.y, b.y)), mul2(a.z, b.z)), mul2(a.w, b.w));
+    r.y = sub2(add2(add2(mul2(a.x, b.y), mul2(a.y, b.x)), mul2(a.z, b.w)), mul2(a.w, b.z));
+    r.z = add2(sub2(add2(mul2(a.x, b.z), mul2(a.z, b.x)), mul2(a.y, b.w)), mul2(a.w, b.y));
+    r.w = sub2(add2(add2(mul2(a.x, b.w), mul2(a.w, b.x)), mul2(a.y, b.z)), mul2(a.z, b.y));
     return r;
 }
 
@@ -254,7 +253,7 @@ template <bool TWICE, bool PACKED> HT_D HyRay hy_map(const Mo &m, const QQ &pv) 
     const Q4 di = qdiv4<PACKED>(q4(d.x, -d.y, -d.z, -d.w), rd, chk);
     HyRay o;
     if constexpr (PACKED) {
-        const QQ og = qq_mul(qq(u, qq_second(av)), di);
+        const QQ og = qq_mul(qq(u, qq_second(av)), qq(di, di));
         o.p = qq_first(og);
         g1 = qq_second(og);
     } else {
@@ -312,7 +311,16 @@ HT_D EuRay ray_eu_map(const Hom &m, V3 p, V3 v) {
     return o;
 }
 // The same map, out of line: the object scan and the hit path share this one copy of its code.
-static __device__ __noinline__ EuRay ray_eu_map_call(const Hom m, const V3 p, const V3 v) { return ray_eu_map(m, p, v); }
+// Packed: the position and the direction are turned side by side (1917x1077, 25 objects, 16 passes:
+// 4.77 -> 4.60 ms).
+static __device__ __noinline__ EuRay ray_eu_map_call(const Hom m, const V3 p, const V3 v) {
+    const Q4 c = q_conj(m.rot);
+    const QQ r = qq_mul(qq_mul(qq(m.rot, m.rot), qq(q4(0.0f, p.x, p.y, p.z), q4(0.0f, v.x, v.y, v.z))), qq(c, c));
+    EuRay o;
+    o.p = v3(r.y.x + m.shift.x, r.z.x + m.shift.y, r.w.x + m.shift.z);
+    o.v = normalize3(v3(r.y.y, r.z.y, r.w.y));
+    return o;
+}
 HT_D Hom hom3_inverse(const Hom &m) {
     Hom s;
     s.shift = v3(-m.shift.x, -m.shift.y, -m.shift.z);
