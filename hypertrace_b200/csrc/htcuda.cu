@@ -1031,12 +1031,16 @@ template <int RF, int FH>
 __global__ void __launch_bounds__(128, HT_BATCH_MINB) render_batch_wave(
     const BatchView *__restrict__ views, const uint32_t *__restrict__ order, uint32_t n_order, uint32_t n_views,
     uint32_t pass, uint32_t h, uint32_t tile_slots, uint32_t smem_objects, WaveQueue in, WaveQueue out,
-    uint32_t *cnt, uint32_t *grab, uint64_t *stats, uint32_t n_sorted) {
+    uint32_t *cnt, uint32_t *grab, uint64_t *stats, uint32_t n_sorted, uint32_t *clear, uint32_t n_clear) {
     extern __shared__ float4 smem[];
     __shared__ uint32_t s_tile, s_next, s_total, s_tsize;
     __shared__ int s_staged_view, s_staged_ok;
     uint32_t *s_pref = reinterpret_cast<uint32_t *>(carve_scene(smem, smem_objects).end);   // n_order + 1 tile offsets
     const uint32_t tid = threadIdx.x, lane = tid & 31;
+    wait_previous();
+    launch_next();
+    if (FH == 1 && blockIdx.x == 0)
+        for (uint32_t i = tid; i < n_clear; i += blockDim.x) clear[i] = 0;
 
     // tiles of every view at this hop, in `order`, as a prefix sum. The tile size adapts to
     // the launch: about 16 tiles per block when the paths are few (a multiple of 128 slots,
@@ -1218,6 +1222,8 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bsort_keys(const BatchView *__
     extern __shared__ uint32_t s_hist[];   // SORT_BINS, then n_seg counts and n_seg + 1 window numbers
     __shared__ SortCells cells;
     uint32_t *s_count = s_hist + SORT_BINS, *s_win = s_count + n_seg;
+    wait_previous();
+    launch_next();
     const uint32_t win = bsort_windows(views, order, n_seg, n_views, pass, h, cnt, s_count, s_win);
     uint32_t of = 0xFFFFFFFFu;   // the view that `cells` are of
     for (uint32_t w = blockIdx.x; w < s_win[n_seg]; w += gridDim.x) {
@@ -1240,6 +1246,8 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bsort_scatter(const BatchView 
                                                                uint32_t *__restrict__ perm) {
     extern __shared__ uint32_t s_base[];   // SORT_BINS, then n_seg counts and n_seg + 1 window numbers
     uint32_t *s_count = s_base + SORT_BINS, *s_win = s_count + n_seg;
+    wait_previous();
+    launch_next();
     const uint32_t win = bsort_windows(views, order, n_seg, n_views, pass, h, cnt, s_count, s_win);
     for (uint32_t b = blockIdx.x * SORT_THREADS + threadIdx.x; b < n_seg * SORT_BINS; b += gridDim.x * SORT_THREADS)
         next_hist[b] = 0;
@@ -1866,7 +1874,7 @@ static int launch_wave(const htc_program *p, const WaveWork &w, uint32_t W, uint
             if (sorted && h > 0) {
                 uint32_t *hist = sb.hist + (sorts & 1u) * SORT_BINS, *other = sb.hist + (~sorts & 1u) * SORT_BINS;
                 ++sorts;
-                HTC_CUDA(launch(true, k_sort_keys, sort_blocks, SORT_THREADS, sort_smem, st, in.p, in.v, in_count, hist, sb.place, sb.key));
+                HTC_CUDA(launch(false, k_sort_keys, sort_blocks, SORT_THREADS, sort_smem, st, in.p, in.v, in_count, hist, sb.place, sb.key));
                 HTC_CUDA(launch(true, k_sort_scatter, sort_blocks, SORT_THREADS, sort_smem, st, sb.key, in_count, hist, other, sb.place, sb.perm));
                 in.o = sb.perm;
             }
@@ -2083,7 +2091,12 @@ struct htc_batch {
     size_t image_words;
     void *sort_buf;          // coherence sort of the hyperbolic views (BatchSortBuf)
     uint64_t sort_slots;     // = wave_slots when allocated
+    uint32_t hops_of[2], passes_of[2];   // the most of the hyperbolic, of the Euclidean views
+    cudaStream_t side;       // where the Euclidean launches run beside the hyperbolic ones
+    cudaEvent_t forked, joined;
 };
+// Counters of one recipe and pass: every view's paths by hop, then the tiles taken by hop.
+static uint32_t batch_counters(uint32_t n_views, uint32_t hops) { return (n_views + 1) * hops; }
 
 static void batch_free(htc_batch *b) {
     if (!b) return;
@@ -2095,6 +2108,9 @@ static void batch_free(htc_batch *b) {
         if (b->p_views[i]) cudaFreeHost(b->p_views[i]);
         if (b->p_order[i]) cudaFreeHost(b->p_order[i]);
     }
+    if (b->forked) cudaEventDestroy(b->forked);
+    if (b->joined) cudaEventDestroy(b->joined);
+    if (b->side) cudaStreamDestroy(b->side);
     if (b->d_order) cudaFree(b->d_order);
     if (b->wave_buf) cudaFree(b->wave_buf);
     if (b->d_wcnt) cudaFree(b->d_wcnt);
@@ -2124,6 +2140,54 @@ static int batch_wave_blocks(htc_batch *b, size_t smem, unsigned *blocks) {
     return HTC_OK;
 }
 
+// The launches of a batch. The two geometries share nothing but the stage before them, so the
+// Euclidean ones run on a stream of their own beside the hyperbolic ones (`st_eu`), and fill
+// what those leave of the chip at the end of every launch and while few paths are left; within a
+// stream the launches overlap at their edges, except with the sort's first kernel: its 148
+// large blocks would crowd on the multiprocessors that are free first. 24 mixed views: 35.34 ms one
+// after another, 34.54 on two streams, 34.65 with the overlap as well; a server's steps of 1 to 4
+// views (12 requests) 52.7, 50.7 and 49.95; the sort's first kernel overlapping too 34.8 and 50.4.
+static int batch_passes(htc_batch *b, const WaveQueue (&q)[2], unsigned blocks_hy, unsigned blocks_eu, size_t smem, uint32_t n_seg,
+                        uint64_t *stats, cudaStream_t st, cudaStream_t st_eu) {
+    // each geometry has counters of its own, in two sets: a pass's hop 0 clears the next one's
+    const uint32_t words = batch_counters(b->n_views, b->hops_max);
+    const uint32_t *order_hy = b->d_order + b->n_order, *order_eu = order_hy + b->n_hy;
+    const unsigned sort_blocks = (unsigned)b->num_sms;
+    const BatchSortBuf sb = n_seg ? batch_sort_at(b->sort_buf, b->sort_slots, sort_blocks) : BatchSortBuf{};
+    const size_t sort_smem = sizeof(uint32_t) * (SORT_BINS + 2 * n_seg + 1);
+    uint32_t sorts = 0;   // both sets of histograms start cleared; k_bsort_scatter clears the one its depth did not use
+    for (uint32_t pass = 0; pass < b->passes_max; ++pass) {
+        uint32_t *set = b->d_wcnt + (size_t)(pass & 1u) * words, *next = b->d_wcnt + (size_t)(~pass & 1u) * words;
+        for (uint32_t h = 0; h < b->hops_max; ++h) {
+            const WaveQueue &in = q[(h + 1) & 1], &out = q[h & 1];
+            uint32_t *cnt = set, *grab = cnt + (size_t)b->n_views * b->hops_max + h;
+            if (pass < b->passes_of[0] && h < b->hops_of[0]) {
+                WaveQueue in_hy = in;
+                if (n_seg && h > 0) {
+                    uint32_t *hist = sb.hist + (size_t)(sorts & 1u) * BATCH_SORT_VIEWS * SORT_BINS;
+                    uint32_t *other = sb.hist + (size_t)(~sorts & 1u) * BATCH_SORT_VIEWS * SORT_BINS;
+                    ++sorts;
+                    HTC_CUDA(launch(false, k_bsort_keys, sort_blocks, SORT_THREADS, sort_smem, st, b->d_views, order_hy, n_seg, b->n_views, pass, h,
+                                    cnt, in.p, in.v, hist, sb.place, sb.key));
+                    HTC_CUDA(launch(true, k_bsort_scatter, sort_blocks, SORT_THREADS, sort_smem, st, b->d_views, order_hy, n_seg, b->n_views, pass, h,
+                                    cnt, sb.key, hist, other, sb.place, sb.perm));
+                    in_hy.o = sb.perm;
+                }
+                HTC_CUDA(launch(true, h == 0 ? render_batch_wave<RECIPE_HY, 1> : render_batch_wave<RECIPE_HY, 2>, blocks_hy, 128, smem, st,
+                                b->d_views, order_hy, b->n_hy, b->n_views, pass, h, b->tile_pixels, b->smem_objects, in_hy, out, cnt, grab,
+                                stats, n_seg, next, words));
+            }
+            if (pass < b->passes_of[1] && h < b->hops_of[1]) {
+                cnt += 2 * words;
+                HTC_CUDA(launch(true, h == 0 ? render_batch_wave<RECIPE_EU, 1> : render_batch_wave<RECIPE_EU, 2>, blocks_eu, 128, smem, st_eu,
+                                b->d_views, order_eu, b->n_eu, b->n_views, pass, h, b->tile_pixels, b->smem_objects, in, out, cnt, grab + 2 * words,
+                                stats, 0u, next + 2 * words, words));
+            }
+        }
+    }
+    return HTC_OK;
+}
+
 static int batch_launch_wave(htc_batch *b, uint64_t *stats, cudaStream_t st) {
     if (b->n_order == 0) return HTC_OK;
     const size_t smem = smem_bytes(b->smem_objects) + sizeof(uint32_t) * ((size_t)b->n_views + 1);
@@ -2142,45 +2206,20 @@ static int batch_launch_wave(htc_batch *b, uint64_t *stats, cudaStream_t st) {
     int rc = batch_wave_blocks<RECIPE_HY>(b, smem, &blocks_hy);
     if (!rc) rc = batch_wave_blocks<RECIPE_EU>(b, smem, &blocks_eu);
     if (rc) return rc;
-    const size_t words = (size_t)(b->n_views + 3) * b->hops_max;
-    uint32_t *grab = b->d_wcnt + (size_t)b->n_views * b->hops_max;   // 3 words per hop depth
-    const uint32_t *order_hy = b->d_order + b->n_order, *order_eu = order_hy + b->n_hy;
     // coherence sort of the first n_seg hyperbolic views in launch order (the expensive ones)
     const uint32_t n_seg = HT_BATCH_SORT && b->sort_buf ? std::min(b->n_hy, BATCH_SORT_VIEWS) : 0u;
-    const unsigned sort_blocks = (unsigned)b->num_sms;
-    const BatchSortBuf sb = n_seg ? batch_sort_at(b->sort_buf, b->sort_slots, sort_blocks) : BatchSortBuf{};
-    const size_t sort_smem = sizeof(uint32_t) * (SORT_BINS + 2 * n_seg + 1);
+    if (n_seg) HTC_CUDA(cudaMemsetAsync(batch_sort_at(b->sort_buf, b->sort_slots, (unsigned)b->num_sms).hist, 0,
+                                        2 * sizeof(uint32_t) * (size_t)BATCH_SORT_VIEWS * SORT_BINS, st));
+    HTC_CUDA(cudaMemsetAsync(b->d_wcnt, 0, 4 * sizeof(uint32_t) * (size_t)batch_counters(b->n_views, b->hops_max), st));
     k_batch_stage<<<b->n_order, STAGE_THREADS, 0, st>>>(b->d_views, b->d_order, b->d_err);
     HTC_CUDA(cudaGetLastError());
-    uint32_t sorts = 0;   // both sets of histograms start cleared; k_bsort_scatter clears the one its depth did not use
-    if (n_seg) HTC_CUDA(cudaMemsetAsync(sb.hist, 0, 2 * sizeof(uint32_t) * (size_t)BATCH_SORT_VIEWS * SORT_BINS, st));
-    for (uint32_t pass = 0; pass < b->passes_max; ++pass) {
-        HTC_CUDA(cudaMemsetAsync(b->d_wcnt, 0, sizeof(uint32_t) * words, st));
-        for (uint32_t h = 0; h < b->hops_max; ++h) {
-            const WaveQueue &in = q[(h + 1) & 1], &out = q[h & 1];
-            WaveQueue in_hy = in;
-            if (n_seg && h > 0) {
-                uint32_t *hist = sb.hist + (size_t)(sorts & 1u) * BATCH_SORT_VIEWS * SORT_BINS;
-                uint32_t *other = sb.hist + (size_t)(~sorts & 1u) * BATCH_SORT_VIEWS * SORT_BINS;
-                ++sorts;
-                k_bsort_keys<<<sort_blocks, SORT_THREADS, sort_smem, st>>>(b->d_views, order_hy, n_seg, b->n_views, pass, h,
-                                                                          b->d_wcnt, in.p, in.v, hist, sb.place, sb.key);
-                k_bsort_scatter<<<sort_blocks, SORT_THREADS, sort_smem, st>>>(b->d_views, order_hy, n_seg, b->n_views, pass, h,
-                                                                             b->d_wcnt, sb.key, hist, other, sb.place, sb.perm);
-                in_hy.o = sb.perm;
-            }
-            if (b->n_hy)
-                (h == 0 ? render_batch_wave<RECIPE_HY, 1> : render_batch_wave<RECIPE_HY, 2>)<<<blocks_hy, 128, smem, st>>>(b->d_views, order_hy, b->n_hy, b->n_views,
-                                                                           pass, h, b->tile_pixels, b->smem_objects, in_hy,
-                                                                           out, b->d_wcnt, grab + 3 * h + 1, stats, n_seg);
-            if (b->n_eu)
-                (h == 0 ? render_batch_wave<RECIPE_EU, 1> : render_batch_wave<RECIPE_EU, 2>)<<<blocks_eu, 128, smem, st>>>(b->d_views, order_eu, b->n_eu, b->n_views,
-                                                                           pass, h, b->tile_pixels, b->smem_objects, in,
-                                                                           out, b->d_wcnt, grab + 3 * h + 2, stats, 0u);
-        }
-        HTC_CUDA(cudaGetLastError());
-    }
-    return HTC_OK;
+    if (!b->n_hy || !b->n_eu) return batch_passes(b, q, blocks_hy, blocks_eu, smem, n_seg, stats, st, st);
+    HTC_CUDA(cudaEventRecord(b->forked, st));
+    HTC_CUDA(cudaStreamWaitEvent(b->side, b->forked, 0));
+    rc = batch_passes(b, q, blocks_hy, blocks_eu, smem, n_seg, stats, st, b->side);
+    HTC_CUDA(cudaEventRecord(b->joined, b->side));
+    HTC_CUDA(cudaStreamWaitEvent(st, b->joined, 0));
+    return rc;
 }
 
 extern "C" {
@@ -2199,6 +2238,9 @@ int htc_batch_create(uint32_t max_views, htc_batch **out) {
     if (e == cudaSuccess) e = cudaMalloc(&b->d_order, 2 * sizeof(uint32_t) * max_views);   // all, then by recipe
     if (e == cudaSuccess) e = cudaMalloc(&b->d_err, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->joined, cudaEventDisableTiming);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
         e = cudaHostAlloc(reinterpret_cast<void **>(&b->p_views[i]), sizeof(BatchView) * max_views, cudaHostAllocDefault);
         if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&b->p_order[i]), 2 * sizeof(uint32_t) * max_views, cudaHostAllocDefault);
@@ -2317,7 +2359,7 @@ int htc_batch_set_views(htc_batch *b, const htc_view *views, uint32_t n_views, u
     // wavefront queues: one region of W*H slots (rounded to 64: 16-byte aligned arrays) per view
     uint64_t slots = 0;
     size_t images = 0;
-    uint32_t hops_max = 0, passes_max = 0;
+    uint32_t hops_max = 0, passes_max = 0, hops_of[2] = {0, 0}, passes_of[2] = {0, 0};
     for (const auto &o : order) {
         BatchView &d = b->h_views[o.second];
         d.qoff = slots;
@@ -2325,13 +2367,16 @@ int htc_batch_set_views(htc_batch *b, const htc_view *views, uint32_t n_views, u
         images += image_words(d.max_objects);
         hops_max = std::max(hops_max, d.hops);
         passes_max = std::max(passes_max, d.passes);
+        const int k = d.recipe == RECIPE_HY ? 0 : 1;
+        hops_of[k] = std::max(hops_of[k], d.hops);
+        passes_of[k] = std::max(passes_of[k], d.passes);
     }
     b->smem_objects = smem_objects;
     b->blocks_per_sm = blocks_per_sm;
     b->tile_pixels = tile_pixels;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     {
-        int rc = batch_grow(b, slots, (size_t)(n_views + 3) * hops_max, images, st);
+        int rc = batch_grow(b, slots, 4 * (size_t)batch_counters(n_views, hops_max), images, st);
         if (rc) return rc;
     }
     images = 0;
@@ -2343,6 +2388,10 @@ int htc_batch_set_views(htc_batch *b, const htc_view *views, uint32_t n_views, u
     b->n_order = (uint32_t)order.size();
     b->hops_max = hops_max;
     b->passes_max = passes_max;
+    for (int k = 0; k < 2; ++k) {
+        b->hops_of[k] = hops_of[k];
+        b->passes_of[k] = passes_of[k];
+    }
     // Asynchronous upload through the next pinned slot: wait only for that slot's previous
     // copy, then copy on `stream` (ordered after any launch still reading the device arrays).
     const int k = b->slot;

@@ -45,6 +45,38 @@ def test_batch_tiles_cover_hop_0_tiles(built, tile):
         assert np.array_equal(_bits(canvas)[0], _bits(v.canvas)[0]) and np.array_equal(_bits(canvas)[1], _bits(v.canvas)[1])
 
 
+@pytest.mark.parametrize("kinds", [[("hy", 30, 2, 3), ("eu", 9, 7, 1)], [("eu", 6, 1, 4), ("hy", 5, 5, 1), ("eu", 20, 3, 2)],
+                                   [("eu", 9, 4, 2)], [("hy", 120, 4, 2), ("hy", 3, 1, 1)]])
+@pytest.mark.parametrize("capture", [False, True])
+def test_batch_geometries_side_by_side(built, kinds, capture):
+    """Batches whose geometries differ in hops and passes, or that have one only, called directly and
+    as a captured graph that is replayed: (geometry, objects, hops, passes) of each view."""
+    ctx = P.Context(0)
+    views = []
+    for i, (geometry, n, hops, _) in enumerate(kinds):
+        views.append(B.View(_scene(geometry, n, hops), 300 + 17 * i, 120, 16, 70 + i))
+        views[-1].allocate(ctx)
+    renderer = B.BatchRenderer(ctx)
+    renderer.set_views(views, [k[3] for k in kinds])
+    calls = 3
+    if capture:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            renderer.render()
+        for _ in range(calls):
+            graph.replay()
+    else:
+        for _ in range(calls):
+            renderer.render()
+    torch.cuda.synchronize()
+    renderer.check()
+    for v, k in zip(views, kinds):
+        canvas = P.Canvas(ctx, (v.width, v.height), v.global_seed)
+        P.Render(ctx, v.scene.recipe, v.scene.hops).render_wavefront(v.buffer, canvas, calls * k[3])
+        assert np.array_equal(_bits(canvas)[0], _bits(v.canvas)[0]) and np.array_equal(_bits(canvas)[1], _bits(v.canvas)[1])
+
+
 def _bits(canvas):
     return canvas.image.cpu().numpy().view(np.uint32), canvas.seeds.cpu().numpy()
 
