@@ -37,28 +37,19 @@ using namespace ht;
 // ============================================================================ errors
 thread_local std::string g_last_error;
 
-// Minimum resident blocks per SM requested from ptxas for the render kernels (register cap).
-// The scan is latency-bound on dependent FP32 chains, so resident warps matter, but the
-// packed point-bound loop and the slot bookkeeping hold more values than the earlier scan.
-// Measured at 4 / 5 / 6 blocks: later hops of the wavefronts 9.30 / 9.32 / - ms (1080p, 200 objects, 8
-// passes), hop 0 9.35 / 9.30 / 9.24 ms (and 4.87 / 4.92 / 4.74 ms, Euclidean 1917x1077, 16 passes), the
-// batched kernels 37.3 / 36.2 / 37.7 ms (24 mixed views), the one-pass kernel - / 3.32 / 3.43 ms, 8 blocks
-// 3.48 (one pass of the 1080p frame).
-#ifndef HT_PERSIST_MINB
-#define HT_PERSIST_MINB 6
-#endif
-#ifndef HT_PLAIN_MINB
-#define HT_PLAIN_MINB 5
-#endif
-#ifndef HT_WAVE_MINB    // render_wave, hop depths after the first
-#define HT_WAVE_MINB 4
-#endif
-#ifndef HT_WAVE0_MINB   // render_wave, hop depth 0
-#define HT_WAVE0_MINB 6
-#endif
-#ifndef HT_BATCH_MINB   // render_batch_wave (one recipe per kernel)
-#define HT_BATCH_MINB 5
-#endif
+// Minimum resident blocks per SM requested from ptxas for the render kernels (register cap). The
+// scan is latency-bound on dependent FP32 chains, so resident warps matter, but a hyperbolic
+// ray map and the scan's thresholds hold many values; Euclidean paths need far fewer.
+// Measured (ms; 1080p / 200 objects, 8 passes, and 24 mixed views for the batch; Euclidean: 1917x1077,
+// 25 objects, 16 passes):
+//   later hops   hyperbolic 4 blocks 8.99, 5 9.11; Euclidean (hop 0 at 9) 5 4.48, 6 4.38, 7 4.48
+//   hop 0        hyperbolic 5 8.91, 6 8.99, 7 9.03; Euclidean (later hops at 6) 8 4.38, 9 4.38, 10 4.51
+//                (4 and 6 for the later hops and hop 0 of both geometries: 4.59)
+//   batched      hyperbolic 4 34.85, 5 34.49, 6 35.9; Euclidean 5 34.6, 6 34.45, 7 34.55
+//   one pass     5 and 6 alike (800x600: 384 us), 4 1 % slower
+constexpr int MINB_PERSIST = 6, MINB_PLAIN = 5;
+constexpr int minb_wave(bool eu, bool first) { return eu ? (first ? 9 : 6) : (first ? 5 : 4); }
+constexpr int minb_batch(bool eu) { return eu ? 6 : 5; }
 #ifndef HT_BATCH_SORT   // coherence sort of the batch's hyperbolic views
 #define HT_BATCH_SORT 1
 #endif
@@ -428,7 +419,7 @@ __device__ __forceinline__ void flush_stats(uint64_t *stats, uint32_t samples32,
 
 // ============================================================================ plain
 template <int R>
-__global__ void __launch_bounds__(128, HT_PLAIN_MINB) render_plain(
+__global__ void __launch_bounds__(128, MINB_PLAIN) render_plain(
     const uint8_t *__restrict__ scene, size_t scene_size, uint32_t max_objects, int address_width,
     uint32_t W, uint32_t H, uint32_t hops, uint32_t flags, float4 *__restrict__ canvas,
     uint32_t *__restrict__ seeds, uint64_t *stats, uint32_t *err) {
@@ -586,7 +577,7 @@ __device__ __forceinline__ void rewind_queue(uint32_t *queue) {
 }
 
 template <int R>
-__global__ void __launch_bounds__(128, HT_PERSIST_MINB) render_persistent(
+__global__ void __launch_bounds__(128, MINB_PERSIST) render_persistent(
     const uint8_t *__restrict__ scene, size_t scene_size, uint32_t max_objects, int address_width,
     uint32_t W, uint32_t H, uint32_t hops, uint32_t passes, uint32_t flags,
     float4 *__restrict__ canvas, uint32_t *__restrict__ seeds, uint64_t *stats, uint32_t *err,
@@ -754,7 +745,7 @@ __device__ __forceinline__ void wave_chunk(const StagedScene &s, uint32_t base, 
 // Hop 0 also clears the `n_clear` counters of the next pass.
 // `image_ready`: the scene's image was complete before the launch before this one started.
 template <int R, int FH>
-__global__ void __launch_bounds__(128, FH == 1 ? HT_WAVE0_MINB : HT_WAVE_MINB) render_wave(
+__global__ void __launch_bounds__(128, minb_wave(R == RECIPE_EU, FH == 1)) render_wave(
     const float4 *image, const uint8_t *__restrict__ scene, uint32_t max_objects, bool image_ready,
     uint32_t W, uint32_t H, uint32_t hops, uint32_t hop_index, uint32_t flags, float4 *__restrict__ canvas,
     uint32_t *__restrict__ seeds, uint64_t *stats, WaveQueue in, const uint32_t *in_count,
@@ -1028,7 +1019,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) k_batch_stage(const BatchView *
 
 // RF: the recipe of the views in `order`.
 template <int RF, int FH>
-__global__ void __launch_bounds__(128, HT_BATCH_MINB) render_batch_wave(
+__global__ void __launch_bounds__(128, minb_batch(RF == RECIPE_EU)) render_batch_wave(
     const BatchView *__restrict__ views, const uint32_t *__restrict__ order, uint32_t n_order, uint32_t n_views,
     uint32_t pass, uint32_t h, uint32_t tile_slots, uint32_t smem_objects, WaveQueue in, WaveQueue out,
     uint32_t *cnt, uint32_t *grab, uint64_t *stats, uint32_t n_sorted, uint32_t *clear, uint32_t n_clear) {
