@@ -1893,10 +1893,10 @@ static int launch_wave_any(const htc_program *p, const WaveWork &w, uint32_t W, 
 // hyperbolic scenes of 18, 77, 200 objects at 400x300 132/145, 234/257, 298/306, at 512x384 184/171,
 // 333/300, 402/342, at 800x600 358/309, 646/479, 821/471; Euclidean scenes of 9, 25, 33 objects at
 // 1024x768 88/107, 176/179, 279/269, at 1600x900 139/151, 282/250, 425/359.
-constexpr uint32_t WAVE_MAX_HOPS = 16;
+constexpr uint32_t WAVE_MAX_HOPS = 16, EU_WAVE_OBJECTS = 16;
 static bool wave_pays(const htc_program *p, uint64_t pixels, uint32_t max_objects) {
     if (p->hops > WAVE_MAX_HOPS) return false;
-    return p->recipe == HTC_RECIPE_HY ? pixels >= 9u << 14 : pixels >= (1u << 20) && max_objects >= 16;
+    return p->recipe == HTC_RECIPE_HY ? pixels >= 9u << 14 : pixels >= (3u << 18) && max_objects >= EU_WAVE_OBJECTS;
 }
 
 // Wavefronts in a workspace taken from the device's pool and given back in stream order, so that
@@ -1988,7 +1988,10 @@ int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene,
     // The program keeps queues of its own for large canvases and for hyperbolic scenes of 100 objects
     // on; the other calls may run on several streams at once and work in the pool.
     const uint64_t pixels = (uint64_t)W * H;
-    if (pixels >= (1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100))
+    // Euclidean scenes of few objects need more pixels to pay for the launches (us per pass, one-pass
+    // kernel / wavefronts, 3 and 9 objects: 1024x768 80/91 and 83/93, 1440x900 122/123 and 125/124).
+    const bool few = p->recipe == HTC_RECIPE_EU && max_objects < EU_WAVE_OBJECTS;
+    if (pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100))
         return render_wavefront_impl(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);
     if (wave_pays(p, pixels, max_objects)) {
         bool done = false;

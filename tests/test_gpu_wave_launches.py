@@ -45,6 +45,23 @@ def test_batch_tiles_cover_hop_0_tiles(built, tile):
         assert np.array_equal(_bits(canvas)[0], _bits(v.canvas)[0]) and np.array_equal(_bits(canvas)[1], _bits(v.canvas)[1])
 
 
+@pytest.mark.parametrize("W,H", [(1024, 767), (1024, 768), (1280, 1023), (1280, 1024)])
+@pytest.mark.parametrize("n", [15, 16])
+def test_euclidean_routes_agree(built, W, H, n):
+    """Around the canvas sizes and object counts where Euclidean calls become wavefronts."""
+    ctx = P.Context(0)
+    scene = _scene("eu", n, 3)
+    render = P.Render(ctx, scene.recipe, scene.hops)
+    buffer = P.EntityBuffer(ctx, scene)
+    canvases = [P.Canvas(ctx, (W, H), 5) for _ in range(3)]
+    for _ in range(2):
+        render.render(buffer, canvases[0])
+    render.render_passes(buffer, canvases[1], 2)
+    render.render_wavefront(buffer, canvases[2], 2)
+    for c in canvases[1:]:
+        assert np.array_equal(_bits(canvases[0])[0], _bits(c)[0]) and np.array_equal(_bits(canvases[0])[1], _bits(c)[1])
+
+
 @pytest.mark.parametrize("kinds", [[("hy", 30, 2, 3), ("eu", 9, 7, 1)], [("eu", 6, 1, 4), ("hy", 5, 5, 1), ("eu", 20, 3, 2)],
                                    [("eu", 9, 4, 2)], [("hy", 120, 4, 2), ("hy", 3, 1, 1)]])
 @pytest.mark.parametrize("capture", [False, True])
