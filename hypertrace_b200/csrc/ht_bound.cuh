@@ -298,6 +298,65 @@ HT_D void limit_lower(Limit &l, float d, float t) {
 // Distance of a crossing from its e^(2 s) bound (the threshold built from it adds 1e-2 margins).
 HT_D float dist_from_e2(float x) { return 0.5f * LN2F * lg2_approx(x); }
 
+// Warp pre-cull (wavefront kernels, full warps whose lanes can all cull): each lane tests
+// one slot of a 32-slot chunk against the whole warp at once — F over the box of the lanes'
+// (|p|^2, x, y), the largest error allowance and the loosest thresholds of the warp — and a
+// slot the warp test culls is culled by every lane's own point test, so the lanes run that
+// test only on the pairs the warp keeps and reach the same candidate masks bit for bit. The
+// warp test adds a slack of 2^-16 of the magnitudes involved, far above the rounding of
+// either evaluation (a few units of 2^-24 each), so float rounding cannot break that
+// implication. After the coherence sort a warp's rays start in one cell, the box is small,
+// and most slots go in one test per warp instead of one per lane.
+struct WarpBox { float r2lo, r2hi, xlo, xhi, ylo, yhi, K; };
+HT_D uint32_t ord_bits(float f) {   // order-preserving map of floats (no NaN) to unsigned
+    const uint32_t b = __float_as_uint(f);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+HT_D float ord_float(uint32_t o) { return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o); }
+HT_D float warp_min(float f) { return ord_float(__reduce_min_sync(0xffffffffu, ord_bits(f))); }
+HT_D float warp_max(float f) { return ord_float(__reduce_max_sync(0xffffffffu, ord_bits(f))); }
+HT_D WarpBox warp_box(const BoundRay &r) {
+    WarpBox b;
+    b.r2lo = warp_min(r.r2); b.r2hi = warp_max(r.r2);
+    b.xlo = warp_min(r.x);   b.xhi = warp_max(r.x);
+    b.ylo = warp_min(r.y);   b.yhi = warp_max(r.y);
+    b.K = warp_max(r.K);
+    return b;
+}
+// interval of a * u over u in [lo, hi], and a bound of |a u| there
+HT_D void box_term(float a, float lo, float hi, float &flo, float &fhi, float &mag) {
+    const float p = a * lo, q = a * hi;
+    flo += fminf(p, q);
+    fhi += fmaxf(p, q);
+    mag += fmaxf(fabsf(p), fabsf(q));
+}
+// Slots of the chunk at c0 that some lane of the warp may keep (every lane calls this); the low
+// two bits of shape[q] are 0 for planes.
+HT_D uint32_t warp_survivors(const float4 *bound, const float *mags, const uint32_t *shape, uint32_t c0, uint32_t valid,
+                             const WarpBox &b, const PointCut &kp, const PointCut &kh) {
+    const uint32_t lane = threadIdx.x & 31;
+    const float hp = warp_max(kp.hi.x);   // planes: lo = -hi
+    const float lh = warp_min(kh.lo.x), hh = warp_max(kh.hi.x);
+    bool keep = false;
+    if (valid >> lane & 1u) {
+        const uint32_t q = c0 + lane;
+        const float4 rec = bound[q];
+        const float e = mags[q] * b.K;
+        float flo = rec.w, fhi = rec.w, mag = fabsf(rec.w);
+        box_term(rec.x, b.r2lo, b.r2hi, flo, fhi, mag);
+        box_term(rec.y, b.xlo, b.xhi, flo, fhi, mag);
+        box_term(rec.z, b.ylo, b.yhi, flo, fhi, mag);
+        const float slack = 0x1p-16f * (mag + e);
+        float lo = lh, hi = hh;
+        if ((shape[q] & 3u) == 0) {
+            lo = -hp;
+            hi = hp;
+        }
+        keep = !((fhi + e) + slack < lo || (flo - e) - slack > hi);   // NaN: kept
+    }
+    return __ballot_sync(0xffffffffu, keep);
+}
+
 // ---------------------------------------------------------------- Euclidean bounds
 // The same idea for unit spheres and planes under rigid maps: world-space tests with wide margins
 // that rule out objects the reference's test cannot report nearer than the best hit so far.

@@ -148,6 +148,7 @@ struct Ctx {
     const u32 *bkind;     // bits 0-1: kind, the rest: the element's index
     u32 culled;
     float4 *win;    // shared, this thread's 2 float4: the local ray of a bounded scan's winner
+    bool full;      // every lane of the warp is in the scan of the top-level vector
 };
 HT_D bool is_repeat(const Ctx &c) { return c.hasher == c.prev; }
 HT_D void hash_usize(Ctx &c, u32 x) { const u32 h = c.hasher; c.hasher = x + (h << 6) + (h << 16) - h; }
@@ -1238,7 +1239,11 @@ HT_D float ObjectVec<G, O>::detect(Ptr self, Ctx &c, Cache &cache, Light<G> &l) 
 // elements nearest the camera sets a threshold before the first exact test, each chunk of 32 elements
 // is culled by the point bound (warp-uniform) and the ray-aware bound (per lane), and the
 // survivors are tested with the threshold tightening on every nearer hit. Culling only skips
-// elements that cannot be nearer than the threshold.
+// elements that cannot be nearer than the threshold. While every lane of a warp is in the scan
+// (c.full), the warp's own bound goes before the lanes': it tests a chunk's elements one a lane,
+// and the ray-aware bound then runs over the same few elements on all lanes, without their
+// divergence (64 tiled objects at 1080p, 8 hops, 4 passes 22.1 -> 19.9 ms; at 800x600, 6 hops, 4 passes:
+// 12 objects 3010 -> 2970 us, 31 3420 -> 3240, 64 3885 -> 3405, 120 4485 -> 3410; 4 and 8 the same).
 template <class G, class O> template <int W, bool F>
 HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light<G> &l) {
     typedef VecBounds<G, O> B;
@@ -1260,6 +1265,13 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
         }
         if (best < __int_as_float(0x7f800000)) limit_lower(lim, dist_from_e2(best), br.t);
     }
+    bool warp_pre = false;
+    WarpBox wb;
+    if (c.full) {
+        __syncwarp();
+        warp_pre = __all_sync(0xFFFFFFFFu, can);
+        if (warp_pre) wb = warp_box(br);
+    }
     float min_dist = -1.0f, min_x = __int_as_float(0x7f800000);
     u32 min_index = 0xFFFFFFFFu, tested = 0;
 #pragma unroll 1
@@ -1268,9 +1280,14 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
         u32 mask = cn == 32u ? 0xFFFFFFFFu : (1u << cn) - 1u;
         if (can) {
             u32 m = 0;
+            if (warp_pre) {
+                __syncwarp();
+                m = warp_survivors(c.brec, c.bmag, c.bkind, c0, mask, wb, lim.kp, lim.kh);
+            } else {
 #pragma unroll 1
-            for (u32 j = 0; j < cn; ++j) {   // warp-uniform: broadcast loads
-                if (!culled_point(c.brec[c0 + j], c.bmag[c0 + j], br, (c.bkind[c0 + j] & 3u) == 0u ? lim.kp : lim.kh)) m |= 1u << j;
+                for (u32 j = 0; j < cn; ++j) {   // warp-uniform: broadcast loads
+                    if (!culled_point(c.brec[c0 + j], c.bmag[c0 + j], br, (c.bkind[c0 + j] & 3u) == 0u ? lim.kp : lim.kh)) m |= 1u << j;
+                }
             }
             mask = 0;
             while (m) {   // per lane: the ray-aware bound on the survivors
@@ -1392,6 +1409,7 @@ render_generic(Ptr scene, uint64_t scene_size, u32 width, u32 height, u32 tiles,
     c.bmag = nullptr;
     c.bkind = nullptr;
     c.win = nullptr;
+    c.full = false;
     if constexpr (SameType<Geo, Hy>::ok) {
         __shared__ float4 s_win[2 * Launch<Geo>::threads];
         c.win = s_win + 2 * threadIdx.x;
@@ -1454,6 +1472,7 @@ render_generic(Ptr scene, uint64_t scene_size, u32 width, u32 height, u32 tiles,
             }
             __syncthreads();
             float dist = -1.0f;
+            c.full = __all_sync(0xFFFFFFFFu, active);
             if (active) dist = Scene::template detect<W>(scene, c, cache, l);
             __syncthreads();
             if (active) {

@@ -291,64 +291,6 @@ HT_D float upper_estimate(const StagedScene &s, const BoundRay &r, uint32_t prev
     return best < __int_as_float(0x7f800000) ? dist_from_e2(best) : best;
 }
 
-// Warp pre-cull (wavefront kernels, full warps whose lanes can all cull): each lane tests
-// one slot of a 32-slot chunk against the whole warp at once — F over the box of the lanes'
-// (|p|^2, x, y), the largest error allowance and the loosest thresholds of the warp — and a
-// slot the warp test culls is culled by every lane's own point test, so the lanes run that
-// test only on the pairs the warp keeps and reach the same candidate masks bit for bit. The
-// warp test adds a slack of 2^-16 of the magnitudes involved, far above the rounding of
-// either evaluation (a few units of 2^-24 each), so float rounding cannot break that
-// implication. After the coherence sort a warp's rays start in one cell, the box is small,
-// and most slots go in one test per warp instead of one per lane.
-struct WarpBox { float r2lo, r2hi, xlo, xhi, ylo, yhi, K; };
-HT_D uint32_t ord_bits(float f) {   // order-preserving map of floats (no NaN) to unsigned
-    const uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-HT_D float ord_float(uint32_t o) { return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o); }
-HT_D float warp_min(float f) { return ord_float(__reduce_min_sync(0xffffffffu, ord_bits(f))); }
-HT_D float warp_max(float f) { return ord_float(__reduce_max_sync(0xffffffffu, ord_bits(f))); }
-HT_D WarpBox warp_box(const BoundRay &r) {
-    WarpBox b;
-    b.r2lo = warp_min(r.r2); b.r2hi = warp_max(r.r2);
-    b.xlo = warp_min(r.x);   b.xhi = warp_max(r.x);
-    b.ylo = warp_min(r.y);   b.yhi = warp_max(r.y);
-    b.K = warp_max(r.K);
-    return b;
-}
-// interval of a * u over u in [lo, hi], and a bound of |a u| there
-HT_D void box_term(float a, float lo, float hi, float &flo, float &fhi, float &mag) {
-    const float p = a * lo, q = a * hi;
-    flo += fminf(p, q);
-    fhi += fmaxf(p, q);
-    mag += fmaxf(fabsf(p), fabsf(q));
-}
-// Slots of chunk [c0, c0 + cn) that some lane of the warp may keep (every lane calls this).
-HT_D uint32_t warp_survivors(const StagedScene &s, uint32_t c0, uint32_t valid, const WarpBox &b,
-                             const PointCut &kp, const PointCut &kh) {
-    const uint32_t lane = threadIdx.x & 31;
-    const float hp = warp_max(kp.hi.x);   // planes: lo = -hi
-    const float lh = warp_min(kh.lo.x), hh = warp_max(kh.hi.x);
-    bool keep = false;
-    if (valid >> lane & 1u) {
-        const uint32_t q = c0 + lane;
-        const float4 rec = s.bound[q];
-        const float e = s.mag[q] * b.K;
-        float flo = rec.w, fhi = rec.w, mag = fabsf(rec.w);
-        box_term(rec.x, b.r2lo, b.r2hi, flo, fhi, mag);
-        box_term(rec.y, b.xlo, b.xhi, flo, fhi, mag);
-        box_term(rec.z, b.ylo, b.yhi, flo, fhi, mag);
-        const float slack = 0x1p-16f * (mag + e);
-        float lo = lh, hi = hh;
-        if (s.shape[q] == 0) {
-            lo = -hp;
-            hi = hp;
-        }
-        keep = !((fhi + e) + slack < lo || (flo - e) - slack > hi);   // NaN: kept
-    }
-    return __ballot_sync(0xffffffffu, keep);
-}
-
 // WARP: the warp pre-cull is compiled in; `full_warp` (all 32 lanes of the warp are in this
 // call together, uniform across the warp) turns it on.
 template <bool WARP = false>
@@ -390,7 +332,7 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
                 // survivors of the point bound: 1080p / 200 objects, 8 passes 15.0 against 14.1 ms)
                 if (warp_pre) {   // uniform: every lane can cull
                     __syncwarp();
-                    m = warp_survivors(s, c0, valid, wb, lim.kp, lim.kh);
+                    m = warp_survivors(s.bound, s.mag, s.shape, c0, valid, wb, lim.kp, lim.kh);
                 }
             } else {
                 // this lane's survivors of the point bound, two slots at once
