@@ -292,8 +292,9 @@ HT_D float upper_estimate(const StagedScene &s, const BoundRay &r, uint32_t prev
 }
 
 // WARP: the warp pre-cull is compiled in; `full_warp` (all 32 lanes of the warp are in this
-// call together, uniform across the warp) turns it on.
-template <bool WARP = false>
+// call together, uniform across the warp) turns it on. 1: callers whose warps are nearly always
+// full, the others look at every object; 2: warps that are not full take the point bound by lane.
+template <int WARP = 0>
 HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &prev_hash,
                  Col &intensity, Col &emission, bool &hit, uint32_t &n_exact, bool last, bool full_warp = false) {
     // Nearest hit with ties to the lowest scene index (object/vector.inl:37-50): candidates
@@ -311,7 +312,7 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
     const uint32_t h0 = (s.n_planes + 1) & ~1u;   // the first horosphere's slot
     bool warp_pre = false;
     WarpBox wb;
-    if constexpr (WARP) {
+    if constexpr (WARP != 0) {
         if (full_warp) {
             __syncwarp();
             warp_pre = __all_sync(0xffffffffu, can_cull);
@@ -326,7 +327,7 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
         uint32_t mask = valid;
         if (can_cull) {
             uint32_t m = valid;   // objects to look at one by one
-            if constexpr (WARP) {
+            if constexpr (WARP != 0) {
                 // those that the warp keeps: one object at a time for all lanes, so loads are
                 // broadcasts and a shape's test runs without divergence (each lane taking its own
                 // survivors of the point bound: 1080p / 200 objects, 8 passes 15.0 against 14.1 ms)
@@ -334,7 +335,8 @@ HT_D bool hop_hy(const StagedScene &s, HyPath &ray, uint32_t &rng, uint32_t &pre
                     __syncwarp();
                     m = warp_survivors(s.bound, s.mag, s.shape, c0, valid, wb, lim.kp, lim.kh);
                 }
-            } else {
+            }
+            if (WARP != 1 && !warp_pre) {
                 // this lane's survivors of the point bound, two slots at once
                 m = 0;
                 // kept rolled: the kernel is bound by instruction fetch as much as by issue
