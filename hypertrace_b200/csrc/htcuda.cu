@@ -1891,13 +1891,15 @@ static int launch_wave_any(const htc_program *p, const WaveWork &w, uint32_t W, 
 // Whether one pass is faster as wavefronts than with the one-pass kernel. Small canvases leave the
 // deeper hop launches most of the GPU idle; a hop count beyond the workloads' would add launches
 // for queues that are empty. Measured, one call of one pass, one-pass kernel / wavefronts in us:
-// hyperbolic scenes of 18, 77, 200 objects at 400x300 132/145, 234/257, 298/306, at 512x384 184/171,
-// 333/300, 402/342, at 800x600 358/309, 646/479, 821/471; Euclidean scenes of 9, 25, 33 objects at
-// 1024x768 88/107, 176/179, 279/269, at 1600x900 139/151, 282/250, 425/359.
-constexpr uint32_t WAVE_MAX_HOPS = 16, EU_WAVE_OBJECTS = 16;
+// hyperbolic scenes of 18, 77, 200 objects at 400x300 126/139, 217/245, 268/300, at 512x384 176/166,
+// 333/297, 402/337, at 800x600 346/297, 646/467, 821/456, of 2, 4 and 8 objects at 512x384 26/46, 67/104,
+// 218/193, at 800x600 47/56, 129/140, 454/360, at 1280x720 88/84, 228/204, 791/594; Euclidean scenes of 9,
+// 17, 25, 33 objects at 800x600 62/86, 118/130, 121/138, 190/217, at 1024x768 89/105, 177/163, 179/172,
+// 281/255.
+constexpr uint32_t WAVE_MAX_HOPS = 16, EU_WAVE_OBJECTS = 16, WAVE_PIXELS = 9u << 14;
 static bool wave_pays(const htc_program *p, uint64_t pixels, uint32_t max_objects) {
     if (p->hops > WAVE_MAX_HOPS) return false;
-    return p->recipe == HTC_RECIPE_HY ? pixels >= 9u << 14 : pixels >= (3u << 18) && max_objects >= EU_WAVE_OBJECTS;
+    return p->recipe == HTC_RECIPE_HY ? pixels >= (max_objects < 6 ? 3u << 18 : WAVE_PIXELS) : pixels >= (3u << 18) && max_objects >= EU_WAVE_OBJECTS;
 }
 
 // Wavefronts in a workspace taken from the device's pool and given back in stream order, so that
@@ -1986,13 +1988,14 @@ int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene,
     int rc = validate_render_args(p, W, H, scene, scene_size, canvas, seeds, &max_objects, &smem);
     if (rc) return rc;
     if (passes == 0) return HTC_OK;
-    // The program keeps queues of its own for large canvases and for hyperbolic scenes of 100 objects
-    // on; the other calls may run on several streams at once and work in the pool.
+    // The program keeps queues of its own for large canvases and, where wavefronts pay at all, for
+    // hyperbolic scenes of 100 objects on (200 objects, us per pass, one-pass kernel / wavefronts: 320x240
+    // 190/252, 400x300 260/280); the other calls may run on several streams at once and work in the pool.
     const uint64_t pixels = (uint64_t)W * H;
     // Euclidean scenes of few objects need more pixels to pay for the launches (us per pass, one-pass
     // kernel / wavefronts, 3 and 9 objects: 1024x768 80/91 and 83/93, 1440x900 122/123 and 125/124).
     const bool few = p->recipe == HTC_RECIPE_EU && max_objects < EU_WAVE_OBJECTS;
-    if (pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100))
+    if (pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100 && pixels >= WAVE_PIXELS))
         return render_wavefront_impl(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);
     if (wave_pays(p, pixels, max_objects)) {
         bool done = false;

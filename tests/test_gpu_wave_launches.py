@@ -62,6 +62,22 @@ def test_euclidean_routes_agree(built, W, H, n):
         assert np.array_equal(_bits(canvases[0])[0], _bits(c)[0]) and np.array_equal(_bits(canvases[0])[1], _bits(c)[1])
 
 
+@pytest.mark.parametrize("W,H,n", [(512, 287, 120), (512, 288, 120), (512, 288, 5), (512, 288, 6), (1024, 767, 5), (1024, 768, 5)])
+def test_hyperbolic_routes_agree(built, W, H, n):
+    """Around the canvas sizes and object counts where hyperbolic calls become wavefronts."""
+    ctx = P.Context(0)
+    scene = _scene("hy", n, 4)
+    render = P.Render(ctx, scene.recipe, scene.hops)
+    buffer = P.EntityBuffer(ctx, scene)
+    canvases = [P.Canvas(ctx, (W, H), 6) for _ in range(3)]
+    for _ in range(2):
+        render.render(buffer, canvases[0])
+    render.render_passes(buffer, canvases[1], 2)
+    render.render_wavefront(buffer, canvases[2], 2)
+    for c in canvases[1:]:
+        assert np.array_equal(_bits(canvases[0])[0], _bits(c)[0]) and np.array_equal(_bits(canvases[0])[1], _bits(c)[1])
+
+
 @pytest.mark.parametrize("kinds", [[("hy", 30, 2, 3), ("eu", 9, 7, 1)], [("eu", 6, 1, 4), ("hy", 5, 5, 1), ("eu", 20, 3, 2)],
                                    [("eu", 9, 4, 2)], [("hy", 120, 4, 2), ("hy", 3, 1, 1)]])
 @pytest.mark.parametrize("capture", [False, True])
