@@ -1162,8 +1162,9 @@ template <class O0, class... O> struct ChoiceTraits<O0, O...> {
 // HTG_BOUND_CAP elements. With the elements ordered by distance even a few are worth it (hy_tiled
 // type at 800x600, 6 hops, 4 passes, with / without the bounds: 4 elements 1645 / 1738 us, 12 3008 /
 // 3616, 31 3414 / 7683; 64 in index order with an estimate over 32 6049, by distance over 16 3874).
-#ifndef HTG_EST   // elements the upper estimate looks at (64 at 1080p, 4 passes: 8 26.6 ms, 12 22.2, 16 22.1, 24 22.6)
-#define HTG_EST 16u
+#ifndef HTG_EST   // elements the upper estimate looks at (64 at 1080p, 4 passes: 8 23.4 ms, 12 19.74, 16 19.84,
+                  // 24 20.7; 20, 31, 120 at 800x600, 12 / 16: 3188 / 3300 us, 3140 / 3235, 3305 / 3405)
+#define HTG_EST 12u
 #endif
 #ifndef HTG_BOUND_CAP
 #define HTG_BOUND_CAP 256u
