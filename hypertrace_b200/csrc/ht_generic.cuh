@@ -1160,8 +1160,8 @@ template <class O0, class... O> struct ChoiceTraits<O0, O...> {
 // record per element (stage_bound of the element's map) in shared memory, staged once per
 // block by render_generic when the vector is the scene's top-level object and holds up to
 // HTG_BOUND_CAP elements. With the elements ordered by distance even a few are worth it (hy_tiled
-// type at 800x600, 6 hops, 4 passes, with / without the bounds: 4 elements 1645 / 1738 us, 12 3008 /
-// 3616, 31 3414 / 7683; 64 in index order with an estimate over 32 6049, by distance over 16 3874).
+// type at 800x600, 6 hops, 4 passes, with / without the bounds: 4 elements 1665 / 1738 us, 12 2965 /
+// 3616, 31 3140 / 7683; 64 in index order with an estimate over 32 6049, by distance over 16 3874).
 #ifndef HTG_EST   // elements the upper estimate looks at (64 at 1080p, 4 passes: 8 23.4 ms, 12 19.74, 16 19.84,
                   // 24 20.7; 20, 31, 120 at 800x600, 12 / 16: 3188 / 3300 us, 3140 / 3235, 3305 / 3405)
 #define HTG_EST 12u
@@ -1268,7 +1268,7 @@ HT_D float ObjectVec<G, O>::detect_bounded(Ptr self, Ctx &c, Cache &cache, Light
     }
     bool warp_pre = false;
     WarpBox wb;
-    if (c.full) {
+    if (staged && c.full) {   // staged: never a vector inside another, whose lanes may come apart
         __syncwarp();
         warp_pre = __all_sync(0xFFFFFFFFu, can);
         if (warp_pre) wb = warp_box(br);

@@ -63,3 +63,23 @@ def test_example_passes_equal_single_passes(built, recipe, W, H):
     assert np.array_equal(a[0].view(np.uint32), canvas.image.cpu().numpy().view(np.uint32))
     assert np.array_equal(a[1], canvas.seeds.cpu().numpy())
     assert a[2][0] == 4 * W * H
+
+
+@pytest.mark.parametrize("W,H", [(64, 64), (333, 77)])
+def test_vector_below_a_mapped_object(built, W, H):
+    """A vector that is not the scene's top-level object has no staged bounds and takes no test of a
+    whole warp: under an identity map it finds what the same vector at the top finds. One hop: the
+    map moves a ray by its last bits, so only pixels within some 1e-6 of an object's edge may differ."""
+    ctx = P.Context(0)
+    scene = S.hyperbolic_scene(14, 26, 3.0, 1, 77, camera=S.random_moebius(np.random.default_rng(7), 0.5))
+    flat = T.hearth_type()
+    vector = T.ObjectVec("Hy", T.MappedObject("Hy", T.Covered("Hy", T.ShapeChoice("Hy", ("Plane", T.PlaneHy()), ("Horosphere", T.Horosphere())),
+                                                              T.hearth_material()), T.Moebius()))
+    nested = T.SceneImpl("Hy", T.MappedView("Hy", T.PointView("Hy"), T.Moebius()), T.MappedObject("Hy", vector, T.Moebius()), T.ConstBg())
+    value = T.hearth_value(scene)
+    below = dict(value, object={"map": np.array([[1, 0], [0, 1]], dtype=np.complex128), "inner": value["object"]})
+    a = _render(P.Render.build(ctx, flat, 1), T.serialize(flat, value), W, H, 2, 3)
+    b = _render(P.Render.build(ctx, nested, 1), T.serialize(nested, below), W, H, 2, 3)
+    assert b[2][0] == a[2][0] == 2 * W * H
+    same = (a[0].view(np.uint32).reshape(-1, 4) == b[0].view(np.uint32).reshape(-1, 4)).all(axis=1)
+    assert same.mean() >= 0.999 and (a[1] == b[1]).mean() >= 0.999
