@@ -142,7 +142,7 @@ HT_D void mixture_last(const Material &m, uint32_t &rng, const Col &intensity, C
 }
 
 // Staged scene, per slot in shared memory (hyperbolic scenes: planes first, then
-// horospheres, each in scene order; Euclidean scenes: slot = scene index).
+// horospheres, each by distance from the camera; Euclidean scenes: slot = scene index).
 struct StagedScene {
     const float4 *inv;       // shared, 2 per slot
     const uint32_t *shape;   // shared

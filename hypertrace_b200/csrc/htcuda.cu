@@ -6,7 +6,9 @@
 //   render_wave<R, FH>   one launch per hop depth of a pass (FH: hop 0 from the pixels, or a
 //                        later hop from a queue of ray states); survivors are appended to
 //                        the other queue with warp-aggregated atomics, so warps scan with
-//                        full lanes. The form htc_render_passes uses.
+//                        full lanes. The form of all but small calls.
+//   k_stage, k_batch_stage  the scene's staged image for these launches, once per call.
+//   k_sort_*, k_bsort_*  the coherence sort of a hop depth's queue.
 //   render_batch_wave<RF, FH>  the same over many views at once, one launch per pass index,
 //                        hop depth and recipe, tiles of the views' queues cut on the device.
 //   render_persistent<R> one launch for P passes: warps pull pixels from a queue, each lane
@@ -14,9 +16,9 @@
 //                        in place (the allocation-free entry point uses it).
 //   post kernels         extract / gamma / pack (processing/src/canvas.rs:126-135,176-186,
 //                        processing/src/filter/gamma.rs:10-19) and their fused form.
-// Every render kernel stages the scene's inverse object maps, distance-bound records and
-// shape indices in shared memory once per block (per view change in the batched kernels);
-// the object scan reads them as warp-uniform broadcasts. Each pixel's samples take the same
+// Every render kernel holds the scene's inverse object maps, distance-bound records and
+// shape indices in shared memory: staged by each block of the one-pass and persistent kernels,
+// copied from the image by the wavefront kernels (per view change in the batched ones). Each pixel's samples take the same
 // float operations in the same order in every form, so all forms give the same bits.
 #include <cuda_runtime.h>
 

@@ -62,7 +62,8 @@ extern "C" {
                                   the OpenCL order (first draw -> x). */
 #define HTC_FLAG_NO_SORT 2u    /* hyperbolic wavefronts (htc_render_wavefront / _passes) take
                                   each hop depth's paths in queue order instead of sorting them
-                                  by direction and start cell first; the results are the same
+                                  by direction and start cell first (which they do from 2^19
+                                  pixels and 100 objects on); the results are the same
                                   bits either way (htc_program_create only). */
 
 /* Render statistics written by the entry points that take a `stats` pointer (device
@@ -125,16 +126,21 @@ int htc_stream_sync(void *stream);
  *   scene       device pointer to the serialized scene bytes (EntityBuffer, buffer.rs:14-29)
  *   scene_size  its size in bytes (bounds every device read of the scene)
  *   canvas      device float4[width*height];  seeds: device uint32[width*height]
- * Asynchronous on `stream`; scene validity is reported by htc_program_check. */
+ * Asynchronous on `stream`; scene validity is reported by htc_program_check.
+ * Larger canvases run as wavefronts (htc_render_wavefront) in a workspace of 136 bytes per
+ * pixel and more, taken from and given back to a stream-ordered pool that the programs of a
+ * device share; small ones, calls on a capturing stream and calls for which the pool has no
+ * memory run a one-pass kernel. The results are the same bits. */
 int htc_render(htc_program *program, uint32_t width, uint32_t height, const void *scene,
                size_t scene_size, float *canvas, uint32_t *seeds, void *stream);
 
 /* `passes` successive passes; bit-identical to `passes` htc_render calls (each pixel's
- * samples run in order and keep its RNG stream). For the built-in recipes this is
- * htc_render_wavefront, so the program keeps the queues that form allocates -- except for
- * canvases under 2^19 pixels whose scene is Euclidean or holds fewer than 100 objects, which
- * run the one-pass kernel once per pass (faster there; the same bits either way). stats (optional, device uint64[HTC_STAT_COUNT])
- * accumulates the HTC_STAT_* counters. */
+ * samples run in order and keep its RNG stream). From 2^19 pixels on (5 * 2^18 for
+ * Euclidean scenes of fewer than 16 objects), and from 147456 pixels on for hyperbolic scenes of
+ * 100 objects and more, this is htc_render_wavefront for the built-in recipes, so the program
+ * keeps the queues that form allocates; smaller canvases render as htc_render does, pass by pass
+ * or as wavefronts in the pool (the same bits either way). stats (optional, device
+ * uint64[HTC_STAT_COUNT]) accumulates the HTC_STAT_* counters. */
 int htc_render_passes(htc_program *program, uint32_t width, uint32_t height, const void *scene,
                       size_t scene_size, float *canvas, uint32_t *seeds, uint32_t passes,
                       uint64_t *stats, void *stream);
@@ -170,7 +176,7 @@ int htc_render_passes_noalloc(int recipe, uint32_t light_hops, int address_width
                               float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats,
                               uint32_t *status, void *stream);
 
-/* htc_render with statistics (the plain one-pass kernel). */
+/* htc_render with statistics. */
 int htc_render_ex(htc_program *program, uint32_t width, uint32_t height, const void *scene,
                   size_t scene_size, float *canvas, uint32_t *seeds, uint64_t *stats,
                   void *stream);
@@ -212,7 +218,8 @@ int htc_batch_set_views(htc_batch *batch, const htc_view *views, uint32_t n_view
  * them (growing waits for the launches already enqueued on `stream`). */
 int htc_batch_reserve(htc_batch *batch, uint64_t pixels, uint32_t max_hops, void *stream);
 /* Renders every view's `passes`: one launch per pass index, hop depth and recipe over all the
- * views (wavefronts). stats as in htc_render_passes. */
+ * views (wavefronts); the Euclidean launches run on a stream of the batch's own, which waits for
+ * `stream` and for which `stream` waits in turn. stats as in htc_render_passes. */
 int htc_batch_render(htc_batch *batch, uint64_t *stats, void *stream);
 /* The same launch through a CUDA graph captured on first use and re-captured after
  * htc_batch_set_views, after an htc_batch_reserve that grows the queues, and when `stats`
