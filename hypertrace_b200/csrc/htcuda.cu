@@ -106,6 +106,8 @@ struct htc_program {
     int double_support;        // scene bytes in the double_support layout, narrowed before rendering
     uint8_t *narrow_buf;       // the narrowed (f32 layout) scene, grown on demand
     size_t narrow_bytes;
+    std::mutex narrow_mutex;   // from a call's narrowing to its last launch
+    cudaEvent_t narrow_done;   // the last call's use of narrow_buf
 };
 
 // ============================================================================ staging
@@ -1589,6 +1591,7 @@ int htc_program_create(int recipe, uint32_t light_hops, int address_width, int d
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&p->max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e == cudaSuccess) e = cudaMalloc(&p->d_err, sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(p->d_err, 0, sizeof(uint32_t));
+    if (e == cudaSuccess && double_support) e = cudaEventCreateWithFlags(&p->narrow_done, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         if (p->d_err) cudaFree(p->d_err);
         delete p;
@@ -1598,6 +1601,7 @@ int htc_program_create(int recipe, uint32_t light_hops, int address_width, int d
     int rc = recipe == HTC_RECIPE_HY ? set_smem_attr<RECIPE_HY>(p->max_smem) : set_smem_attr<RECIPE_EU>(p->max_smem);
     if (rc) {
         cudaFree(p->d_err);
+        if (p->narrow_done) cudaEventDestroy(p->narrow_done);
         delete p;
         return rc;
     }
@@ -1615,6 +1619,7 @@ void htc_program_destroy(htc_program *p) {
     if (p->image) cudaFree(p->image);
     pool_leave(p->device);
     if (p->narrow_buf) cudaFree(p->narrow_buf);
+    if (p->narrow_done) cudaEventDestroy(p->narrow_done);
     if (p->generic) generic_program_destroy(p->generic);
     delete p;
 }
@@ -1700,9 +1705,29 @@ static int render_generic_program(htc_program *p, uint32_t W, uint32_t H, const 
 
 }  // extern "C"
 
+// A call's use of the program's narrowed scene. Its launches read that one buffer to the end, so the
+// uses of several streams and threads follow one another: the next call's stream waits for the event
+// that ends this one. (On a capturing stream there is no event outside the capture to wait for: such a
+// call, and the replays of its graph, are the caller's to keep apart, as the header says.)
+struct NarrowUse {
+    htc_program *p = nullptr;
+    cudaStream_t st = nullptr;
+    std::unique_lock<std::mutex> lock;
+    ~NarrowUse() {
+        if (p) cudaEventRecord(p->narrow_done, st);
+    }
+};
+static bool capturing(cudaStream_t st) {   // or cannot be told
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // A double_support program's scene, narrowed on `stream` into the program's f32-layout buffer
-// (k_narrow_scene); *scene / *scene_size then name that buffer. Other programs: unchanged.
-static int narrow_scene(htc_program *p, const void **scene, size_t *scene_size, void *stream) {
+// (k_narrow_scene); *scene / *scene_size then name that buffer, which is the call's until `use` ends.
+// Other programs: unchanged.
+static int narrow_scene(htc_program *p, const void **scene, size_t *scene_size, void *stream, NarrowUse &use) {
     if (!p || !p->double_support) return HTC_OK;
     const int li = p->recipe == HTC_RECIPE_HY ? 0 : 1;
     if (!*scene) return fail(HTC_ERR_INVALID, "scene must be a device pointer");
@@ -1714,6 +1739,12 @@ static int narrow_scene(htc_program *p, const void **scene, size_t *scene_size, 
     const size_t dst_objects = li == 0 ? Layout<RECIPE_HY>::OBJECTS : Layout<RECIPE_EU>::OBJECTS;
     const size_t bytes = dst_objects + (size_t)cap * OBJ_STRIDE;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    use.lock = std::unique_lock<std::mutex>(p->narrow_mutex);
+    if (!capturing(st)) {
+        HTC_CUDA(cudaStreamWaitEvent(st, p->narrow_done, 0));
+        use.p = p;
+        use.st = st;
+    }
     if (p->narrow_bytes < bytes) {
         if (p->narrow_buf) HTC_CUDA(cudaFree(p->narrow_buf));
         p->narrow_buf = nullptr;
@@ -1905,18 +1936,14 @@ static bool wave_pays(const htc_program *p, uint64_t pixels, uint32_t max_object
 }
 
 // Wavefronts in a workspace taken from the device's pool and given back in stream order, so that
-// calls of one program on several streams or threads do not meet. *done = false: none was to be
+// calls of one program on several streams or threads do not meet (in the scene of a double_support
+// program they would: NarrowUse). *done = false: none was to be
 // had (no memory, a capturing stream); nothing was launched.
 static int render_wave_pooled(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, uint32_t max_objects,
                               size_t smem, float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, cudaStream_t st,
                               bool *done) {
     *done = false;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
-        cudaGetLastError();
-        return HTC_OK;
-    }
-    if (capture != cudaStreamCaptureStatusNone) return HTC_OK;
+    if (capturing(st)) return HTC_OK;
     WaveWork w;
     const size_t bytes = wave_work_block(p, (uint64_t)W * H, max_objects, nullptr, &w);
     void *block = pool_take(p->device, bytes, st);
@@ -1947,8 +1974,9 @@ extern "C" {
 int htc_render_ex(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
                   float *canvas, uint32_t *seeds, uint64_t *stats, void *stream) {
     if (p && p->generic) return render_generic_program(p, W, H, scene, scene_size, canvas, seeds, 1, stats, stream);
+    NarrowUse narrow;
     if (p && canvas && seeds && W && H) {   // argument errors are reported by the render checks
-        int rc = narrow_scene(p, &scene, &scene_size, stream);
+        int rc = narrow_scene(p, &scene, &scene_size, stream, narrow);
         if (rc) return rc;
     }
     uint32_t max_objects = 0;
@@ -1971,8 +1999,9 @@ int htc_render(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t
 
 int htc_render_wavefront(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
                          float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, void *stream) {
+    NarrowUse narrow;
     if (p && canvas && seeds && W && H && passes) {
-        int rc = narrow_scene(p, &scene, &scene_size, stream);
+        int rc = narrow_scene(p, &scene, &scene_size, stream, narrow);
         if (rc) return rc;
     }
     return render_wavefront_impl(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);
@@ -1981,8 +2010,9 @@ int htc_render_wavefront(htc_program *p, uint32_t W, uint32_t H, const void *sce
 int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size,
                       float *canvas, uint32_t *seeds, uint32_t passes, uint64_t *stats, void *stream) {
     if (p && p->generic) return render_generic_program(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);
+    NarrowUse narrow;
     if (p && canvas && seeds && W && H && passes) {
-        int rc = narrow_scene(p, &scene, &scene_size, stream);
+        int rc = narrow_scene(p, &scene, &scene_size, stream, narrow);
         if (rc) return rc;
     }
     uint32_t max_objects = 0;

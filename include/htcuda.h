@@ -91,7 +91,9 @@ int htc_set_device(int device);
  * every render call narrows them on the device to the f32 layout (each f64 rounded to the
  * nearest f32, the value the reference serializes without double_support) into a buffer the
  * program keeps, then transports in FP32 -- the result is bit for bit that of the f32
- * serialization; an object count the buffer cannot hold is reported by htc_program_check. */
+ * serialization; an object count the buffer cannot hold is reported by htc_program_check. Such
+ * calls follow one another on the device whatever their streams, for they share that buffer; a graph
+ * captured from one must not be replayed beside other calls of the program. */
 int htc_program_create(int recipe, uint32_t light_hops, int address_width, int double_support,
                        uint32_t flags, htc_program **out);
 void htc_program_destroy(htc_program *program);
