@@ -60,7 +60,9 @@ constexpr int minb_batch(bool eu) { return eu ? 6 : 5; }
 // dependent launch). A kernel waits for the end of the one before it (wait_previous) and then lets
 // the next one start (launch_next), whose blocks take the places that this one's leave, load
 // the scene and wait in turn. So before its wait a kernel may read what the launch before the
-// last, or anything earlier, wrote: the scene's bytes and image. 1080p / 200 objects, 8 passes:
+// last, or anything earlier, wrote: the scene's bytes and image. And nothing that the launch before
+// writes may be a `const __restrict__` argument: that promises data which no one changes while the
+// kernel runs, and the kernel runs before its wait (test_overlap_qualifiers.py). 1080p / 200 objects, 8 passes:
 // 10.7 -> 9.9 ms; 640x480, the same scene, unsorted: 486 -> 396 us per pass.
 __device__ __forceinline__ void launch_next() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
@@ -1236,9 +1238,9 @@ __global__ void __launch_bounds__(SORT_THREADS) k_bsort_keys(const BatchView *__
 __global__ void __launch_bounds__(SORT_THREADS) k_bsort_scatter(const BatchView *__restrict__ views,
                                                                const uint32_t *__restrict__ order, uint32_t n_seg,
                                                                uint32_t n_views, uint32_t pass, uint32_t h,
-                                                               const uint32_t *cnt, const uint32_t *__restrict__ key,
-                                                               const uint32_t *__restrict__ hist, uint32_t *next_hist,
-                                                               const uint32_t *__restrict__ place,
+                                                               const uint32_t *cnt, const uint32_t *key,
+                                                               const uint32_t *hist, uint32_t *next_hist,
+                                                               const uint32_t *place,
                                                                uint32_t *__restrict__ perm) {
     extern __shared__ uint32_t s_base[];   // SORT_BINS, then n_seg counts and n_seg + 1 window numbers
     uint32_t *s_count = s_base + SORT_BINS, *s_win = s_count + n_seg;
