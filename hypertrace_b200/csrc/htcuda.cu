@@ -102,8 +102,7 @@ struct htc_program {
     uint32_t *d_wave_ctr;      // 2 counters per hop depth, two sets
     void *sort_buf;            // coherence sort of the hyperbolic queues (SortBuf), grown with them
     size_t sort_slots;
-    float4 *image;             // the scene's image (stage_image), grown on demand
-    size_t image_cap;          // its size in float4
+    float4 *image;             // the scene's image (stage_image), of the largest that can be staged
     int device;                // whose pool it uses (render_wave_pooled); -1: none
     int double_support;        // scene bytes in the double_support layout, narrowed before rendering
     uint8_t *narrow_buf;       // the narrowed (f32 layout) scene, grown on demand
@@ -1788,25 +1787,27 @@ static int render_plain_pass(htc_program *p, uint32_t W, uint32_t H, const void 
 // coherence saves less. Measured, sorted / in queue order, us per pass: 1080p / 200 objects (4.7 hops
 // a path) 2764 / 3029, (2.0 hops) 1232 / 1245, 720p / 120 objects 1483 / 1542, 720p / 77 objects 721 / 708,
 // 1080p / 18 objects 1082 / 1070, 640x480 / 200 objects 471 / 396.
+static bool wave_sortable(const htc_program *p, uint64_t pixels) {
+    return p->recipe == HTC_RECIPE_HY && !(p->flags & HTC_FLAG_NO_SORT) && pixels >= (1u << 19);
+}
 static bool wave_sorted(const htc_program *p, uint64_t pixels, uint32_t max_objects) {
-    return !(p->flags & HTC_FLAG_NO_SORT) && pixels >= (1u << 19) && max_objects >= 100;
+    return wave_sortable(p, pixels) && max_objects >= 100;
 }
 // Queues of W*H slots each (a hop never has more paths than pixels) and the hop counters;
-// allocated on the first call that needs more and kept with the program.
-static int wave_reserve(htc_program *p, size_t slots, uint32_t max_objects) {
-    if (p->image_cap < image_words(max_objects)) {
-        if (p->image) HTC_CUDA(cudaFree(p->image));
-        p->image = nullptr;
-        p->image_cap = 0;
-        HTC_CUDA(cudaMalloc(&p->image, sizeof(float4) * image_words(max_objects)));
-        p->image_cap = image_words(max_objects);
-    }
+// allocated on the first call that needs more and kept with the program. All of it goes by the canvas
+// alone, whatever the scene: a call on a canvas no larger than an earlier one's allocates nothing,
+// so it can be captured, and frees nothing that a captured call's graph works in.
+static bool wave_reserved(const htc_program *p, size_t slots) {
+    return p->image && p->d_wave_ctr && p->wave_slots >= slots && (!wave_sortable(p, slots) || p->sort_slots >= slots);
+}
+static int wave_reserve(htc_program *p, size_t slots) {
+    if (!p->image) HTC_CUDA(cudaMalloc(&p->image, sizeof(float4) * (1 + (size_t)p->max_smem / 16)));   // image_words of the largest scene
     if (!p->d_wave_ctr) {
         // 2 words per hop depth, two sets
         HTC_CUDA(cudaMalloc(&p->d_wave_ctr, 4 * sizeof(uint32_t) * (size_t)p->hops));
     }
     slots = (slots + 63) & ~(size_t)63;   // keeps the second queue and every array 16-byte aligned
-    if (p->recipe == HTC_RECIPE_HY && wave_sorted(p, slots, max_objects) && p->sort_slots < slots) {
+    if (wave_sortable(p, slots) && p->sort_slots < slots) {
         if (p->sort_buf) {
             HTC_CUDA(cudaFree(p->sort_buf));
             p->sort_buf = nullptr;
@@ -1848,7 +1849,7 @@ static size_t wave_work_block(const htc_program *p, uint64_t pixels, uint32_t ma
     };
     w->image = reinterpret_cast<float4 *>(take(sizeof(float4) * image_words(max_objects)));
     w->ctr = reinterpret_cast<uint32_t *>(take(4 * sizeof(uint32_t) * (size_t)p->hops));
-    w->sort_slots = p->recipe == HTC_RECIPE_HY && wave_sorted(p, pixels, max_objects) ? slots : 0;
+    w->sort_slots = wave_sorted(p, pixels, max_objects) ? slots : 0;
     w->sort = take(w->sort_slots ? sort_bytes(slots, (uint32_t)p->num_sms) : 0);
     w->queues = take(2 * WAVE_SLOT_BYTES * slots);
     w->slots = slots;
@@ -1882,7 +1883,7 @@ static int launch_wave(const htc_program *p, const WaveWork &w, uint32_t W, uint
     const uint64_t blocks0 = std::min<uint64_t>((uint64_t)per_sm0 * (uint64_t)p->num_sms, needed);
     const WaveQueue q[2] = {wave_queue(w, 0), wave_queue(w, 1)};
     const WaveQueue none = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    const bool sorted = R == RECIPE_HY && wave_sorted(p, (uint64_t)W * H, max_objects);
+    const bool sorted = wave_sorted(p, (uint64_t)W * H, max_objects);
     const unsigned sort_blocks = (unsigned)p->num_sms;
     const SortBuf sb = sorted ? sort_buf_at(w.sort, w.sort_slots, sort_blocks) : SortBuf{};
     const size_t sort_smem = sizeof(uint32_t) * SORT_BINS;
@@ -1965,7 +1966,7 @@ static int render_wavefront_impl(htc_program *p, uint32_t W, uint32_t H, const v
     int rc = validate_render_args(p, W, H, scene, scene_size, canvas, seeds, &max_objects, &smem);
     if (rc) return rc;
     if (passes == 0) return HTC_OK;
-    rc = wave_reserve(p, (size_t)W * H, max_objects);
+    rc = wave_reserve(p, (size_t)W * H);
     if (rc) return rc;
     return launch_wave_any(p, wave_work_owned(p), W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats,
                            reinterpret_cast<cudaStream_t>(stream));
@@ -2029,7 +2030,8 @@ int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene,
     // Euclidean scenes of few objects need more pixels to pay for the launches (us per pass, one-pass
     // kernel / wavefronts, 3 and 9 objects: 1024x768 80/91 and 83/93, 1440x900 122/123 and 125/124).
     const bool few = p->recipe == HTC_RECIPE_EU && max_objects < EU_WAVE_OBJECTS;
-    if (pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100 && pixels >= WAVE_PIXELS))
+    const bool own = pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100 && pixels >= WAVE_PIXELS);
+    if (own && (wave_reserved(p, pixels) || !capturing(reinterpret_cast<cudaStream_t>(stream))))
         return render_wavefront_impl(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);
     if (wave_pays(p, pixels, max_objects)) {
         bool done = false;

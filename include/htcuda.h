@@ -141,8 +141,10 @@ int htc_render(htc_program *program, uint32_t width, uint32_t height, const void
  * Euclidean scenes of fewer than 16 objects), and from 147456 pixels on for hyperbolic scenes of
  * 100 objects and more, this is htc_render_wavefront for the built-in recipes, so the program
  * keeps the queues that form allocates; smaller canvases render as htc_render does, pass by pass
- * or as wavefronts in the pool (the same bits either way). stats (optional, device
- * uint64[HTC_STAT_COUNT]) accumulates the HTC_STAT_* counters. */
+ * or as wavefronts in the pool (the same bits either way). The queues go by the canvas
+ * alone, not by the scene; a captured call runs the one-pass kernel unless an earlier call left queues
+ * as large, and its graph holds until a call on a larger canvas replaces them. stats (optional,
+ * device uint64[HTC_STAT_COUNT]) accumulates the HTC_STAT_* counters. */
 int htc_render_passes(htc_program *program, uint32_t width, uint32_t height, const void *scene,
                       size_t scene_size, float *canvas, uint32_t *seeds, uint32_t passes,
                       uint64_t *stats, void *stream);
