@@ -2123,6 +2123,7 @@ struct htc_batch {
     size_t wcnt_words;
     float4 *images;          // the views' scene images
     size_t image_words;
+    std::vector<float4 *> old_images;   // smaller ones, which launches and graphs may still read
     void *sort_buf;          // coherence sort of the hyperbolic views (BatchSortBuf)
     uint64_t sort_slots;     // = wave_slots when allocated
     uint32_t hops_of[2], passes_of[2];   // the most of the hyperbolic, of the Euclidean views
@@ -2150,6 +2151,7 @@ static void batch_free(htc_batch *b) {
     if (b->d_wcnt) cudaFree(b->d_wcnt);
     if (b->sort_buf) cudaFree(b->sort_buf);
     if (b->images) cudaFree(b->images);
+    for (float4 *old : b->old_images) cudaFree(old);
     if (b->graph_exec) cudaGraphExecDestroy(b->graph_exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     cudaFree(b->d_views);
@@ -2299,8 +2301,8 @@ void htc_batch_destroy(htc_batch *b) { batch_free(b); }
 
 // Grows the wavefront queues (slots per queue) and counters (words) when a view set needs
 // more; launches already enqueued on `st` may still use the old ones, so they finish first.
-static int batch_grow(htc_batch *b, uint64_t slots, size_t words, size_t images, cudaStream_t st) {
-    if (slots <= b->wave_slots && words <= b->wcnt_words && images <= b->image_words && (!HT_BATCH_SORT || b->sort_slots >= b->wave_slots)) return HTC_OK;
+static int batch_grow(htc_batch *b, uint64_t slots, size_t words, cudaStream_t st) {
+    if (slots <= b->wave_slots && words <= b->wcnt_words && (!HT_BATCH_SORT || b->sort_slots >= b->wave_slots)) return HTC_OK;
     HTC_CUDA(cudaStreamSynchronize(st));
     // a captured graph holds the old buffers' addresses: the next graph launch captures anew
     if (b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
@@ -2320,13 +2322,6 @@ static int batch_grow(htc_batch *b, uint64_t slots, size_t words, size_t images,
         HTC_CUDA(cudaMalloc(&b->d_wcnt, sizeof(uint32_t) * words));
         b->wcnt_words = words;
     }
-    if (images > b->image_words) {
-        if (b->images) HTC_CUDA(cudaFree(b->images));
-        b->images = nullptr;
-        b->image_words = 0;
-        HTC_CUDA(cudaMalloc(&b->images, sizeof(float4) * (images + images / 4)));
-        b->image_words = images + images / 4;
-    }
     if (HT_BATCH_SORT && b->sort_slots < b->wave_slots) {
         if (b->sort_buf) HTC_CUDA(cudaFree(b->sort_buf));
         b->sort_buf = nullptr;
@@ -2336,14 +2331,31 @@ static int batch_grow(htc_batch *b, uint64_t slots, size_t words, size_t images,
     }
     return HTC_OK;
 }
+// Room for the views' scene images. Nothing waits: the view table of the launches enqueued so far
+// points into the buffer that was, which is kept until the batch is destroyed (the new one is at least
+// twice as large, so all of them together are less than it).
+static int batch_grow_images(htc_batch *b, size_t words) {
+    if (words <= b->image_words) return HTC_OK;
+    words = std::max(words, 2 * b->image_words);
+    float4 *images = nullptr;
+    HTC_CUDA(cudaMalloc(&images, sizeof(float4) * words));
+    if (b->images) b->old_images.push_back(b->images);
+    b->images = images;
+    b->image_words = words;
+    return HTC_OK;
+}
 
 extern "C" {
 
 int htc_batch_reserve(htc_batch *b, uint64_t pixels, uint32_t max_hops, void *stream) {
     if (!b) return fail(HTC_ERR_INVALID, "batch is NULL");
     if (max_hops == 0) return fail(HTC_ERR_INVALID, "max_hops must be positive");
+    // images of the largest scenes for as many views as 64 MB hold (287; more by demand, batch_grow_images)
+    const size_t largest = 1 + (size_t)b->max_smem / 16;
+    int rc = batch_grow_images(b, std::min(b->max_views * largest, (size_t)(64u << 20) / sizeof(float4)));
+    if (rc) return rc;
     // each view's region is rounded up to 64 slots
-    return batch_grow(b, pixels + 64ull * b->max_views, (size_t)(b->max_views + 3) * max_hops, 0,
+    return batch_grow(b, pixels + 64ull * b->max_views, 4 * (size_t)batch_counters(b->max_views, max_hops),
                       reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -2410,7 +2422,8 @@ int htc_batch_set_views(htc_batch *b, const htc_view *views, uint32_t n_views, u
     b->tile_pixels = tile_pixels;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     {
-        int rc = batch_grow(b, slots, 4 * (size_t)batch_counters(n_views, hops_max), images, st);
+        int rc = batch_grow(b, slots, 4 * (size_t)batch_counters(n_views, hops_max), st);
+        if (!rc) rc = batch_grow_images(b, images);
         if (rc) return rc;
     }
     images = 0;

@@ -217,9 +217,10 @@ void htc_batch_destroy(htc_batch *batch);
  * copied (two calls back). */
 int htc_batch_set_views(htc_batch *batch, const htc_view *views, uint32_t n_views,
                         uint32_t tile_pixels, uint32_t blocks_per_sm, void *stream);
-/* Sizes the batch's wavefront queues (2 x 68 bytes per pixel) for view sets of up to `pixels`
- * pixels in total and up to `max_hops` light hops, so that htc_batch_set_views need not grow
- * them (growing waits for the launches already enqueued on `stream`). */
+/* Sizes the batch's wavefront queues (2 x 68 bytes per pixel) and counters for view sets of up to
+ * `pixels` pixels in total and up to `max_hops` light hops, so that htc_batch_set_views need not grow
+ * them (growing waits for the launches already enqueued on `stream`), and takes up to 64 MB for the
+ * views' scene images (a view set that needs more takes it without waiting). */
 int htc_batch_reserve(htc_batch *batch, uint64_t pixels, uint32_t max_hops, void *stream);
 /* Renders every view's `passes`: one launch per pass index, hop depth and recipe over all the
  * views (wavefronts); the Euclidean launches run on a stream of the batch's own, which waits for
