@@ -1765,6 +1765,7 @@ static int narrow_scene(htc_program *p, const void **scene, size_t *scene_size, 
 }
 
 // One pass with the one-pass kernel (checked arguments).
+constexpr uint32_t PLAIN_ROWS = 4u * 65535u;   // 4 rows a block, 65535 blocks
 static int render_plain_pass(htc_program *p, uint32_t W, uint32_t H, const void *scene, size_t scene_size, uint32_t max_objects,
                              size_t smem, float *canvas, uint32_t *seeds, uint64_t *stats, void *stream) {
     dim3 grid((W + 31) / 32, (H + 3) / 4);
@@ -2029,7 +2030,8 @@ int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene,
     const uint64_t pixels = (uint64_t)W * H;
     // Euclidean scenes of few objects need more pixels to pay for the launches (us per pass, one-pass
     // kernel / wavefronts, 3 and 9 objects: 1024x768 80/91 and 83/93, 1440x900 122/123 and 125/124).
-    const bool few = p->recipe == HTC_RECIPE_EU && max_objects < EU_WAVE_OBJECTS;
+    // The one-pass kernel's grid ends at PLAIN_ROWS rows.
+    const bool few = p->recipe == HTC_RECIPE_EU && max_objects < EU_WAVE_OBJECTS && H <= PLAIN_ROWS;
     const bool own = pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100 && pixels >= WAVE_PIXELS);
     if (own && (wave_reserved(p, pixels) || !capturing(reinterpret_cast<cudaStream_t>(stream))))
         return render_wavefront_impl(p, W, H, scene, scene_size, canvas, seeds, passes, stats, stream);

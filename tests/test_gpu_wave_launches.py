@@ -217,3 +217,16 @@ def test_one_pass_calls_equal_one_pass_kernel(built, geometry, n, W, H, hops):
     got = _bits(canvas)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
     assert stats.cpu().tolist() == want_stats
+
+
+@pytest.mark.parametrize("geometry,n,W,H", [("eu", 9, 2, 262144), ("eu", 9, 3, 262141), ("eu", 3, 1, 524291), ("eu", 15, 4, 300001),
+                                            ("hy", 5, 2, 262145)])
+def test_canvases_of_more_rows_than_the_one_pass_kernel_takes(built, geometry, n, W, H):
+    ctx = P.Context(0)
+    scene = _scene(geometry, n, 3)
+    render = P.Render(ctx, scene.recipe, scene.hops)
+    buffer = P.EntityBuffer(ctx, scene)
+    canvases = [P.Canvas(ctx, (W, H), 6) for _ in range(2)]
+    render.render_passes(buffer, canvases[0], 2)
+    render.render_wavefront(buffer, canvases[1], 2)
+    assert np.array_equal(_bits(canvases[0])[0], _bits(canvases[1])[0]) and np.array_equal(_bits(canvases[0])[1], _bits(canvases[1])[1])
