@@ -1028,7 +1028,7 @@ template <int RF, int FH>
 __global__ void __launch_bounds__(128, minb_batch(RF == RECIPE_EU)) render_batch_wave(
     const BatchView *__restrict__ views, const uint32_t *__restrict__ order, uint32_t n_order, uint32_t n_views,
     uint32_t pass, uint32_t h, uint32_t tile_slots, uint32_t smem_objects, WaveQueue in, WaveQueue out,
-    uint32_t *cnt, uint32_t *grab, uint64_t *stats, uint32_t n_sorted, uint32_t *clear, uint32_t n_clear) {
+    uint32_t *cnt, uint32_t *grab, uint64_t *stats, uint32_t n_sorted, uint32_t *clear, size_t n_clear) {
     extern __shared__ float4 smem[];
     __shared__ uint32_t s_tile, s_next, s_total, s_tsize;
     __shared__ int s_staged_view, s_staged_ok;
@@ -1037,7 +1037,7 @@ __global__ void __launch_bounds__(128, minb_batch(RF == RECIPE_EU)) render_batch
     wait_previous();
     launch_next();
     if (FH == 1 && blockIdx.x == 0)
-        for (uint32_t i = tid; i < n_clear; i += blockDim.x) clear[i] = 0;
+        for (size_t i = tid; i < n_clear; i += blockDim.x) clear[i] = 0;
 
     // tiles of every view at this hop, in `order`, as a prefix sum. The tile size adapts to
     // the launch: about 16 tiles per block when the paths are few (a multiple of 128 slots,
@@ -2133,7 +2133,8 @@ struct htc_batch {
     cudaEvent_t forked, joined;
 };
 // Counters of one recipe and pass: every view's paths by hop, then the tiles taken by hop.
-static uint32_t batch_counters(uint32_t n_views, uint32_t hops) { return (n_views + 1) * hops; }
+constexpr size_t batch_counters(uint32_t n_views, uint32_t hops) { return ((size_t)n_views + 1) * hops; }
+static_assert(batch_counters(4096, 0xFFFFFFFFu) == 4097ull * 0xFFFFFFFFull && batch_counters(0xFFFFFFFFu, 1) == 1ull << 32, "counted in 64 bits");
 
 static void batch_free(htc_batch *b) {
     if (!b) return;
@@ -2188,14 +2189,14 @@ static int batch_wave_blocks(htc_batch *b, size_t smem, unsigned *blocks) {
 static int batch_passes(htc_batch *b, const WaveQueue (&q)[2], unsigned blocks_hy, unsigned blocks_eu, size_t smem, uint32_t n_seg,
                         uint64_t *stats, cudaStream_t st, cudaStream_t st_eu) {
     // each geometry has counters of its own, in two sets: a pass's hop 0 clears the next one's
-    const uint32_t words = batch_counters(b->n_views, b->hops_max);
+    const size_t words = batch_counters(b->n_views, b->hops_max);
     const uint32_t *order_hy = b->d_order + b->n_order, *order_eu = order_hy + b->n_hy;
     const unsigned sort_blocks = (unsigned)b->num_sms;
     const BatchSortBuf sb = n_seg ? batch_sort_at(b->sort_buf, b->sort_slots, sort_blocks) : BatchSortBuf{};
     const size_t sort_smem = sizeof(uint32_t) * (SORT_BINS + 2 * n_seg + 1);
     uint32_t sorts = 0;   // both sets of histograms start cleared; k_bsort_scatter clears the one its depth did not use
     for (uint32_t pass = 0; pass < b->passes_max; ++pass) {
-        uint32_t *set = b->d_wcnt + (size_t)(pass & 1u) * words, *next = b->d_wcnt + (size_t)(~pass & 1u) * words;
+        uint32_t *set = b->d_wcnt + (pass & 1u) * words, *next = b->d_wcnt + (~pass & 1u) * words;
         for (uint32_t h = 0; h < b->hops_max; ++h) {
             const WaveQueue &in = q[(h + 1) & 1], &out = q[h & 1];
             uint32_t *cnt = set, *grab = cnt + (size_t)b->n_views * b->hops_max + h;
@@ -2248,7 +2249,7 @@ static int batch_launch_wave(htc_batch *b, uint64_t *stats, cudaStream_t st) {
     const uint32_t n_seg = HT_BATCH_SORT && b->sort_buf ? std::min(b->n_hy, BATCH_SORT_VIEWS) : 0u;
     if (n_seg) HTC_CUDA(cudaMemsetAsync(batch_sort_at(b->sort_buf, b->sort_slots, (unsigned)b->num_sms).hist, 0,
                                         2 * sizeof(uint32_t) * (size_t)BATCH_SORT_VIEWS * SORT_BINS, st));
-    HTC_CUDA(cudaMemsetAsync(b->d_wcnt, 0, 4 * sizeof(uint32_t) * (size_t)batch_counters(b->n_views, b->hops_max), st));
+    HTC_CUDA(cudaMemsetAsync(b->d_wcnt, 0, 4 * sizeof(uint32_t) * batch_counters(b->n_views, b->hops_max), st));
     k_batch_stage<<<b->n_order, STAGE_THREADS, 0, st>>>(b->d_views, b->d_order, b->d_err);
     HTC_CUDA(cudaGetLastError());
     if (!b->n_hy || !b->n_eu) return batch_passes(b, q, blocks_hy, blocks_eu, smem, n_seg, stats, st, st);
@@ -2357,7 +2358,7 @@ int htc_batch_reserve(htc_batch *b, uint64_t pixels, uint32_t max_hops, void *st
     int rc = batch_grow_images(b, std::min(b->max_views * largest, (size_t)(64u << 20) / sizeof(float4)));
     if (rc) return rc;
     // each view's region is rounded up to 64 slots
-    return batch_grow(b, pixels + 64ull * b->max_views, 4 * (size_t)batch_counters(b->max_views, max_hops),
+    return batch_grow(b, pixels + 64ull * b->max_views, 4 * batch_counters(b->max_views, max_hops),
                       reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -2424,7 +2425,7 @@ int htc_batch_set_views(htc_batch *b, const htc_view *views, uint32_t n_views, u
     b->tile_pixels = tile_pixels;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     {
-        int rc = batch_grow(b, slots, 4 * (size_t)batch_counters(n_views, hops_max), st);
+        int rc = batch_grow(b, slots, 4 * batch_counters(n_views, hops_max), st);
         if (!rc) rc = batch_grow_images(b, images);
         if (rc) return rc;
     }
