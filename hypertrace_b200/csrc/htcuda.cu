@@ -1454,9 +1454,18 @@ void pool_leave(int dev) {
         d.largest = 0;
     }
 }
+// While another stream captures in the global mode, calls that are not stream-ordered on every thread
+// would break its capture, and so do those of a pool. They do not touch that stream, so the thread
+// leaves the mode for as long as it works with the pool.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 // A block of `bytes` for work on `st`, or NULL.
 void *pool_take(int dev, size_t bytes, cudaStream_t st) {
     if (dev < 0) return nullptr;
+    const RelaxedCapture relaxed;
     DevicePool &d = g_pools[dev];
     std::lock_guard<std::mutex> lock(d.mutex);
     cudaError_t e = cudaSuccess;
@@ -1480,6 +1489,11 @@ void *pool_take(int dev, size_t bytes, cudaStream_t st) {
         return nullptr;
     }
     return block;
+}
+// Gives the block back when the work enqueued on `st` so far is done.
+cudaError_t pool_give(void *block, cudaStream_t st) {
+    const RelaxedCapture relaxed;
+    return cudaFreeAsync(block, st);
 }
 }  // namespace
 
@@ -1955,7 +1969,7 @@ static int render_wave_pooled(htc_program *p, uint32_t W, uint32_t H, const void
     *done = true;
     wave_work_block(p, (uint64_t)W * H, max_objects, reinterpret_cast<uint8_t *>(block), &w);
     const int rc = launch_wave_any(p, w, W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats, st);
-    const cudaError_t e = cudaFreeAsync(block, st);
+    const cudaError_t e = pool_give(block, st);
     return rc ? rc : e != cudaSuccess ? cuda_fail(e, "cudaFreeAsync") : HTC_OK;
 }
 
@@ -2341,6 +2355,7 @@ static int batch_grow_images(htc_batch *b, size_t words) {
     if (words <= b->image_words) return HTC_OK;
     words = std::max(words, 2 * b->image_words);
     float4 *images = nullptr;
+    const RelaxedCapture relaxed;
     HTC_CUDA(cudaMalloc(&images, sizeof(float4) * words));
     if (b->images) b->old_images.push_back(b->images);
     b->images = images;

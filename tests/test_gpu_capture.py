@@ -93,3 +93,34 @@ def test_captured_call_without_queues(built, earlier):
         graph.replay()
         stream.synchronize()
     assert _same(got, want)
+
+
+@pytest.mark.parametrize("size", [(200, 150), (512, 288), (1031, 521)])
+@pytest.mark.parametrize("earlier_call", [False, True])
+def test_one_pass_call_on_another_stream_while_one_captures(built, size, earlier_call):
+    """The capture forbids calls that might disturb it, on every stream and thread (the global mode, torch's
+    default): a one-pass call on a stream of its own is none, whatever workspace it takes."""
+    ctx = P.Context(0)
+    scene = _scene(40)
+    buffer = P.EntityBuffer(ctx, scene)
+    want = P.Canvas(ctx, size, 5)
+    captured, beside = P.Canvas(ctx, size, 5), P.Canvas(ctx, size, 5)
+    reference = P.Render(ctx, scene.recipe, HOPS)
+    for _ in range(2):
+        reference.render(buffer, want)
+    del reference   # the device has no program, and no pool, but this one's
+    render = P.Render(ctx, scene.recipe, HOPS)
+    if earlier_call:
+        render.render(buffer, P.Canvas(ctx, size, 5))
+    streams, graph = [torch.cuda.Stream(), torch.cuda.Stream()], torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=streams[0]):
+        render.render(buffer, captured, sync=False)
+        with torch.cuda.stream(streams[1]):
+            render.render(buffer, beside, sync=False)
+            render.render(buffer, beside, sync=False)
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    for canvas in (captured, beside):
+        assert _same(canvas, want)
