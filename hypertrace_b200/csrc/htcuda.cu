@@ -1426,17 +1426,19 @@ __global__ void __launch_bounds__(256) k_fma_probe(float *out, int iters) {
 // One memory pool per device for the workspaces that calls take and give back in stream order
 // (render_wave_pooled), shared by the device's programs so that a new program finds memory that
 // an earlier one's calls have mapped (a pool per program made its first call 2 to 15 ms long). Made
-// by the first call that needs it, destroyed with the last program; between calls it keeps two
+// by the first call that needs it, destroyed with the last program; between calls it keeps up to two
 // workspaces of the largest size taken so far and 64 MB (its reservations are larger than what
 // is taken from them, and what is over the limit goes back to the system at every
-// synchronisation: 200 us a call).
+// synchronisation: 200 us a call). What it keeps is not lost to others: an allocation that needs it
+// gets it (cudaMalloc of the device's free memory and half of what the pool kept succeeds).
 namespace {
 constexpr int MAX_DEVICES = 64;
 struct DevicePool {
     std::mutex mutex;
     cudaMemPool_t pool = nullptr;
     uint32_t programs = 0;
-    size_t largest = 0;
+    size_t largest = 0;    // workspace taken so far
+    uint32_t without = 0;  // passes that asked for a larger one since
 } g_pools[MAX_DEVICES];
 int pool_enter(int dev) {
     if (dev < 0 || dev >= MAX_DEVICES) return -1;
@@ -1453,6 +1455,7 @@ void pool_leave(int dev) {
         d.pool = nullptr;
         d.largest = 0;
     }
+    if (d.programs == 0) d.without = 0;
 }
 // While another stream captures in the global mode, calls that are not stream-ordered on every thread
 // would break its capture, and so do those of a pool. They do not touch that stream, so the thread
@@ -1462,12 +1465,22 @@ struct RelaxedCapture {
     RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
     ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
-// A block of `bytes` for work on `st`, or NULL.
-void *pool_take(int dev, size_t bytes, cudaStream_t st) {
+// A block of `bytes` for `passes` passes on `st`, or NULL. A workspace larger than any before has to be
+// mapped, which takes 1.2 ms at 800x600 and 3 at 1080p, more than wavefronts save on a few passes. So
+// the first POOL_WITHOUT passes that ask for one go without, in calls of up to POOL_LONG passes: a program
+// that is made for a frame or two and destroyed maps nothing (made, one frame, destroyed: 18 objects at
+// 800x600 2.1 -> 1.1 ms, 200 at 1080p 6.0 -> 3.7; two frames 2.6 -> 1.5 and 7.3 -> 6.5; 8 passes in one call
+// of 18 and of 77 objects 5.3 -> 4.1 and 3.6 -> 3.4, 16 passes 9.1 with either).
+constexpr uint32_t POOL_WITHOUT = 4, POOL_LONG = 8;
+void *pool_take(int dev, size_t bytes, uint32_t passes, cudaStream_t st) {
     if (dev < 0) return nullptr;
     const RelaxedCapture relaxed;
     DevicePool &d = g_pools[dev];
     std::lock_guard<std::mutex> lock(d.mutex);
+    if (bytes > d.largest && d.without < POOL_WITHOUT && passes <= POOL_LONG) {
+        d.without += passes;
+        return nullptr;
+    }
     cudaError_t e = cudaSuccess;
     if (!d.pool) {
         cudaMemPoolProps props = {};
@@ -1480,7 +1493,10 @@ void *pool_take(int dev, size_t bytes, cudaStream_t st) {
     if (e == cudaSuccess && bytes > d.largest) {
         uint64_t keep = 2 * (uint64_t)bytes + (64u << 20);
         e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e == cudaSuccess) d.largest = bytes;
+        if (e == cudaSuccess) {
+            d.largest = bytes;
+            d.without = 0;
+        }
     }
     void *block = nullptr;
     if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&block, bytes, d.pool, st);
@@ -1964,7 +1980,7 @@ static int render_wave_pooled(htc_program *p, uint32_t W, uint32_t H, const void
     if (capturing(st)) return HTC_OK;
     WaveWork w;
     const size_t bytes = wave_work_block(p, (uint64_t)W * H, max_objects, nullptr, &w);
-    void *block = pool_take(p->device, bytes, st);
+    void *block = pool_take(p->device, bytes, H > PLAIN_ROWS ? 0xFFFFFFFFu : passes, st);   // the one-pass kernel ends there
     if (!block) return HTC_OK;
     *done = true;
     wave_work_block(p, (uint64_t)W * H, max_objects, reinterpret_cast<uint8_t *>(block), &w);
