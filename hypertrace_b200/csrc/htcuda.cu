@@ -116,7 +116,8 @@ struct htc_program {
 // false (uniformly across the block) when the scene bytes fail validation.
 //
 // Hyperbolic scenes are staged in scan order, geodesic planes first, then horospheres, each by
-// their distance from the camera (scenes of up to STAGE_SORT_MAX objects; index order beyond):
+// their distance from the camera (scenes of 7 to STAGE_SORT_MAX objects; index order for fewer, where the
+// order gains nothing and its keys cost 3 objects at 1024x700 66 -> 71 us a pass, and beyond):
 // the paths of a view stay near it, so the first few slots of a shape nearly always hold a sure
 // crossing close to the winner's (upper_estimate), and the later chunks fall to the warp
 // pre-cull. When the plane count is odd a dummy slot follows the planes,
@@ -246,7 +247,8 @@ __device__ bool stage_scene(const uint8_t *scene, size_t scene_size, uint32_t ma
         // pass 1: the number of planes, and every object's sort key (shape, distance from the
         // camera; both shapes' distances grow with |F| or max(F, 1 / F) of the bound record)
         uint32_t *keys = reinterpret_cast<uint32_t *>(sm.win);
-        const bool by_distance = n <= STAGE_SORT_MAX;
+        // (up to HT_EST_OBJECTS / 2 objects the estimate looks at all of them, whatever their order)
+        const bool by_distance = n > HT_EST_OBJECTS / 2 && n <= STAGE_SORT_MAX;
         const Q4 cam = mo_apply_pos(load_mo(scene), q4(0.0f, 0.0f, 1.0f, 0.0f));
         const BoundRay at = bound_ray(cam, q4(1.0f, 0.0f, 0.0f, 0.0f));
         for (uint32_t r0 = 0; r0 < n; r0 += nthreads) {
