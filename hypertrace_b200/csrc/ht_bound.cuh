@@ -155,14 +155,14 @@ HT_D Cull cull_none() {
 //   geodesic plane  culled when |F| - eF > 2 t S (sinh of the distance to the plane);
 //   horosphere      culled when t > E (F + eF) or t E < F - eF (the local height t' = t / F
 //                   outside [e^-thr, e^thr] even with F's error).
-// The point bound of two slots of one shape at once (packed FP32: each component rounds as the
-// scalar operation does). An object is culled when F + eF < lo or F - eF > hi:
-//   geodesic plane  lo = -2 t S, hi = 2 t S: the same decision as |F| - eF > 2 t S, op for
-//                   op (|F| - eF = -(F + eF) exactly when F < 0);
+// The point bound as thresholds on F: an object is culled when F + eF < lo or F - eF > hi. (In the packed
+// form, two slots of one shape at once, the product mag K and its sum with F may be rounded once
+// instead of twice, as ht_math.cuh says of packed sums: a last place of eF, which is 1e-5 of F and more.)
+//   geodesic plane  lo = -2 t S, hi = 2 t S: |F| - eF > 2 t S (|F| - eF = -(F + eF) when F < 0);
 //   horosphere      lo = t / E (E an upper bound of e^thr raised by 1e-5, so this stays below
 //                   t e^-thr after its rounding and the rcp approximation), hi = t E: the
 //                   test t > E (F + eF) or t E < F - eF with the division moved to the threshold.
-// A NaN record (ill-conditioned map) is never culled. Returns the survivors as bits 0 and 1.
+// A NaN record (ill-conditioned map) is never culled.
 struct PointCut { float2 lo, hi; };
 HT_D PointCut point_cut(uint32_t shape, float t, const Cull &c) {
     PointCut k;
@@ -183,7 +183,6 @@ HT_D bool culled_point(float4 rec, float mag, const BoundRay &r, const PointCut 
     const float eF = mag * r.K;
     return F + eF < k.lo.x || F - eF > k.hi.x;
 }
-// true when object `rec` provably cannot be hit nearer than the current threshold
 // F, W of one object along the ray and the bounds of their float error
 struct BoundFW { float F, eF, W, eW; };
 HT_D BoundFW bound_fw(float4 rec, float mag, const BoundRay &r) {

@@ -1162,13 +1162,12 @@ template <class O0, class... O> struct ChoiceTraits<O0, O...> {
 // HTG_BOUND_CAP elements. With the elements ordered by distance even a few are worth it (hy_tiled
 // type at 800x600, 6 hops, 4 passes, with / without the bounds: 4 elements 1665 / 1738 us, 12 2965 /
 // 3616, 31 3140 / 7683; 64 in index order with an estimate over 32 6049, by distance over 16 3874).
-#ifndef HTG_EST   // elements the upper estimate looks at (64 at 1080p, 4 passes: 8 23.4 ms, 12 19.74, 16 19.84,
-                  // 24 20.7; 20, 31, 120 at 800x600, 12 / 16: 3188 / 3300 us, 3140 / 3235, 3305 / 3405)
-#define HTG_EST 12u
-#endif
-#ifndef HTG_BOUND_CAP
-#define HTG_BOUND_CAP 256u
-#endif
+// Vectors of more elements, and those below a mapped object, are scanned without bounds (a cap of 512 takes
+// 300 elements at 800x600, 4 passes 45.5 -> 3.7 ms, but the example at 800x600 3.57 -> 3.70 ms for its
+// shared memory).
+constexpr u32 HTG_EST = 12;   // elements the upper estimate looks at (64 at 1080p, 4 passes: 8 23.4 ms, 12 19.74, 16 19.84,
+                              // 24 20.7; 20, 31, 120 at 800x600, 12 / 16: 3188 / 3300 us, 3140 / 3235, 3305 / 3405)
+constexpr u32 HTG_BOUND_CAP = 256;
 template <class G, class O> struct VecBounds { static constexpr bool ok = false; };
 template <class X> struct VecBounds<Hy, MappedObject<Hy, X, Moebius>> {
     static constexpr bool ok = BoundKind<X>::kind >= 0;

@@ -8,9 +8,9 @@
 // view/mapped.inl:20-26) and the constant background (background/constant.inl:18-21).
 //
 // Scheduling differs from the reference, results do not:
-//  * the object scan keeps only (distance, index) per candidate and recomputes the
-//    winner's local hit afterwards -- the same inputs through the same operations give the
-//    same bits, so this equals keeping every candidate's light/cache copy;
+//  * the object scan keeps the best candidate's distance, index and local ray, and computes
+//    its hit point and normal from that ray afterwards -- the same inputs through the same
+//    operations give the same bits, so this equals keeping every candidate's light/cache copy;
 //  * only the winner is mapped back to world space (the reference maps every candidate
 //    back, mapped.inl:34, but only the kept copy is observable);
 //  * inverse maps are computed once per launch and staged in shared memory.
@@ -149,7 +149,7 @@ struct StagedScene {
     const float4 *bound;     // shared, 1 per slot: world-space form for distance bounds
     const float4 *pa, *pb;   // shared, per pair of slots: {x0, x1, y0, y1}, {z0, z1, w0, w1} of bound
     const float2 *pmag;      // shared, per pair of slots: {mag0, mag1}
-    const float *mag;        // shared, 1 per slot: BOUND_EPS * max |bound component|
+    const float *mag;        // shared, 1 per slot: the record's error magnitude (bound_mag)
     const uint32_t *orig;    // shared, 1 per slot: the object's index in the scene
     float4 *win;             // shared, this thread's 2 float4: the scan winner's local ray
     const uint8_t *objects;  // global, OBJ_STRIDE per object (forward maps, materials), by scene index
@@ -246,10 +246,10 @@ static __device__ __noinline__ HyPath camera_hy(const StagedScene &s, float px, 
 // 11.84 ms, 12 11.29, 16 11.56, 24 12.10; 24 mixed views batched 41.1, 41.0, 41.9, 44.0 ms. In scene
 // order 24 to 40 objects were best, and the scan tested 3.2-4.9 objects per hop where it now
 // tests 1.4-2.2 (16.3 and 55.3 ms before the slot order, the allowances of ht_bound.cuh and the
-// warp-uniform ray-aware tests).
-#ifndef HT_EST_OBJECTS
-#define HT_EST_OBJECTS 12u
-#endif
+// warp-uniform ray-aware tests). Scenes of more than 1024 objects stay in scene order and take the
+// same 12: with all of that together 1025, 1500 and 2500 objects at 1280x720, 4 passes take 7.3, 39.4 and
+// 19.9 ms (8.8, 60.5 and 24.4 before it, with 24).
+constexpr uint32_t HT_EST_OBJECTS = 12;
 struct PairRay { float2 r2, x, y, K; };   // the bound ray's constants, each in both halves
 HT_D PairRay pair_ray(const BoundRay &r) {
     PairRay p;

@@ -52,9 +52,6 @@ thread_local std::string g_last_error;
 constexpr int MINB_PERSIST = 6, MINB_PLAIN = 5;
 constexpr int minb_wave(bool eu, bool first) { return eu ? (first ? 9 : 6) : (first ? 5 : 4); }
 constexpr int minb_batch(bool eu) { return eu ? 6 : 5; }
-#ifndef HT_BATCH_SORT   // coherence sort of the batch's hyperbolic views
-#define HT_BATCH_SORT 1
-#endif
 
 // Launches of one call that follow each other directly overlap at their edges (programmatic
 // dependent launch). A kernel waits for the end of the one before it (wait_previous) and then lets
@@ -81,9 +78,8 @@ static cudaError_t launch(bool overlap, void (*kernel)(P...), unsigned grid, uns
     return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
-#ifndef HT_SORT_MIN
-#define HT_SORT_MIN 131072u
-#endif
+constexpr uint32_t SORT_MIN = 131072;   // paths from which on a queue of a single view is sorted
+
 // Device error word bits.
 constexpr uint32_t ERR_SCENE = 1u;
 constexpr uint32_t ERR_SMEM = 2u;
@@ -783,7 +779,7 @@ __global__ void __launch_bounds__(128, minb_wave(R == RECIPE_EU, FH == 1)) rende
 
     const uint32_t lane = threadIdx.x & 31;
     const bool last = hop_index + 1 >= hops;
-    if (FH != 1 && n < HT_SORT_MIN) in.o = nullptr;   // too few paths for the sort
+    if (FH != 1 && n < SORT_MIN) in.o = nullptr;   // too few paths for the sort
     LaneStats st;
     for (;;) {
         uint32_t base = 0;
@@ -817,10 +813,7 @@ __global__ void __launch_bounds__(128, minb_wave(R == RECIPE_EU, FH == 1)) rende
 constexpr uint32_t SORT_THREADS = 1024;
 constexpr uint32_t SORT_PER = 16;                            // slots per thread of the largest window
 constexpr uint32_t SORT_WINDOW_MAX = SORT_THREADS * SORT_PER, SORT_WINDOW_MIN = 2048;
-#ifndef SORT_POS
-#define SORT_POS 2
-#endif
-constexpr uint32_t SORT_POS_BITS = SORT_POS;                        // per axis
+constexpr uint32_t SORT_POS_BITS = 2;                        // per axis
 constexpr uint32_t SORT_BINS = 96u << (3 * SORT_POS_BITS);   // 6144
 static_assert(SORT_BINS % SORT_THREADS == 0, "the scan gives every thread a whole number of bins");
 struct SortBuf {
@@ -930,7 +923,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_keys(const float4 *__rest
     wait_previous();
     launch_next();
     const uint32_t n = *reinterpret_cast<const volatile uint32_t *>(count), win = sort_window(n, gridDim.x);
-    if (n < HT_SORT_MIN || (uint64_t)blockIdx.x * win >= n) return;
+    if (n < SORT_MIN || (uint64_t)blockIdx.x * win >= n) return;
     sort_cells(p, n, &cells);
     for (uint32_t w = blockIdx.x; (uint64_t)w * win < n; w += gridDim.x) {
         const uint32_t base = w * win, m = min(win, n - base);
@@ -974,7 +967,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint32_t *k
     launch_next();
     const uint32_t n = *reinterpret_cast<const volatile uint32_t *>(count), t = threadIdx.x, win = sort_window(n, gridDim.x);
     for (uint32_t b = blockIdx.x * SORT_THREADS + t; b < SORT_BINS; b += gridDim.x * SORT_THREADS) next_hist[b] = 0;
-    if (n < HT_SORT_MIN || (uint64_t)blockIdx.x * win >= n) return;
+    if (n < SORT_MIN || (uint64_t)blockIdx.x * win >= n) return;
     sort_scan(hist, s_base);
     for (uint32_t w = blockIdx.x; (uint64_t)w * win < n; w += gridDim.x) {
         const uint32_t base = w * win, m = min(win, n - base);
@@ -2060,8 +2053,12 @@ int htc_render_passes(htc_program *p, uint32_t W, uint32_t H, const void *scene,
     // hyperbolic scenes of 100 objects on (200 objects, us per pass, one-pass kernel / wavefronts: 320x240
     // 190/252, 400x300 260/280); the other calls may run on several streams at once and work in the pool.
     const uint64_t pixels = (uint64_t)W * H;
-    // Euclidean scenes of few objects need more pixels to pay for the launches (us per pass, one-pass
-    // kernel / wavefronts, 3 and 9 objects: 1024x768 80/91 and 83/93, 1440x900 122/123 and 125/124).
+    // Several passes pay for wavefronts on smaller canvases than one does, since the staging is shared and the
+    // launches overlap: 2^19 pixels for hyperbolic scenes of any size and Euclidean ones of 16 objects on
+    // (1024x520 and 1024x700, us of 8 passes, one-pass kernel / wavefronts: hyperbolic 1, 2, 4, 5 objects
+    // 343/291, 2210/2519, 1370/1280, 2958/2680 and 440/341, 2930/3301, 1722/1539, 4277/3808; Euclidean 16, 25, 33
+    // 731/843, 1217/1166, 1388/1314 and 970/988, 1592/1358, 1942/1619). Euclidean scenes of fewer objects need
+    // more pixels (us per pass, 3 and 9 objects: 1024x768 80/91 and 83/93, 1440x900 122/123 and 125/124).
     // The one-pass kernel's grid ends at PLAIN_ROWS rows.
     const bool few = p->recipe == HTC_RECIPE_EU && max_objects < EU_WAVE_OBJECTS && H <= PLAIN_ROWS;
     const bool own = pixels >= (few ? 5u << 18 : 1u << 19) || (p->recipe == HTC_RECIPE_HY && max_objects >= 100 && pixels >= WAVE_PIXELS);
@@ -2278,7 +2275,7 @@ static int batch_launch_wave(htc_batch *b, uint64_t *stats, cudaStream_t st) {
     if (!rc) rc = batch_wave_blocks<RECIPE_EU>(b, smem, &blocks_eu);
     if (rc) return rc;
     // coherence sort of the first n_seg hyperbolic views in launch order (the expensive ones)
-    const uint32_t n_seg = HT_BATCH_SORT && b->sort_buf ? std::min(b->n_hy, BATCH_SORT_VIEWS) : 0u;
+    const uint32_t n_seg = b->sort_buf ? std::min(b->n_hy, BATCH_SORT_VIEWS) : 0u;
     if (n_seg) HTC_CUDA(cudaMemsetAsync(batch_sort_at(b->sort_buf, b->sort_slots, (unsigned)b->num_sms).hist, 0,
                                         2 * sizeof(uint32_t) * (size_t)BATCH_SORT_VIEWS * SORT_BINS, st));
     HTC_CUDA(cudaMemsetAsync(b->d_wcnt, 0, 4 * sizeof(uint32_t) * batch_counters(b->n_views, b->hops_max), st));
@@ -2337,7 +2334,7 @@ void htc_batch_destroy(htc_batch *b) { batch_free(b); }
 // Grows the wavefront queues (slots per queue) and counters (words) when a view set needs
 // more; launches already enqueued on `st` may still use the old ones, so they finish first.
 static int batch_grow(htc_batch *b, uint64_t slots, size_t words, cudaStream_t st) {
-    if (slots <= b->wave_slots && words <= b->wcnt_words && (!HT_BATCH_SORT || b->sort_slots >= b->wave_slots)) return HTC_OK;
+    if (slots <= b->wave_slots && words <= b->wcnt_words && b->sort_slots >= b->wave_slots) return HTC_OK;
     HTC_CUDA(cudaStreamSynchronize(st));
     // a captured graph holds the old buffers' addresses: the next graph launch captures anew
     if (b->graph_exec) { cudaGraphExecDestroy(b->graph_exec); b->graph_exec = nullptr; }
@@ -2357,7 +2354,7 @@ static int batch_grow(htc_batch *b, uint64_t slots, size_t words, cudaStream_t s
         HTC_CUDA(cudaMalloc(&b->d_wcnt, sizeof(uint32_t) * words));
         b->wcnt_words = words;
     }
-    if (HT_BATCH_SORT && b->sort_slots < b->wave_slots) {
+    if (b->sort_slots < b->wave_slots) {
         if (b->sort_buf) HTC_CUDA(cudaFree(b->sort_buf));
         b->sort_buf = nullptr;
         b->sort_slots = 0;
