@@ -96,8 +96,7 @@ struct htc_program {
     void *wave_buf;            // two wavefront queues (WAVE_SLOT_BYTES per slot each), grown on demand
     size_t wave_slots;         // slots per queue
     uint32_t *d_wave_ctr;      // 2 counters per hop depth, two sets
-    void *sort_buf;            // coherence sort of the hyperbolic queues (SortBuf), grown with them
-    size_t sort_slots;
+    void *sort_buf;            // coherence sort of the hyperbolic queues (SortBuf), as many slots as they have
     float4 *image;             // the scene's image (stage_image), of the largest that can be staged
     int device;                // whose pool it uses (render_wave_pooled); -1: none
     int double_support;        // scene bytes in the double_support layout, narrowed before rendering
@@ -1813,56 +1812,44 @@ static int render_plain_pass(htc_program *p, uint32_t W, uint32_t H, const void 
 // coherence saves less. Measured, sorted / in queue order, us per pass: 1080p / 200 objects (4.7 hops
 // a path) 2764 / 3029, (2.0 hops) 1232 / 1245, 720p / 120 objects 1483 / 1542, 720p / 77 objects 721 / 708,
 // 1080p / 18 objects 1082 / 1070, 640x480 / 200 objects 471 / 396.
-static bool wave_sortable(const htc_program *p, uint64_t pixels) {
-    return p->recipe == HTC_RECIPE_HY && !(p->flags & HTC_FLAG_NO_SORT) && pixels >= (1u << 19);
-}
 static bool wave_sorted(const htc_program *p, uint64_t pixels, uint32_t max_objects) {
-    return wave_sortable(p, pixels) && max_objects >= 100;
+    return p->recipe == HTC_RECIPE_HY && !(p->flags & HTC_FLAG_NO_SORT) && pixels >= (1u << 19) && max_objects >= 100;
 }
-// Queues of W*H slots each (a hop never has more paths than pixels) and the hop counters;
-// allocated on the first call that needs more and kept with the program. All of it goes by the canvas
-// alone, whatever the scene: a call on a canvas no larger than an earlier one's allocates nothing,
-// so it can be captured, and frees nothing that a captured call's graph works in.
-static bool wave_reserved(const htc_program *p, size_t slots) {
-    return p->image && p->d_wave_ctr && p->wave_slots >= slots && (!wave_sortable(p, slots) || p->sort_slots >= slots);
-}
-static int wave_reserve(htc_program *p, size_t slots) {
+// Queues of W*H slots each (a hop never has more paths than pixels), the hop counters and the scene's
+// image; allocated on the first call that needs more and kept with the program. They go by the canvas
+// alone, whatever the scene, and the sort's buffer, which comes with the first call that sorts, by the
+// queues: a call on a canvas no larger than an earlier one's frees nothing that a captured call's graph
+// works in, and can be captured itself (if none sorted before it, it takes its paths in queue order).
+static bool wave_reserved(const htc_program *p, size_t slots) { return p->image && p->d_wave_ctr && p->wave_slots >= slots; }
+static int wave_reserve(htc_program *p, size_t slots, bool sorted) {
     if (!p->image) HTC_CUDA(cudaMalloc(&p->image, sizeof(float4) * (1 + (size_t)p->max_smem / 16)));   // image_words of the largest scene
     if (!p->d_wave_ctr) {
         // 2 words per hop depth, two sets
         HTC_CUDA(cudaMalloc(&p->d_wave_ctr, 4 * sizeof(uint32_t) * (size_t)p->hops));
     }
     slots = (slots + 63) & ~(size_t)63;   // keeps the second queue and every array 16-byte aligned
-    if (wave_sortable(p, slots) && p->sort_slots < slots) {
-        if (p->sort_buf) {
-            HTC_CUDA(cudaFree(p->sort_buf));
-            p->sort_buf = nullptr;
-            p->sort_slots = 0;
-        }
-        HTC_CUDA(cudaMalloc(&p->sort_buf, sort_bytes(slots, (uint32_t)p->num_sms)));
-        p->sort_slots = slots;
-    }
-    if (p->wave_slots >= slots) return HTC_OK;
-    if (p->wave_buf) {
-        HTC_CUDA(cudaFree(p->wave_buf));
+    if (p->wave_slots < slots) {
+        if (p->sort_buf) HTC_CUDA(cudaFree(p->sort_buf));
+        p->sort_buf = nullptr;
+        if (p->wave_buf) HTC_CUDA(cudaFree(p->wave_buf));
         p->wave_buf = nullptr;
         p->wave_slots = 0;
+        HTC_CUDA(cudaMalloc(&p->wave_buf, 2 * WAVE_SLOT_BYTES * slots));
+        p->wave_slots = slots;
     }
-    HTC_CUDA(cudaMalloc(&p->wave_buf, 2 * WAVE_SLOT_BYTES * slots));
-    p->wave_slots = slots;
+    if (sorted && !p->sort_buf) HTC_CUDA(cudaMalloc(&p->sort_buf, sort_bytes(p->wave_slots, (uint32_t)p->num_sms)));
     return HTC_OK;
 }
 // What one call's launches work in: the program's own buffers, or a block of the device's pool.
 struct WaveWork {
     float4 *image;
     uint32_t *ctr;      // 4 words per hop depth
-    void *sort;
-    size_t sort_slots;
+    void *sort;         // NULL: the paths stay in queue order
     void *queues;
-    size_t slots;       // per queue
+    size_t slots;       // per queue, and of the sort's buffer
 };
-static WaveWork wave_work_owned(const htc_program *p) {
-    return WaveWork{p->image, p->d_wave_ctr, p->sort_buf, p->sort_slots, p->wave_buf, p->wave_slots};
+static WaveWork wave_work_owned(const htc_program *p, bool sorted) {
+    return WaveWork{p->image, p->d_wave_ctr, sorted ? p->sort_buf : nullptr, p->wave_buf, p->wave_slots};
 }
 // The same laid out in one block at `base`; returns its size.
 static size_t wave_work_block(const htc_program *p, uint64_t pixels, uint32_t max_objects, uint8_t *base, WaveWork *w) {
@@ -1875,8 +1862,7 @@ static size_t wave_work_block(const htc_program *p, uint64_t pixels, uint32_t ma
     };
     w->image = reinterpret_cast<float4 *>(take(sizeof(float4) * image_words(max_objects)));
     w->ctr = reinterpret_cast<uint32_t *>(take(4 * sizeof(uint32_t) * (size_t)p->hops));
-    w->sort_slots = wave_sorted(p, pixels, max_objects) ? slots : 0;
-    w->sort = take(w->sort_slots ? sort_bytes(slots, (uint32_t)p->num_sms) : 0);
+    w->sort = wave_sorted(p, pixels, max_objects) ? take(sort_bytes(slots, (uint32_t)p->num_sms)) : nullptr;
     w->queues = take(2 * WAVE_SLOT_BYTES * slots);
     w->slots = slots;
     return at;
@@ -1909,9 +1895,9 @@ static int launch_wave(const htc_program *p, const WaveWork &w, uint32_t W, uint
     const uint64_t blocks0 = std::min<uint64_t>((uint64_t)per_sm0 * (uint64_t)p->num_sms, needed);
     const WaveQueue q[2] = {wave_queue(w, 0), wave_queue(w, 1)};
     const WaveQueue none = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    const bool sorted = wave_sorted(p, (uint64_t)W * H, max_objects);
+    const bool sorted = w.sort != nullptr;
     const unsigned sort_blocks = (unsigned)p->num_sms;
-    const SortBuf sb = sorted ? sort_buf_at(w.sort, w.sort_slots, sort_blocks) : SortBuf{};
+    const SortBuf sb = sorted ? sort_buf_at(w.sort, w.slots, sort_blocks) : SortBuf{};
     const size_t sort_smem = sizeof(uint32_t) * SORT_BINS;
     uint32_t sorts = 0;   // both histograms start cleared; k_sort_scatter clears the one its depth did not use
     if (sorted) HTC_CUDA(cudaMemsetAsync(sb.hist, 0, 2 * sizeof(uint32_t) * SORT_BINS, st));
@@ -1992,9 +1978,10 @@ static int render_wavefront_impl(htc_program *p, uint32_t W, uint32_t H, const v
     int rc = validate_render_args(p, W, H, scene, scene_size, canvas, seeds, &max_objects, &smem);
     if (rc) return rc;
     if (passes == 0) return HTC_OK;
-    rc = wave_reserve(p, (size_t)W * H);
+    const bool sorted = wave_sorted(p, (uint64_t)W * H, max_objects);
+    rc = wave_reserve(p, (size_t)W * H, sorted && !(wave_reserved(p, (size_t)W * H) && capturing(reinterpret_cast<cudaStream_t>(stream))));
     if (rc) return rc;
-    return launch_wave_any(p, wave_work_owned(p), W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats,
+    return launch_wave_any(p, wave_work_owned(p, sorted), W, H, scene, scene_size, max_objects, smem, canvas, seeds, passes, stats,
                            reinterpret_cast<cudaStream_t>(stream));
 }
 

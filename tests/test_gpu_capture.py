@@ -50,9 +50,10 @@ def test_capture_after_a_call_with_another_scene(built, first, captured):
     torch.cuda.synchronize()
 
 
-def test_graph_survives_a_call_with_a_larger_scene(built):
+@pytest.mark.parametrize("first", [30, 120])   # a captured call in queue order, one that sorts
+def test_graph_survives_a_call_with_a_larger_scene(built, first):
     ctx = P.Context(0)
-    scenes = [_scene(30), _scene(150), _scene(900)]
+    scenes = [_scene(first), _scene(150), _scene(900)]
     buffers = [P.EntityBuffer(ctx, s) for s in scenes]
     want = [_want(ctx, b, scenes[0].recipe, 2) for b in buffers]
     render, canvases = P.Render(ctx, scenes[0].recipe, HOPS), [P.Canvas(ctx, (W, H), 5) for _ in buffers]
