@@ -239,7 +239,7 @@ class Server:
 
 
 def plain_fifo(ctx: Context, requests: Sequence[Request], gamma: float = 1.0 / 2.2) -> Dict[str, object]:
-    """One request at a time in arrival order; each pass one launch of the plain kernel."""
+    """One request at a time in arrival order; each pass one htc_render call."""
     arrivals = sorted(requests, key=lambda r: r.arrival)
     renders: Dict[tuple, Render] = {}
     t0 = time.perf_counter()
